@@ -10,7 +10,7 @@
 // 2081-2126 (effective DOF, support mask).
 //
 // Everything except the exchange scoring is K-dimensional (K <= 32): one
-// warp per scene, lane i owning row i.  Fourier atoms are never
+// block per scene, lane i owning row i.  Fourier atoms are never
 // materialised:
 //   Gram      G[k][l] = D1[(n1k-n1l) mod N1] * D2[(n2k-n2l) mod N2]
 //             (Dirichlet kernels summed in FP64 once per plan),
@@ -91,260 +91,281 @@ FBME_DEV void load_dirichlet(const PolishArgs& A, float2* d1, float2* d2) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(d2 + i)), "l"(A.p.dir2 + i) : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncwarp();
+  __syncthreads();
 }
 
-// Exact reduced posterior + negative log evidence for the work set.
-// Returns in lane k: mean_k, pv_k, dd_k; nle (all lanes); status bits.
+// One scene's K-dimensional algebra runs on a block of kPolishWarps warps:
+// lane i owns row i, warp w the columns w, w + 8, w + 16, w + 24 of every
+// row.  Its cost is the serial chain of the factorisation, so the block is
+// there to shorten a step, not to add throughput: four entries of a row and
+// of the inverse a thread instead of up to 32 each.  Measured (B200, K = 32):
+// the three polish launches of one Stable scene 138 us in a single warp, 60 us
+// so; of a 512-scene replay 157 -> 128 us.  Every entry keeps its operations
+// and their order.
+constexpr int kPolishWarps = 8;
+constexpr int kPolishThreads = 32 * kPolishWarps;
+constexpr int kPolishCols = kMaxPolish / kPolishWarps;  // columns of a row per thread
+
+struct PolishShared {
+  float2 M[kMaxPolish][kMaxPolish + 1];  // the system, for its transpose
+  float2 L[kMaxPolish][kMaxPolish + 1];  // its Cholesky factor by columns: L[q][i] is entry (i, q)
+  float rl[kMaxPolish];                  // 1 / L[q][q]
+  float eqv[kMaxPolish];                 // squared column norms of L^-1
+  float2 mean[kMaxPolish];
+  double ev[3][kMaxPolish];              // logarithms of the evidence
+  double log_nu;
+  double2 gm[kPolishWarps][kMaxPolish];  // G mu, one partial sum per warp
+  float trace[kMaxEval];
+  int status;
+};
+
+// Column q of the factorisation: its owner warp arrives, the others wait.
+FBME_DEV void column_arrive(int q) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + (q & 1)), "n"(kPolishThreads) : "memory");
+}
+FBME_DEV void column_sync(int q) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (q & 1)), "n"(kPolishThreads) : "memory");
+}
+
+// Exact reduced posterior + negative log evidence for the work set, on the
+// whole block; every warp returns the same values: in lane k mean_k, pv_k,
+// dd_k; nle (all lanes).  Factorisation failures go to S.status.
 struct EvalOut {
   float2 mean;
   float pv, dd;
   double nle;
-  int status;
   float dscale;  // equilibration scale sqrt(S_kk) of lane k's row
 };
 
-FBME_DEV EvalOut evaluate(const PolishArgs& A, float2 (*M)[33], float2 (*X)[33], const float2* d1,
-                          const float2* d2, int K, int my_idx, float my_gamma, float nu, float2 my_c,
-                          float data_energy) {
-  const int lane = threadIdx.x & 31;
+// Complex updates of the factorisation with their rounding spelled out (the
+// first product fused, then one rounded sum), so that every kernel holding
+// them gives the same bits however the compiler contracts; the reduced
+// systems of close atoms are ill-conditioned enough to show the difference.
+FBME_DEV float2 add_mul(float2 v, float2 a, float2 b) {  // v + a b
+  return make_float2(__fadd_rn(v.x, fmaf(a.x, b.x, -__fmul_rn(a.y, b.y))),
+                     __fadd_rn(v.y, fmaf(a.x, b.y, __fmul_rn(a.y, b.x))));
+}
+FBME_DEV float2 sub_mul(float2 v, float2 a, float2 b) {  // v - a b
+  return make_float2(__fsub_rn(v.x, fmaf(a.x, b.x, -__fmul_rn(a.y, b.y))),
+                     __fsub_rn(v.y, fmaf(a.x, b.y, __fmul_rn(a.y, b.x))));
+}
+FBME_DEV float2 sub_mulc(float2 v, float2 a, float2 b) {  // v - a conj(b)
+  return make_float2(__fsub_rn(v.x, fmaf(a.x, b.x, __fmul_rn(a.y, b.y))),
+                     __fsub_rn(v.y, fmaf(a.y, b.x, -__fmul_rn(a.x, b.y))));
+}
+FBME_DEV float2 sub_cmul(float2 v, float2 a, float2 b) {  // v - conj(a) b
+  return make_float2(__fsub_rn(v.x, fmaf(a.x, b.x, __fmul_rn(a.y, b.y))),
+                     __fsub_rn(v.y, fmaf(a.x, b.y, -__fmul_rn(a.y, b.x))));
+}
+
+FBME_DEV EvalOut evaluate(const PolishArgs& A, PolishShared& S, const float2* d1, const float2* d2, int K,
+                          int my_idx, float my_gamma, float nu, float2 my_c, float data_energy) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const BatchShape& s = A.s;
   const bool on = lane < K;
   const int n1i = my_idx / s.n2, n2i = my_idx % s.n2;
   // One reciprocal per scale, reused by multiplication: a division here is
-  // a full IEEE sequence with a slow-path branch, on the critical path of
-  // a single warp.
+  // a full IEEE sequence with a slow-path branch, on the critical path.
   const float inv_nu = 1.0f / nu, inv_g = 1.0f / my_gamma;
   // system S = diag(1/gamma) + G / nu, Hermitian-symmetrised
+  float2 r[kPolishCols];
 #pragma unroll
-  for (int j = 0; j < kMaxPolish; ++j) {
+  for (int u = 0; u < kPolishCols; ++u) {
+    const int j = w + kPolishWarps * u;
     const int n1j = __shfl_sync(0xffffffffu, n1i, j), n2j = __shfl_sync(0xffffffffu, n2i, j);
+    r[u] = make_float2(0.f, 0.f);
     if (on && j < K) {
       const float2 g = gram_at(A, d1, d2, n1i, n2i, n1j, n2j);
-      float2 a = make_float2(g.x * inv_nu, g.y * inv_nu);
-      if (j == lane) a.x += inv_g;
-      M[lane][j] = a;
+      r[u] = make_float2(g.x * inv_nu, g.y * inv_nu);
+      if (j == lane) r[u].x = __fadd_rn(r[u].x, inv_g);
+      S.M[lane][j] = r[u];
     }
   }
-  __syncwarp();
-  float2 row[kMaxPolish];
-#pragma unroll
-  for (int j = 0; j < kMaxPolish; ++j)
-    if (on && j < K) {
-      const float2 a = M[lane][j], b = M[j][lane];
-      row[j] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-    }
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < kMaxPolish; ++j)
-    if (on && j < K) M[lane][j] = row[j];
-  __syncwarp();
-  const float dscale = on ? sqrtf(fmaxf(M[lane][lane].x, kTinyP)) : 1.0f;
+  __syncthreads();
+  const float diag = on ? S.M[lane][lane].x : 1.0f;
+  const float dscale = on ? sqrtf(fmaxf(diag, kTinyP)) : 1.0f;
   const float inv_d = 1.0f / dscale;
-  // equilibrate: E[i][j] = S[i][j] / (d_i d_j), symmetrise again
-  {
-#pragma unroll
-    for (int j = 0; j < kMaxPolish; ++j) {
-      const float idj = __shfl_sync(0xffffffffu, inv_d, j);
-      if (on && j < K) {
-        const float2 a = M[lane][j];
-        const float f = inv_d * idj;
-        row[j] = make_float2(a.x * f, a.y * f);
-      }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kMaxPolish; ++j)
-      if (on && j < K) M[lane][j] = row[j];
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kMaxPolish; ++j)
-      if (on && j < K) {
-        const float2 a = M[lane][j], b = M[j][lane];
-        row[j] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
-      }
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kMaxPolish; ++j)
-      if (on && j < K) M[lane][j] = row[j];
-    __syncwarp();
-  }
   // deterministic diagonal loading: multiplier * eps * mean|Re diag|
-  float dsum = on ? fabsf(M[lane][lane].x) : 0.f;
+  float dsum = on ? fabsf(diag * (inv_d * inv_d)) : 0.f;
   dsum = warp_sum(dsum);
   const float scale = fmaxf(dsum / static_cast<float>(K), kTinyP);
   const float jitter = A.c.jitter * (kEpsP * scale);
-  if (on) M[lane][lane].x += jitter;
-  __syncwarp();
-  // Cholesky, lower, in place, right-looking: once column q is final,
-  // lane i > q subtracts L[i][q] conj(L[k][q]) from its row entries k in
-  // (q, i] -- independent updates instead of one dot-product chain per
-  // entry.  Every entry receives its terms in the same order q = 0, 1, ...
-  // as the dot-product form.
-  // Each lane writes only its own row inside the loop.  Every lane computes
-  // the pivot from the diagonal entry; the column entries L[k][q] reach
-  // the other lanes through shared memory.  A row's diagonal takes its last
-  // update before the row updates of the step, so the next pivot's entry
-  // is final, and is loaded, before those updates.
-  int status = 0;
-  __syncwarp();
-  float dnext = K > 0 ? M[0][0].x : 1.0f;
-  for (int q = 0; q < K; ++q) {
-    float sdiag = dnext;
-    if (!(sdiag > 0.f)) {
-      if (lane == q) status |= isfinite(sdiag) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;
-      sdiag = kTinyP;
-    }
-    const float piv = sqrtf(sdiag);
-    const float rq = 1.0f / piv;
-    if (lane == q) M[q][q] = make_float2(piv, 0.f);
-    float2 a = make_float2(0.f, 0.f);
-    if (on && lane > q) {
-      const float2 v = M[lane][q];
-      a = make_float2(v.x * rq, v.y * rq);
-      M[lane][q] = a;
-      M[lane][lane].x -= abs2(a);
-    }
-    // column q reaches the other lanes through shared memory (X is free
-    // until the inverse factor); the row updates then go in batches of 8:
-    // all loads, then the arithmetic, then the stores, so the batch's
-    // shared-memory round trips overlap instead of running one by one
-    X[0][lane] = a;
-    __syncwarp();
-    if (q + 1 < K) dnext = M[q + 1][q + 1].x;
-    for (int k0 = q + 1; k0 < K; k0 += 8) {
-      float2 b[8], v[8];
+  // equilibrate: E[i][j] = S[i][j] / (d_i d_j).  S is exactly Hermitian
+  // after its symmetrisation and the scale is the same product for (i, j)
+  // and (j, i), so E is exactly Hermitian as well.
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (on && k0 + u < lane) {
-          b[u] = X[0][k0 + u];
-          v[u] = M[lane][k0 + u];
-        }
-#pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (on && k0 + u < lane) {
-          v[u].x -= a.x * b[u].x + a.y * b[u].y;  // a * conj(b)
-          v[u].y -= a.y * b[u].x - a.x * b[u].y;
-          M[lane][k0 + u] = v[u];
-        }
+  for (int u = 0; u < kPolishCols; ++u) {
+    const int j = w + kPolishWarps * u;
+    const float f = inv_d * __shfl_sync(0xffffffffu, inv_d, j);
+    if (on && j < K) {
+      const float2 b = S.M[j][lane];
+      r[u] = make_float2(0.5f * (r[u].x + b.x) * f, 0.5f * (r[u].y - b.y) * f);
+      if (j == lane) r[u].x = __fadd_rn(r[u].x, jitter);
     }
-    __syncwarp();
   }
-  __syncwarp();
-  status = __reduce_or_sync(0xffffffffu, status);
-  // mean: L z = c / nu / d, L^H w = z, mu = w / d
-  const float rl = on ? 1.0f / M[lane][lane].x : 1.0f;  // 1 / L[lane][lane]
+  // Cholesky, lower, right-looking, and in the same pass over q the inverse
+  // factor X = L^-1 and the forward solve L z = c / nu / d (in every warp).  A
+  // thread's entry r[u] is first the system's, updated by the columns left
+  // of its own, then (once its column is posted) the sum over k of
+  // L[lane][k] X[k][j], final for row q at step q, when row q of X lies in
+  // lane q of the same warp.  The chain that sets the time is column q ->
+  // entry (q+1, q+1) -> square root, reciprocal -> column q+1, so the warp
+  // that owns column q+1 takes it first, posts it, arrives at the column's
+  // barrier without waiting there, and makes the step's other updates after
+  // it (one barrier a step for all: 75 us for those three launches).  Columns
+  // stay where they are posted and the barrier ids alternate: a warp can
+  // reach the barrier of column q+2 only after every warp passed column q's.
   const float2 rhs = on ? make_float2(my_c.x * inv_nu, my_c.y * inv_nu) : make_float2(0.f, 0.f);
   float2 z = make_float2(rhs.x * inv_d, rhs.y * inv_d);
-  for (int q = 0; q < K; ++q) {
-    if (lane == q) z = make_float2(z.x * rl, z.y * rl);
-    const float2 zq = make_float2(__shfl_sync(0xffffffffu, z.x, q), __shfl_sync(0xffffffffu, z.y, q));
-    if (on && lane > q) {
-      const float2 l = M[lane][q];
-      z.x -= l.x * zq.x - l.y * zq.y;
-      z.y -= l.x * zq.y + l.y * zq.x;
-    }
-  }
-  float2 w = z;
-  for (int q = K - 1; q >= 0; --q) {
-    if (lane == q) w = make_float2(w.x * rl, w.y * rl);
-    const float2 wq = make_float2(__shfl_sync(0xffffffffu, w.x, q), __shfl_sync(0xffffffffu, w.y, q));
-    if (on && lane < q) {
-      const float2 l = M[q][lane];  // conj(L[q][lane]) * wq
-      w.x -= l.x * wq.x + l.y * wq.y;
-      w.y -= l.x * wq.y - l.y * wq.x;
-    }
-  }
-  EvalOut o;
-  o.dscale = dscale;
-  o.mean = make_float2(w.x * inv_d, w.y * inv_d);
-  // inverse factor column `lane`: X = L^{-1}, eq_var = sum_i |X[i][lane]|^2.
-  // Right-looking: when X[q][lane] is final, its contribution L[i][q] X[q]
-  // is added to the accumulators of every row i > q (held in X until row
-  // i is final) -- the same terms in the same order as the dot-product
-  // form, without its dependency chain.
-  float eqv = 0.f;
-  {
-    const float2(*__restrict__ L)[33] = M;
-    float2(*__restrict__ Xc)[33] = X;
-    if (on)
-      for (int i = 0; i < K; ++i) Xc[i][lane] = make_float2(0.f, 0.f);
-    float2 carry = make_float2(0.f, 0.f);  // Xc[q][lane], kept from step q-1
-    for (int q = 0; q < K; ++q) {
-      const float rlq = __shfl_sync(0xffffffffu, rl, q);
-      if (on && lane <= q) {
-        float2 xq;
-        if (lane == q) {
-          xq = make_float2(rlq, 0.f);
-        } else {
-          xq = make_float2(-carry.x * rlq, -carry.y * rlq);
+  float eqv[kPolishCols];
+#pragma unroll
+  for (int u = 0; u < kPolishCols; ++u) eqv[u] = 0.f;
+  int failed = 0;
+  auto post = [&](int q, float2& v) {
+    const float sdiag = __shfl_sync(0xffffffffu, v.x, q);
+    const float piv = sqrtf(sdiag > 0.f ? sdiag : kTinyP);
+    const float rq = 1.0f / piv;
+    const float2 a = make_float2(lane == q ? piv : lane > q ? v.x * rq : 0.f, lane > q ? v.y * rq : 0.f);
+    S.L[q][lane] = a;
+    S.rl[q] = rq;  // the same value from every lane
+    column_arrive(q);
+    v = make_float2(0.f, 0.f);
+    failed |= sdiag > 0.f ? 0 : isfinite(sdiag) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;
+  };
+  if (w == 0) post(0, r[0]);
+#pragma unroll
+  for (int uq = 0; uq < kPolishCols; ++uq) {
+#pragma unroll 1
+    for (int wq = 0; wq < kPolishWarps; ++wq) {
+      const int q = kPolishWarps * uq + wq;
+      if (q >= K) break;
+      if (w != wq) column_sync(q);
+      const float2 a = S.L[q][lane];  // column q: L[lane][q]
+      const float rlq = S.rl[q];
+      const int next = q + 1 < K ? q + 1 : -1;
+      if (wq + 1 < kPolishWarps) {
+        if (w == wq + 1 && next > 0) {
+          if (lane >= next) r[uq] = sub_mulc(r[uq], a, S.L[q][next]);
+          post(next, r[uq]);
         }
-        Xc[q][lane] = xq;
-        eqv += abs2(xq);
-        // batches of 8 rows: loads, arithmetic, stores (as the Cholesky)
-        for (int i0 = q + 1; i0 < K; i0 += 8) {
-          float2 l[8], acc[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (i0 + u < K) {
-              l[u] = L[i0 + u][q];
-              acc[u] = Xc[i0 + u][lane];
-            }
-#pragma unroll
-          for (int u = 0; u < 8; ++u)
-            if (i0 + u < K) {
-              acc[u].x += l[u].x * xq.x - l[u].y * xq.y;
-              acc[u].y += l[u].x * xq.y + l[u].y * xq.x;
-              Xc[i0 + u][lane] = acc[u];
-            }
-          if (i0 == q + 1) carry = acc[0];
+      } else if (uq + 1 < kPolishCols) {
+        if (w == 0 && next > 0) {
+          if (lane >= next) r[uq + 1] = sub_mulc(r[uq + 1], a, S.L[q][next]);
+          post(next, r[uq + 1]);
         }
       }
+      // the rest of the step, without branches: right of column q the
+      // system's update, else the inverse's (u == uq: by warp)
+#pragma unroll
+      for (int u = 0; u < kPolishCols; ++u) {
+        const int j = w + kPolishWarps * u;
+        const bool right = u > uq || (u == uq && w > wq);
+        float2 v = r[u];
+        if (u >= uq) {
+          const float2 t = sub_mulc(r[u], a, S.L[q][j]);
+          if (right && j != next && lane >= j) v = t;
+        }
+        if (u <= uq) {
+          float2 xq = make_float2(__shfl_sync(0xffffffffu, r[u].x, q), __shfl_sync(0xffffffffu, r[u].y, q));
+          xq = j == q ? make_float2(rlq, 0.f) : make_float2(-xq.x * rlq, -xq.y * rlq);
+          const float e = __fadd_rn(eqv[u], fmaf(xq.x, xq.x, __fmul_rn(xq.y, xq.y)));
+          const float2 t = add_mul(r[u], a, xq);
+          eqv[u] = right ? eqv[u] : e;
+          if (!right && lane > q) v = t;
+        }
+        r[u] = v;
+      }
+      const float2 zs = make_float2(z.x * rlq, z.y * rlq);
+      const float2 zq = make_float2(__shfl_sync(0xffffffffu, zs.x, q), __shfl_sync(0xffffffffu, zs.y, q));
+      const float2 zt = sub_mul(z, a, zq);
+      z = lane == q ? zs : lane > q ? zt : z;
     }
   }
-  __syncwarp();
-  o.pv = on ? fmaxf(eqv * (inv_d * inv_d), 0.f) : 0.f;
+  if (lane == 0) {
+#pragma unroll
+    for (int u = 0; u < kPolishCols; ++u) S.eqv[w + kPolishWarps * u] = eqv[u];
+  }
+  if (failed && lane == 0) atomicOr(&S.status, failed);
+  // warp 7: L^H w = z, mu = w / d; warps 0-3 the evidence's logarithms
+  if (w == kPolishWarps - 1) {
+    const float rl = on ? S.rl[lane] : 1.0f;
+    float2 v = z;
+#pragma unroll 1
+    for (int q0 = kMaxPolish - 8; q0 >= 0; q0 -= 8) {
+      float2 l[8];  // L[q][lane], ahead of the chain
+#pragma unroll
+      for (int i = 0; i < 8; ++i) l[i] = S.L[lane][q0 + i];
+#pragma unroll
+      for (int i = 7; i >= 0; --i) {
+        const int q = q0 + i;
+        if (lane == q) v = make_float2(v.x * rl, v.y * rl);
+        const float2 vq = make_float2(__shfl_sync(0xffffffffu, v.x, q), __shfl_sync(0xffffffffu, v.y, q));
+        if (lane < q && q < K) v = sub_cmul(v, l[i], vq);
+      }
+    }
+    S.mean[lane] = make_float2(v.x * inv_d, v.y * inv_d);
+  } else if (w == 0) {
+    S.ev[0][lane] = on ? log(static_cast<double>(fmaxf(S.L[lane][lane].x, kTinyP))) : 0.0;
+  } else if (w == 1) {
+    S.ev[1][lane] = on ? log(static_cast<double>(dscale)) : 0.0;
+  } else if (w == 2) {
+    S.ev[2][lane] = on ? log(static_cast<double>(my_gamma)) : 0.0;
+  } else if (w == 3) {
+    const double l = log(static_cast<double>(nu));
+    if (lane == 0) S.log_nu = l;
+  }
+  __syncthreads();
+  EvalOut o;
+  o.dscale = dscale;
+  o.mean = on ? S.mean[lane] : make_float2(0.f, 0.f);
+  o.pv = on ? fmaxf(S.eqv[lane] * (inv_d * inv_d), 0.f) : 0.f;
   o.dd = on ? fmaxf((my_gamma - o.pv) * (inv_g * inv_g), 0.f) : 0.f;
   // evidence (FP64 accumulation)
-  double ld = 0.0, lg = 0.0, qd = 0.0;
-  if (on) {
-    ld = log(static_cast<double>(fmaxf(M[lane][lane].x, kTinyP))) + log(static_cast<double>(dscale));
-    lg = log(static_cast<double>(my_gamma));
-    qd = static_cast<double>(rhs.x) * o.mean.x + static_cast<double>(rhs.y) * o.mean.y;
-  }
+  double ld = S.ev[0][lane] + S.ev[1][lane], lg = S.ev[2][lane];
+  double qd = on ? static_cast<double>(rhs.x) * o.mean.x + static_cast<double>(rhs.y) * o.mean.y : 0.0;
   ld = warp_sum(ld);
   lg = warp_sum(lg);
   qd = warp_sum(qd);
-  const double logdet = observed_samples(s, A.c) * log(static_cast<double>(nu)) + lg + 2.0 * ld;
+  const double logdet = observed_samples(s, A.c) * S.log_nu + lg + 2.0 * ld;
   double quad = static_cast<double>(data_energy) / nu - qd;
   if (quad < 0.0) quad = 0.0;
   o.nle = logdet + quad;
-  if (!isfinite(o.nle)) status |= FBME_STATUS_NONFINITE;
-  o.status = status;
+  if (!isfinite(o.nle) && threadIdx.x == 0) atomicOr(&S.status, FBME_STATUS_NONFINITE);
   return o;
 }
 
-// ||y - A_S mu||^2 by the Gram identity, FP64.
-FBME_DEV double residual_energy(const PolishArgs& A, const float2* d1, const float2* d2, int K,
+// ||y - A_S mu||^2 by the Gram identity, FP64, on the whole block (every
+// warp returns the sum): warp w adds the columns j = w, w + 8, ... of G mu.
+FBME_DEV double residual_energy(const PolishArgs& A, PolishShared& S, const float2* d1, const float2* d2, int K,
                                 int my_idx, float2 my_mu, float2 my_c, float data_energy) {
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const BatchShape& s = A.s;
-  double cross = 0.0, quad = 0.0;
-  if (lane < K) {
-    cross = static_cast<double>(my_c.x) * my_mu.x + static_cast<double>(my_c.y) * my_mu.y;
-    const int n1i = my_idx / s.n2, n2i = my_idx % s.n2;
-    double gr = 0.0, gi = 0.0;  // (G mu)_i
-    // unrolled: the shuffles and Gram entries of later j issue ahead of the
-    // FP64 sums, which still run in the order j = 0, 1, ...
-    const unsigned am = __activemask();
-#pragma unroll 8
-    for (int j = 0; j < K; ++j) {
-      const int n1j = __shfl_sync(am, n1i, j), n2j = __shfl_sync(am, n2i, j);
-      const float mjx = __shfl_sync(am, my_mu.x, j);
-      const float mjy = __shfl_sync(am, my_mu.y, j);
+  const int n1i = my_idx / s.n2, n2i = my_idx % s.n2;
+  double gr = 0.0, gi = 0.0;  // (G mu)_i
+#pragma unroll
+  for (int u = 0; u < kPolishCols; ++u) {
+    const int j = w + kPolishWarps * u;
+    const int n1j = __shfl_sync(0xffffffffu, n1i, j), n2j = __shfl_sync(0xffffffffu, n2i, j);
+    const float mjx = __shfl_sync(0xffffffffu, my_mu.x, j);
+    const float mjy = __shfl_sync(0xffffffffu, my_mu.y, j);
+    if (lane < K && j < K) {
       const float2 g = gram_at(A, d1, d2, n1i, n2i, n1j, n2j);
       gr += static_cast<double>(g.x) * mjx - static_cast<double>(g.y) * mjy;
       gi += static_cast<double>(g.x) * mjy + static_cast<double>(g.y) * mjx;
+    }
+  }
+  __syncthreads();  // an earlier call's sums have been read
+  S.gm[w][lane] = make_double2(gr, gi);
+  __syncthreads();
+  double cross = 0.0, quad = 0.0;
+  if (lane < K) {
+    cross = static_cast<double>(my_c.x) * my_mu.x + static_cast<double>(my_c.y) * my_mu.y;
+    gr = gi = 0.0;
+#pragma unroll
+    for (int v = 0; v < kPolishWarps; ++v) {
+      const double2 t = S.gm[v][lane];
+      gr += t.x;
+      gi += t.y;
     }
     quad = my_mu.x * gr + my_mu.y * gi;  // Re(conj(mu_i) (G mu)_i)
   }
@@ -382,16 +403,14 @@ FBME_DEV int warp_sort_desc(float val, int pos, float* out_val) {
   return pos;
 }
 
-constexpr int kPolishWarps = 1;
-
-// Evaluations p in [state.evals, P) until done or an exchange is needed.
-// phase 0: initialise from the top-K; phase 1: apply the exchange whose
-// candidates are in p.xcand_*, then continue.
-FBME_DEV void polish_body(const PolishArgs& A, int phase, int scene) {
-  __shared__ float2 Msm[kPolishWarps][32][33];
-  __shared__ float2 Xsm[kPolishWarps][32][33];
+// Evaluations p in [state.evals, P) until done or an exchange is needed,
+// one block per scene.  phase 0: initialise from the top-K; phase 1: apply
+// the exchange whose candidates are in p.xcand_*, then continue.  Every
+// warp holds the same lane values (active set, variances, best model), so
+// the decisions need no broadcast; warp 0 writes the state.
+FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int scene) {
   extern __shared__ float2 dtab[];  // D1 (n1) then D2 (n2)
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (scene >= A.s.B) return;
   const BatchShape& s = A.s;
   const DevConfig& c = A.c;
@@ -403,42 +422,48 @@ FBME_DEV void polish_body(const PolishArgs& A, int phase, int scene) {
   const float Mf = static_cast<float>(observed_samples(s, c));
   const long long N = s.n();
   const float2* bp = A.p.bp + scene * N;
-  float2(*M)[33] = Msm[threadIdx.x >> 5];
-  float2(*X)[33] = Xsm[threadIdx.x >> 5];
   float2* d1 = dtab;
   float2* d2 = dtab + s.n1;
-  load_dirichlet(A, d1, d2);
-  int status = 0;
+  if (threadIdx.x == 0) S.status = 0;
 
+  // the work set of the next evaluation and the best model so far
+  int idx = 0, bidx = 0, pending = 0, exch_acc = 0, has_best = 0, evals = 0;
+  float gam = 1.0f, nu = 0.f, bnoise = 0.f, bpv = 0.f, bdd = 0.f, bg = 1.0f;
+  float2 bmu = make_float2(0.f, 0.f);
+  double best_nle = 0.0;
   if (phase == 0) {
     // prune + reinitialise (solver.py:4087-4106)
     if (on) {
-      const int idx = A.p.active[scene * K + lane];
-      ps->work_active[lane] = idx;
+      idx = A.p.active[scene * K + lane];
       const float g0 = A.p.gamma[scene * N + idx];
-      ps->work_gamma[lane] = c.reinit ? fmaxf(A.p.score[scene * K + lane], fl) : g0;
+      gam = c.reinit ? fmaxf(A.p.score[scene * K + lane], fl) : g0;
     }
-    if (lane == 0) {
-      ps->work_noise = A.p.sc.noise[scene];
-      ps->evals = 0;
-      ps->pending = 0;
-      ps->exch_acc = 0;
-      ps->has_best = 0;
-    }
-    __syncwarp();
+    nu = A.p.sc.noise[scene];
+    load_dirichlet(A, d1, d2);
   } else {
+    evals = ps->evals;
+    has_best = ps->has_best;
+    exch_acc = ps->exch_acc;
+    nu = ps->work_noise;
+    bnoise = ps->best_noise;
+    best_nle = ps->best_nle;
+    if (on) {
+      idx = ps->work_active[lane];
+      gam = ps->work_gamma[lane];
+      bidx = ps->active[lane];
+      bmu = ps->best_mean[lane];
+      bpv = ps->best_pv[lane];
+      bdd = ps->best_dd[lane];
+      bg = ps->best_gamma[lane];
+    }
+    load_dirichlet(A, d1, d2);
     // residual support exchange (solver.py:4397-4494), using the best
     // state after evaluation 0 as the base.
     const int E = c.exchange;
-    const float2 mu = on ? ps->best_mean[lane] : make_float2(0.f, 0.f);
-    const float pv = on ? ps->best_pv[lane] : 0.f;
-    const float g = on ? ps->best_gamma[lane] : 0.f;
-    const float base_noise = ps->best_noise;
-    const float del = on ? deletion_gain(mu, pv, g) : -INFINITY;
+    const float del = on ? deletion_gain(bmu, bpv, bg) : -INFINITY;
     float sval;
-    const int spos = warp_sort_desc(on ? del : -INFINITY, on ? lane : 0x7fffffff, &sval);
-    // lane r < E: removal position spos, addition candidate r
-    const int rem_pos = spos;
+    const int rem_pos = warp_sort_desc(on ? del : -INFINITY, on ? lane : 0x7fffffff, &sval);
+    // lane r < E: removal position rem_pos, addition candidate r
     int repl_idx = -1;
     float repl_gamma = 0.f;
     int xmask = 0;
@@ -446,10 +471,10 @@ FBME_DEV void polish_body(const PolishArgs& A, int phase, int scene) {
       const float add_e = A.p.xcand_val[scene * E + lane];
       const int add_i = A.p.xcand_idx[scene * E + lane];
       const float ce = Mf;
-      const float ratio = add_e / fmaxf(base_noise * ce, kTinyP);
+      const float ratio = add_e / fmaxf(bnoise * ce, kTinyP);
       const float add_gain = ratio > 1.0f ? ratio - 1.0f - logf(fmaxf(ratio, kTinyP)) : 0.0f;
       xmask = (add_gain + sval) > 0.0f;
-      float ag = fmaxf(add_e - base_noise * ce, 0.0f) / (ce * ce);
+      float ag = fmaxf(add_e - bnoise * ce, 0.0f) / (ce * ce);
       ag = fminf(fmaxf(ag, fl), c.max_prec);
       repl_idx = add_i;
       repl_gamma = ag;
@@ -461,68 +486,45 @@ FBME_DEV void polish_body(const PolishArgs& A, int phase, int scene) {
       const int ri = __shfl_sync(0xffffffffu, repl_idx, r);
       const float rg = __shfl_sync(0xffffffffu, repl_gamma, r);
       if (xm && lane == pr) {
-        ps->work_active[lane] = ri;
-        ps->work_gamma[lane] = rg;
+        idx = ri;
+        gam = rg;
       }
     }
-    const int any = __any_sync(0xffffffffu, xmask != 0);
-    if (lane == 0) ps->pending = any;
-    __syncwarp();
+    pending = __any_sync(0xffffffffu, xmask != 0);
   }
 
   const int P = c.polish_iters;
-  for (int p = ps->evals; p < P; ++p) {
-    const int idx = on ? ps->work_active[lane] : 0;
-    const float gam = on ? ps->work_gamma[lane] : 1.0f;
-    const float nu = ps->work_noise;
+  for (int p = evals; p < P; ++p) {
     const float2 cvec = on ? bp[idx] : make_float2(0.f, 0.f);
-    const EvalOut o = evaluate(A, M, X, d1, d2, K, idx, gam, nu, cvec, data_energy);
-    status |= o.status;
+    const EvalOut o = evaluate(A, S, d1, d2, K, idx, gam, nu, cvec, data_energy);
     // evidence gate (solver.py:4168-4298)
     bool accept = true;
-    if (c.gate && ps->has_best) {
-      const double best = ps->best_nle;
+    if (c.gate && has_best) {
       const double margin = static_cast<double>(c.margin_factor) * kEpsP *
-                            (1.0 + fabs(o.nle) + fabs(best));
-      accept = isfinite(o.nle) && (!isfinite(best) || o.nle <= best - margin);
-    }
-    __syncwarp();
-    if (lane == 0) {
-      if (c.gate && ps->has_best && ps->pending && accept) ps->exch_acc += 1;
-      if (c.gate && ps->has_best) ps->pending = 0;
+                            (1.0 + fabs(o.nle) + fabs(best_nle));
+      accept = isfinite(o.nle) && (!isfinite(best_nle) || o.nle <= best_nle - margin);
+      if (pending && accept) exch_acc += 1;
+      pending = 0;
     }
     if (accept) {
-      if (on) {
-        ps->active[lane] = idx;
-        ps->best_mean[lane] = o.mean;
-        ps->best_pv[lane] = o.pv;
-        ps->best_dd[lane] = o.dd;
-        ps->best_gamma[lane] = gam;
-      }
-      if (lane == 0) {
-        ps->best_noise = nu;
-        ps->best_nle = o.nle;
-        ps->has_best = 1;
-      }
+      bidx = idx;
+      bmu = o.mean;
+      bpv = o.pv;
+      bdd = o.dd;
+      bg = gam;
+      bnoise = nu;
+      best_nle = o.nle;
+      has_best = 1;
     }
-    __syncwarp();
-    if (lane == 0) {
-      ps->trace[p] = static_cast<float>(ps->best_nle);
-      ps->evals = p + 1;
-    }
-    __syncwarp();
+    if (threadIdx.x == 0) ps->trace[p] = static_cast<float>(best_nle);
+    evals = p + 1;
     if (p + 1 == P) break;
     // EM between evaluations (solver.py:4320-4391), from the best state
-    const int bidx = on ? ps->active[lane] : 0;
-    const float2 bmu = on ? ps->best_mean[lane] : make_float2(0.f, 0.f);
-    const float bpv = on ? ps->best_pv[lane] : 0.f;
-    const float bg = on ? ps->best_gamma[lane] : 1.0f;
-    const float bnoise = ps->best_noise;
-    float ng = fminf(fmaxf(abs_sq(bmu) + bpv, fl), c.max_prec);
+    const float ng = fminf(fmaxf(abs_sq(bmu) + bpv, fl), c.max_prec);
     const float keep = c.polish_damping;
     const float upd_g = keep * bg + (1.0f - keep) * ng;
     const float2 bc = on ? bp[bidx] : make_float2(0.f, 0.f);
-    const double er = residual_energy(A, d1, d2, K, bidx, bmu, bc, data_energy);
+    const double er = residual_energy(A, S, d1, d2, K, bidx, bmu, bc, data_energy);
     float dof = on ? fminf(fmaxf(1.0f - bpv / fmaxf(bg, kTinyP), 0.f), 1.f) : 0.f;
     dof = warp_sum(dof);
     float un;
@@ -536,20 +538,38 @@ FBME_DEV void polish_body(const PolishArgs& A, int phase, int scene) {
                               fmax(static_cast<double>(Mf) - dof + c.noise_shape, kEpsP));
     }
     un = fmaxf(un, fl);
-    const float new_noise = c.fixed_noise > 0.f ? un : keep * bnoise + (1.0f - keep) * un;
-    if (on) {
-      ps->work_active[lane] = bidx;
-      ps->work_gamma[lane] = upd_g;
-    }
-    if (lane == 0) ps->work_noise = new_noise;
-    __syncwarp();
+    nu = c.fixed_noise > 0.f ? un : keep * bnoise + (1.0f - keep) * un;
+    idx = bidx;
+    gam = upd_g;
     const int E = c.exchange;
     if (E > 0 && p == 0) break;  // exchange candidates are scored over the grid next
   }
-  if (status && lane == 0) atomicOr(&A.p.status[scene], status);
+  if (w == 0) {
+    if (on) {
+      ps->active[lane] = bidx;
+      ps->best_mean[lane] = bmu;
+      ps->best_pv[lane] = bpv;
+      ps->best_dd[lane] = bdd;
+      ps->best_gamma[lane] = bg;
+      ps->work_active[lane] = idx;
+      ps->work_gamma[lane] = gam;
+    }
+    if (lane == 0) {
+      ps->best_noise = bnoise;
+      ps->best_nle = best_nle;
+      ps->has_best = has_best;
+      ps->work_noise = nu;
+      ps->evals = evals;
+      ps->pending = pending;
+      ps->exch_acc = exch_acc;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && S.status) atomicOr(&A.p.status[scene], S.status);
 }
-__global__ void __launch_bounds__(32 * kPolishWarps) polish_kernel(PolishArgs A, int phase) {
-  polish_body(A, phase, blockIdx.x * kPolishWarps + (threadIdx.x >> 5));
+__global__ void __launch_bounds__(kPolishThreads) polish_kernel(PolishArgs A, int phase) {
+  __shared__ PolishShared S;
+  polish_body(A, S, phase, blockIdx.x);
 }
 
 // Residual exchange scoring (solver.py:4398-4412) without the M-space
@@ -744,7 +764,7 @@ using ExWidest = ExTile<4, 8, 64, 256, 512>;
 
 // Final K-space outputs, fixed-budget diagnostics, effective DOF
 // (solver.py:1989-2021, 2081-2092, 3408-3496, 2108-2126).
-FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, int scene) {
+FBME_DEV void polish_finish_body(const PolishArgs& A, PolishShared& S, const FbmeOutputs& out, int scene) {
   extern __shared__ float2 dtab[];
   const int lane = threadIdx.x & 31;
   if (scene >= A.s.B) return;
@@ -772,7 +792,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, in
   const float max_dof = static_cast<float>(observed_samples(s, c) * (1.0 - 10.0 * kEpsP));
   const float sc = fminf(1.0f, max_dof / fmaxf(raw, kEpsP));
   const float dof = warp_sum(rel * sc);
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     out.noise_variance[scene] = nu;
     out.effective_dof[scene] = dof;
     out.negative_log_evidence[scene] = static_cast<float>(ps->best_nle);
@@ -784,7 +804,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, in
       out.support_score_threshold[scene] =
           static_cast<float>(log(static_cast<double>(N) / static_cast<double>(c.false_alarm)));
   }
-  if (on && out.active_indices) out.active_indices[scene * K + lane] = idx;
+  if (threadIdx.x < K && out.active_indices) out.active_indices[scene * K + lane] = idx;
   if (c.fixed_budget && out.fixed_budget_gamma_residual) {
     const float ag = fmaxf(g, kTinyP);
     const float gt = fminf(fmaxf(abs_sq(mu) + pv, fl), c.max_prec);
@@ -793,7 +813,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, in
     float dofd = on ? fminf(fmaxf(1.0f - pv / ag, 0.f), 1.f) : 0.f;
     dofd = warp_sum(dofd);
     const float2 cv = on ? A.p.bp[scene * N + idx] : make_float2(0.f, 0.f);
-    const double er = residual_energy(A, d1, d2, K, idx, mu, cv, A.p.sc.data_energy[scene]);
+    const double er = residual_energy(A, S, d1, d2, K, idx, mu, cv, A.p.sc.data_energy[scene]);
     float nt;
     if (c.fixed_noise > 0.f) {
       nt = nu;
@@ -806,7 +826,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, in
     }
     nt = fminf(fmaxf(nt, fl), c.max_prec);
     const float ns = fmaxf(fmaxf(fabsf(nu), fabsf(nt)), kTinyP);
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       out.fixed_budget_gamma_residual[scene] = gr;
       out.fixed_budget_noise_residual[scene] = c.fixed_noise > 0.f ? 0.f : fabsf(nu - nt) / ns;
       bool fin = true, mono = true;
@@ -817,8 +837,9 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, const FbmeOutputs& out, in
     }
   }
 }
-__global__ void __launch_bounds__(32) polish_finish_kernel(PolishArgs A, FbmeOutputs out) {
-  polish_finish_body(A, out, blockIdx.x);
+__global__ void __launch_bounds__(kPolishThreads) polish_finish_kernel(PolishArgs A, FbmeOutputs out) {
+  __shared__ PolishShared S;
+  polish_finish_body(A, S, out, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1036,25 +1057,25 @@ FBME_DEV CertBest* cert_parts(void* ws, int B, int scene) {
          kCertMaxBlocks;
 }
 
-// Warp 0 of a step: evaluate the work set (idx, gam) and stage its factor
-// and active set for the scan.
-FBME_DEV EvalOut cert_model(const PolishArgs& A, CertScratch* cs, float2 (*M)[33], float2 (*X)[33],
-                            const float2* d1, const float2* d2, int idx, float gam, float nu, const float2* bp,
-                            float data_energy) {
-  const int lane = threadIdx.x & 31;
+// Evaluate the work set (idx, gam) on the block and stage its factor and
+// active set for the scan.
+FBME_DEV EvalOut cert_model(const PolishArgs& A, CertScratch* cs, PolishShared& S, const float2* d1,
+                            const float2* d2, int idx, float gam, float nu, const float2* bp, float data_energy) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int K = A.c.polish_size;
   const bool on = lane < K;
-  const EvalOut o = evaluate(A, M, X, d1, d2, K, idx, gam, nu, on ? bp[idx] : make_float2(0.f, 0.f), data_energy);
-  if (on) {
-    for (int k = 0; k < lane; ++k) cs->L[lane][k] = M[lane][k];
+  const EvalOut o = evaluate(A, S, d1, d2, K, idx, gam, nu, on ? bp[idx] : make_float2(0.f, 0.f), data_energy);
+  if (on)
+    for (int k = w; k < lane; k += kPolishWarps) cs->L[lane][k] = S.L[k][lane];
+  if (on && w == 0) {
     cs->m.idx[lane] = idx;
     cs->m.a1[lane] = idx / A.s.n2;
     cs->m.a2[lane] = idx % A.s.n2;
     cs->m.mu[lane] = o.mean;
     cs->m.inv_d[lane] = 1.0f / o.dscale;
-    cs->m.inv_l[lane] = 1.0f / M[lane][lane].x;
+    cs->m.inv_l[lane] = 1.0f / S.L[lane][lane].x;
   }
-  if (lane == 0) cs->nu_bits = __float_as_int(nu);
+  if (threadIdx.x == 0) cs->nu_bits = __float_as_int(nu);
   return o;
 }
 
@@ -1067,7 +1088,7 @@ FBME_DEV CertBest cert_merge(void* ws, int B, int scene, int nblk) {
   return cert_warp_best(b);
 }
 
-// One certificate step of one scene (one warp).  Step 0 stages the model
+// One certificate step of one scene (one block; warp 0 writes the state).  Step 0 stages the model
 // the polish kept.  Step t in [1, R] merges the previous scan (the kept
 // model's certificate at t = 1; otherwise repair t-1's certificate and its
 // decision: kept when the inactive ratio that proposed it exceeds 1 and
@@ -1075,10 +1096,9 @@ FBME_DEV CertBest cert_merge(void* ws, int B, int scene, int nblk) {
 // atom replaces the active atom of largest deletion delta, with variance
 // max(optimal, floor).  Step R + 1 merges the last scan and writes the
 // final certificate (solver.py:4851-4870, 5388-5460).
-__global__ void __launch_bounds__(32) cert_step_kernel(PolishArgs A, FbmeCertificate C, void* ws, int nblk,
-                                                       int t) {
-  __shared__ float2 M[32][33];
-  __shared__ float2 X[32][33];
+__global__ void __launch_bounds__(kPolishThreads) cert_step_kernel(PolishArgs A, FbmeCertificate C, void* ws,
+                                                                   int nblk, int t) {
+  __shared__ PolishShared S;
   extern __shared__ float2 dtab[];
   const int scene = blockIdx.x;
   if (scene >= A.s.B) return;
@@ -1094,34 +1114,36 @@ __global__ void __launch_bounds__(32) cert_step_kernel(PolishArgs A, FbmeCertifi
   const float fl = A.p.sc.floor_[scene];
   const float data_energy = A.p.sc.data_energy[scene];
   const float nu = ps->best_noise;
-  int status = 0;
+  if (threadIdx.x == 0) S.status = 0;
   if (t > 0) {
-    const CertState next = cert_state(cert_merge(ws, s.B, scene, nblk));
-    bool keep = true;
-    if (cs->pending) {  // decide the repair the scan certified
-      const CertState prop = cs->cur;
-      const double nle = cs->p_nle;
-      keep = prop.ratio > 1.0f && isfinite(nle) && static_cast<float>(nle) <= static_cast<float>(ps->best_nle);
-      __syncwarp();
-      if (keep) {
-        if (on) {
-          ps->active[lane] = cs->p_idx[lane];
-          ps->best_mean[lane] = cs->p_mean[lane];
-          ps->best_pv[lane] = cs->p_pv[lane];
-          ps->best_dd[lane] = cs->p_dd[lane];
-          ps->best_gamma[lane] = cs->p_gam[lane];
+    if (threadIdx.x < 32) {
+      const CertState next = cert_state(cert_merge(ws, s.B, scene, nblk));
+      bool keep = true;
+      if (cs->pending) {  // decide the repair the scan certified
+        const CertState prop = cs->cur;
+        const double nle = cs->p_nle;
+        keep = prop.ratio > 1.0f && isfinite(nle) && static_cast<float>(nle) <= static_cast<float>(ps->best_nle);
+        __syncwarp();
+        if (keep) {
+          if (on) {
+            ps->active[lane] = cs->p_idx[lane];
+            ps->best_mean[lane] = cs->p_mean[lane];
+            ps->best_pv[lane] = cs->p_pv[lane];
+            ps->best_dd[lane] = cs->p_dd[lane];
+            ps->best_gamma[lane] = cs->p_gam[lane];
+          }
+          if (lane == 0) {
+            ps->best_nle = nle;
+            ps->exch_acc += 1;
+          }
         }
-        if (lane == 0) {
-          ps->best_nle = nle;
-          ps->exch_acc += 1;
-        }
+        __syncwarp();
+        if (lane == 0) ps->trace[P + t - 2] = static_cast<float>(ps->best_nle);
       }
       __syncwarp();
-      if (lane == 0) ps->trace[P + t - 2] = static_cast<float>(ps->best_nle);
+      if (lane == 0 && keep) cs->cur = next;
     }
-    __syncwarp();
-    if (lane == 0 && keep) cs->cur = next;
-    __syncwarp();
+    __syncthreads();
   }
   if (t <= R) {
     float2* d1 = dtab;
@@ -1140,16 +1162,15 @@ __global__ void __launch_bounds__(32) cert_step_kernel(PolishArgs A, FbmeCertifi
         gam = fmaxf(cur.optvar, fl);
       }
     }
-    const EvalOut o = cert_model(A, cs, M, X, d1, d2, idx, gam, nu, bp, data_energy);
-    status |= o.status;
-    if (on) {
+    const EvalOut o = cert_model(A, cs, S, d1, d2, idx, gam, nu, bp, data_energy);
+    if (threadIdx.x < K) {
       cs->p_idx[lane] = idx;
       cs->p_gam[lane] = gam;
       cs->p_mean[lane] = o.mean;
       cs->p_pv[lane] = o.pv;
       cs->p_dd[lane] = o.dd;
     }
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       cs->p_nle = o.nle;
       cs->pending = t > 0;
     }
@@ -1166,7 +1187,7 @@ __global__ void __launch_bounds__(32) cert_step_kernel(PolishArgs A, FbmeCertifi
     warp_argmax(on ? at.current : -INFINITY, &max_del);
     const int best_idx = __shfl_sync(0xffffffffu, idx, gp);
     const float best_var = __shfl_sync(0xffffffffu, at.optvar, gp);
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
       const CertState cur = cs->cur;
       const float tol = C.coordinate_tolerance;
       const float pen = fmaxf(max_nondel, fmaxf(max_del, 0.f));
@@ -1186,8 +1207,8 @@ __global__ void __launch_bounds__(32) cert_step_kernel(PolishArgs A, FbmeCertifi
         C.familywise_no_discovery[scene] = cur.ratio <= C.familywise_ratio_threshold;
     }
   }
-  status = __reduce_or_sync(0xffffffffu, status);
-  if (status && lane == 0) atomicOr(&A.p.status[scene], status);
+  __syncthreads();
+  if (threadIdx.x == 0 && S.status) atomicOr(&A.p.status[scene], S.status);
 }
 
 // Block (bx, scene) scores atoms [bx chunk, (bx + 1) chunk) against the
@@ -1290,10 +1311,11 @@ static_assert(sizeof(PolishSet) <= 32764, "kernel parameter limit");
 
 FBME_DEV bool has_exchange(const DevConfig& c) { return c.exchange > 0 && c.polish_iters > 1; }
 
-__global__ void __launch_bounds__(32 * kPolishWarps) polish_set_kernel(const PolishSet S, int phase) {
-  const PolishArgs& A = S.a[blockIdx.z];
+__global__ void __launch_bounds__(kPolishThreads) polish_set_kernel(const PolishSet set, int phase) {
+  __shared__ PolishShared S;
+  const PolishArgs& A = set.a[blockIdx.z];
   if (phase == 1 && !has_exchange(A.c)) return;
-  polish_body(A, phase, blockIdx.x * kPolishWarps + (threadIdx.x >> 5));
+  polish_body(A, S, phase, blockIdx.x);
 }
 
 template <typename T>
@@ -1304,8 +1326,9 @@ __global__ void __launch_bounds__(T::threads, 2) exchange_set_kernel(const Polis
   exchange_body<T>(A, A.p.cand_key, A.p.cand_idx, blockIdx.y, blockIdx.x, nbx);
 }
 
-__global__ void __launch_bounds__(32) polish_finish_set_kernel(const PolishSet S) {
-  polish_finish_body(S.a[blockIdx.z], S.out[blockIdx.z], blockIdx.x);
+__global__ void __launch_bounds__(kPolishThreads) polish_finish_set_kernel(const PolishSet set) {
+  __shared__ PolishShared S;
+  polish_finish_body(set.a[blockIdx.z], S, set.out[blockIdx.z], blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256) output_set_kernel(const PolishSet S) {
@@ -1393,7 +1416,7 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
   FBME_TIMED(prof, FBME_GROUP_TOPK,
              launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * K, K, s.B, p.active, p.score, st));
   const size_t dsm = (s.n1 + s.n2) * sizeof(float2);
-  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, 32, dsm, st>>>(A, 0)));
+  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 0)));
   if (c.exchange > 0 && c.polish_iters > 1 && p.gram2d) {
     const long long nblk = (s.n() + 255) / 256;
     FBME_TIMED(prof, FBME_GROUP_EXCHANGE,
@@ -1403,7 +1426,7 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * c.exchange, c.exchange, s.B,
                                  p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, 32, dsm, st>>>(A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 1)));
   } else if (c.exchange > 0 && c.polish_iters > 1) {
     const int nb = exchange_blocks(s);
     if (s.n2 <= 64)
@@ -1417,7 +1440,7 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_merge(p.cand_key, p.cand_idx, nb * c.exchange, c.exchange, s.B,
                                  p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, 32, dsm, st>>>(A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 1)));
   }
   if (cert) {  // model, scan, (decide + model, scan) per repair, final
     int resident = 1;
@@ -1427,13 +1450,13 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     const int nblk = cert_blocks(s, resident);
     for (int t = 0; t <= c.repairs + 1; ++t) {
       FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
-                 (cert_step_kernel<<<s.B, 32, dsm, st>>>(A, *cert, cert->workspace, nblk, t)));
+                 (cert_step_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, *cert, cert->workspace, nblk, t)));
       if (t <= c.repairs)
         FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
                    (cert_scan_kernel<<<dim3(nblk, s.B), kCertThreads, dsm, st>>>(A, cert->workspace)));
     }
   }
-  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_finish_kernel<<<s.B, 32, dsm, st>>>(A, out)));
+  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_finish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, out)));
   const int fb = static_cast<int>((s.n() + 2047) / 2048);
   FBME_TIMED(prof, FBME_GROUP_OUTPUT, (output_kernel<<<dim3(fb < 64 ? fb : 64, s.B), 256, 0, st>>>(A, out)));
 }
@@ -1488,8 +1511,7 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
     }
     launch_topk_blocks_multi(tj, max_slices, max_b, st);
     launch_topk_merge_multi(tm, max_b, st);
-    const int pb = (max_b + kPolishWarps - 1) / kPolishWarps;
-    polish_set_kernel<<<dim3(pb, 1, m), 32 * kPolishWarps, dsm, st>>>(*S, 0);
+    polish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S, 0);
     // the exchange, one launch per row-tile class, then its candidates' merge
     bool any = false;
     for (int cls = 0; cls < 4; ++cls) {
@@ -1525,9 +1547,9 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
                                     A.p.xcand_val};
       }
       launch_topk_merge_multi(tx, max_b, st);
-      polish_set_kernel<<<dim3(pb, 1, m), 32 * kPolishWarps, dsm, st>>>(*S, 1);
+      polish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S, 1);
     }
-    polish_finish_set_kernel<<<dim3(max_b, 1, m), 32, dsm, st>>>(*S);
+    polish_finish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S);
     output_set_kernel<<<dim3(max_out, max_b, m), 256, 0, st>>>(*S);
     for (int i = 0; i < m; ++i) {
       const PolishBucket& k = b[plain[i]];
