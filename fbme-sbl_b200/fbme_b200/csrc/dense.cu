@@ -6,10 +6,10 @@
 //             d in (-(M1-1)..M1-1) x (-(M2-1)..M2-1), separable (two passes)
 //   Q         Q[i][j] = L(m_i - m_j) + noise delta_ij, plus the deterministic
 //             loading of the CUDA Cholesky branch (m * eps64 * mean|diag|)
-//   Cholesky  blocked right-looking, 32-column panels (one CTA per scene)
-//             and 64 x 64 tiles of the trailing update (the whole GPU)
-//   L^-1      blocked forward substitution on the identity, same split
-//   Q^-1      = L^-H L^-1 (lower tiles, over the rows below each tile)
+//   Q^-1      in place by blocked symmetric sweeps: 32-column panels, each
+//             step one Hermitian rank-32 update of the whole lower triangle
+//             that advances the Cholesky factor's trailing matrix, L^-1 and
+//             L^-H L^-1 together (dense_sweep_kernel)
 //   Q^-1 y, the lag sums of Q^-1 and the data diagonal
 //             diag(A^H Q^-1 A) = Re N ifft2(lag sums); A^H Q^-1 y; the
 //             residual energy from the identity y - A mean = (noise +
@@ -36,9 +36,10 @@ namespace {
 // (solver.py:2907-2920) takes eps of the arithmetic's precision: FP64 here,
 // as the reference's complex128 path does.
 constexpr double kEps64 = 2.220446049250313e-16;
-constexpr int kPanel = 32;   // Cholesky / inverse panel width
+constexpr int kPanel = 32;   // panel width of the sweeps
+constexpr int kDiagWarps = 8;
+constexpr int kDiagCols = kPanel / kDiagWarps;
 constexpr int kTile = 64;    // output tile of the update kernels
-constexpr int kDk = 16;      // depth chunk of the update kernels
 
 __device__ __forceinline__ double2 zadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
@@ -57,13 +58,25 @@ __global__ void dense_twiddle_kernel(double2* tw, int L) {
   tw[k] = make_double2(c, s);
 }
 
-// w^(sign * e) from the table of w = exp(-2 pi i / L), e any integer
-__device__ __forceinline__ double2 twid(const double2* tw, int L, long long e, int sign) {
-  long long r = e % L;
-  if (r < 0) r += L;
-  const double2 w = tw[r];
-  return sign < 0 ? w : make_double2(w.x, -w.y);
-}
+// w^(sign e) for e = e0, e0 + step, e0 + 2 step, ... from the table of
+// w = exp(-2 pi i / L): the exponent is kept reduced, one compare and
+// subtract a term instead of a 64-bit remainder.
+struct TwidStep {
+  const double2* tw;
+  int L, e, step;
+  __device__ TwidStep(const double2* t, int len, long long e0, long long s)
+      : tw(t), L(len), e(reduce(e0, len)), step(reduce(s, len)) {}
+  static __device__ int reduce(long long v, int len) {
+    const int r = static_cast<int>(v % len);
+    return r < 0 ? r + len : r;
+  }
+  __device__ double2 next(int sign) {
+    const double2 w = tw[e];
+    e += step;
+    if (e >= L) e -= L;
+    return sign < 0 ? w : make_double2(w.x, -w.y);
+  }
+};
 
 // Lag pass 1: T[b][n1][e2] = sum_n2 gamma[b][n1][n2] w2^(d2 n2), d2 = e2 - (M2 - 1)
 __global__ void dense_lag1_kernel(const float* gamma, int B, int n1, int n2, int m2, const double2* tw2,
@@ -77,8 +90,9 @@ __global__ void dense_lag1_kernel(const float* gamma, int B, int n1, int n2, int
     const int d2 = e2 - (m2 - 1);
     const float* g = gamma + r * n2;
     double2 acc = make_double2(0.0, 0.0);
+    TwidStep tw(tw2, n2, 0, d2);
     for (int k = 0; k < n2; ++k) {
-      const double2 w = twid(tw2, n2, static_cast<long long>(d2) * k, -1);
+      const double2 w = tw.next(-1);
       const double v = g[k];
       acc.x += v * w.x;
       acc.y += v * w.y;
@@ -101,7 +115,8 @@ __global__ void dense_lag2_kernel(const double2* T, int B, int n1, int m1, int m
     const int d1 = e1 - (m1 - 1);
     const double2* tb = T + static_cast<long long>(b) * n1 * W2 + e2;
     double2 acc = make_double2(0.0, 0.0);
-    for (int k = 0; k < n1; ++k) acc = zadd(acc, zmul(twid(tw1, n1, static_cast<long long>(d1) * k, -1), tb[k * W2]));
+    TwidStep tw(tw1, n1, 0, d1);
+    for (int k = 0; k < n1; ++k) acc = zadd(acc, zmul(tw.next(-1), tb[k * W2]));
     lag[t] = acc;
   }
 }
@@ -131,188 +146,270 @@ __global__ void dense_build_q_kernel(const double2* lag, int B, int m1, int m2, 
 }
 
 
-// The diagonal block [k, k + 32) of the Cholesky factor, in shared memory:
-// one warp per scene, lane i owning row i of the block.
-__global__ void __launch_bounds__(32) dense_diag_chol_kernel(double2* Q, int M, int k, int* status) {
-  __shared__ double2 D[kPanel][kPanel + 1];
-  double2* A = Q + static_cast<long long>(blockIdx.x) * M * M;
-  const int nb = M - k < kPanel ? M - k : kPanel, lane = threadIdx.x;
-  for (int c = 0; c < nb; ++c)
-    if (lane < nb && lane >= c) D[lane][c] = A[static_cast<long long>(k + c) * M + k + lane];
-  __syncwarp();
-  for (int c = 0; c < nb; ++c) {
-    double d = D[c][c].x;
-    if (!(d > 0.0)) {
-      if (lane == 0 && status)
-        atomicOr(status + blockIdx.x, isfinite(d) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE);
-      d = 2.2250738585072014e-308;
-    }
-    const double piv = sqrt(d);
-    __syncwarp();
-    if (lane > c && lane < nb) D[lane][c] = make_double2(D[lane][c].x / piv, D[lane][c].y / piv);
-    if (lane == c) D[c][c] = make_double2(piv, 0.0);
-    __syncwarp();
-    if (lane > c && lane < nb) {
-      const double2 li = D[lane][c];
-      for (int j = c + 1; j <= lane; ++j) {
-        const double2 v = zmulc(li, D[j][c]);
-        D[lane][j] = make_double2(D[lane][j].x - v.x, D[lane][j].y - v.y);
+// ---------------------------------------------------------------------------
+// Q^-1 by blocked symmetric sweeps, in place in the lower triangle of S
+// ---------------------------------------------------------------------------
+// With Q = L L^H and X = L^-1, before the sweep of panel [k, k + nb) entry
+// (i, j), i >= j, of S holds
+//     j >= k       the trailing matrix of the right-looking Cholesky,
+//     j < k <= i   minus the sum that becomes X[i][j],
+//     i < k        the sum over the swept rows r of conj(X[r][i]) X[r][j].
+// Let Z = L11^-1 of the diagonal block and W (M x nb) the panel
+//     W[r][c] = sum_c' s_r[c'] conj(Z[c][c']),   s_r = row r of the panel's
+// columns of the Hermitian S (the identity's rows for r in the panel).  Then
+// W[r] is row r of L below the panel and conj(column r of X) above and in
+// it, and the whole sweep is D = W W^H: S -= D for the rows below the
+// panel and S += D for the others, starting from zero in the panel's own
+// rows (columns j <= k) and columns (rows i >= k).  After the last panel S is
+// Q^-1.  Every sweep has the same work (M^2 / 2 entries, depth nb), which
+// fills the GPU at M = 1024 (136 tiles), and takes one launch: each block
+// forms the rows of W that its tile needs, and writes what becomes the next
+// sweep's panel to a separate buffer, so that no block reads what another
+// one writes; an extra block updates, factors and inverts the next diagonal
+// block meanwhile.  What sets the time is that block's chain of 32 square
+// roots.  Separate factor, inverse and product passes took five launches a
+// panel, with 32-column triangular solves and a one-warp factorisation in
+// series between them: 4.9 ms an EM iteration at M = 1024, REPLACEME so.
+
+// Factor and invert an nb x nb diagonal block on 256 threads: lane i owns
+// row i, warp w columns w, w + 8, w + 16, w + 24 (r: its entries).  An
+// entry is first the block's, then (once its column is posted) the sum that
+// becomes the inverse's; the warp owning column q + 1 takes it first and
+// arrives at its barrier without waiting, as its square root is the chain
+// that sets the time.  Z (row-major, lower) goes to global memory.
+struct DiagShared {
+  double2 L[kPanel][kPanel + 1];  // by columns: L[q][i] is entry (i, q)
+  double rl[kPanel];              // 1 / L[q][q]
+};
+
+__device__ __forceinline__ void diag_arrive(int q) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(1 + (q & 1)), "n"(32 * kDiagWarps) : "memory");
+}
+__device__ __forceinline__ void diag_sync(int q) {
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + (q & 1)), "n"(32 * kDiagWarps) : "memory");
+}
+
+__device__ __forceinline__ void diag_factor(DiagShared& S, double2 (&r)[kDiagCols], int nb, double2* Z, int* status) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int failed = 0;
+  auto post = [&](int q, double2& v) {
+    const double d = __shfl_sync(0xffffffffu, v.x, q);
+    const double rq = rsqrt(d > 0.0 ? d : 2.2250738585072014e-308);
+    S.L[q][lane] = lane > q ? make_double2(v.x * rq, v.y * rq) : make_double2(0.0, 0.0);
+    S.rl[q] = rq;  // the same value from every lane
+    diag_arrive(q);
+    v = make_double2(0.0, 0.0);
+    failed |= d > 0.0 ? 0 : isfinite(d) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;
+  };
+  auto sub_c = [](double2 v, double2 a, double2 b) {  // v - a conj(b)
+    return make_double2(v.x - (a.x * b.x + a.y * b.y), v.y - (a.y * b.x - a.x * b.y));
+  };
+  if (w == 0) post(0, r[0]);
+#pragma unroll
+  for (int uq = 0; uq < kDiagCols; ++uq) {
+#pragma unroll 1
+    for (int wq = 0; wq < kDiagWarps; ++wq) {
+      const int q = kDiagWarps * uq + wq;
+      if (q >= nb) break;
+      if (w != wq) diag_sync(q);
+      const double2 a = S.L[q][lane];
+      const double rlq = S.rl[q];
+      const int next = q + 1 < nb ? q + 1 : -1;
+      if (wq + 1 < kDiagWarps) {
+        if (w == wq + 1 && next > 0) {
+          if (lane >= next) r[uq] = sub_c(r[uq], a, S.L[q][next]);
+          post(next, r[uq]);
+        }
+      } else if (uq + 1 < kDiagCols) {
+        if (w == 0 && next > 0) {
+          if (lane >= next) r[uq + 1] = sub_c(r[uq + 1], a, S.L[q][next]);
+          post(next, r[uq + 1]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kDiagCols; ++u) {
+        const int j = w + kDiagWarps * u;
+        const bool right = u > uq || (u == uq && w > wq);
+        double2 v = r[u];
+        if (u >= uq) {
+          const double2 t = sub_c(r[u], a, S.L[q][j]);
+          if (right && j != next && lane >= j) v = t;
+        }
+        if (u <= uq) {
+          double2 xq = make_double2(__shfl_sync(0xffffffffu, r[u].x, q), __shfl_sync(0xffffffffu, r[u].y, q));
+          xq = j == q ? make_double2(rlq, 0.0) : make_double2(-xq.x * rlq, -xq.y * rlq);
+          const double2 t = zadd(r[u], zmul(a, xq));
+          if (!right) {
+            if (lane > q) v = t;
+            if (lane == 0) Z[q * kPanel + j] = xq;
+          }
+        }
+        r[u] = v;
       }
     }
-    __syncwarp();
   }
-  for (int c = 0; c < nb; ++c)
-    if (lane < nb && lane >= c) A[static_cast<long long>(k + c) * M + k + lane] = D[lane][c];
+  if (failed && lane == 0 && status) atomicOr(status, failed);
 }
 
-// The panel below the diagonal block: L21 = A21 L11^-H, one warp per row r
-// (lane c holding column k + c), forward over the block's columns.
-__global__ void __launch_bounds__(256) dense_panel_trsm_kernel(double2* Q, int M, int k) {
-  double2* A = Q + static_cast<long long>(blockIdx.y) * M * M;
-  const int r = k + kPanel + blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= M) return;  // whole warps: r is uniform in a warp
-  double2 a = A[static_cast<long long>(k + lane) * M + r];
-  for (int c = 0; c < kPanel; ++c) {
-    if (lane == c) {
-      const double piv = A[static_cast<long long>(k + c) * M + k + c].x;
-      a = make_double2(a.x / piv, a.y / piv);
-    }
-    const double2 x = make_double2(__shfl_sync(0xffffffffu, a.x, c), __shfl_sync(0xffffffffu, a.y, c));
-    if (lane > c) {
-      const double2 v = zmulc(x, A[static_cast<long long>(k + c) * M + k + lane]);  // x conj(L11[lane][c])
-      a = make_double2(a.x - v.x, a.y - v.y);
-    }
+// The first panel's diagonal block.
+__global__ void __launch_bounds__(32 * kDiagWarps) dense_diag_kernel(const double2* Sm, double2* Z, int M, int* status) {
+  __shared__ DiagShared S;
+  const double2* A = Sm + static_cast<long long>(blockIdx.x) * M * M;
+  const int nb = M < kPanel ? M : kPanel, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double2 r[kDiagCols];
+#pragma unroll
+  for (int u = 0; u < kDiagCols; ++u) {
+    const int j = w + kDiagWarps * u;
+    r[u] = (lane < nb && j < nb && lane >= j) ? A[static_cast<long long>(j) * M + lane] : make_double2(0.0, 0.0);
   }
-  A[static_cast<long long>(k + lane) * M + r] = a;
+  diag_factor(S, r, nb, Z + blockIdx.x * kPanel * kPanel, status ? status + blockIdx.x : nullptr);
 }
 
-// Rows [k, k + 32) of X = L^-1, forward substitution within the diagonal
-// block: one warp per column j < k + 32, lane i holding row k + i.
-__global__ void __launch_bounds__(256) dense_inv_panel_kernel(const double2* L, double2* X, int M, int k) {
-  const long long MM = static_cast<long long>(M) * M;
-  const double2* Lb = L + blockIdx.y * MM;
-  double2* Xb = X + blockIdx.y * MM;
-  const int nb = M - k < kPanel ? M - k : kPanel;
-  const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (j >= k + nb) return;
-  const int row = k + lane;
-  const bool own = lane < nb && row >= j;  // X is lower triangular
-  double2 v = own ? Xb[static_cast<long long>(j) * M + row] : make_double2(0.0, 0.0);
-  for (int c = 0; c < nb; ++c) {
-    if (lane == c) {
-      const double piv = Lb[static_cast<long long>(k + c) * M + k + c].x;
-      v = make_double2(v.x / piv, v.y / piv);
-    }
-    const double2 x = make_double2(__shfl_sync(0xffffffffu, v.x, c), __shfl_sync(0xffffffffu, v.y, c));
-    if (lane > c && lane < nb) {
-      const double2 p = zmul(Lb[static_cast<long long>(k + c) * M + row], x);
-      v = make_double2(v.x - p.x, v.y - p.y);
+// Shared memory of a sweep's block: the panel's rows of the tile's rows and
+// columns, the conjugated Z, and the rows of W formed from them.
+struct SweepShared {
+  double2 src[2][kPanel][kTile];
+  double2 W[2][kPanel][kTile];
+  double2 z[kPanel][kPanel];
+};
+union SweepUnion {
+  SweepShared s;
+  struct {
+    double2 src[kPanel][kPanel];
+    double2 z[kPanel][kPanel];
+    double2 W[kPanel][kPanel];
+    DiagShared d;
+  } g;
+};
+
+// Rows r0 .. r0 + RB of W (RB = 32 or 64) from the panel P: lane = row
+// (and row + 32), warp w the columns w, w + 8, w + 16, w + 24.
+template <int RB>
+__device__ __forceinline__ void sweep_rows(const double2* P, int M, int k, int nb, int r0, double2 (*src)[RB],
+                                           const double2 (*z)[kPanel], double2 (*W)[RB]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int e = threadIdx.x; e < kPanel * RB; e += 256) {
+    const int c = e / RB, r = r0 + e % RB;
+    double2 v = make_double2(0.0, 0.0);
+    if (r >= k && r < k + kPanel) v.x = r - k == c ? 1.0 : 0.0;  // the panel's own rows: the identity
+    else if (c < nb && r < M) v = P[static_cast<long long>(c) * M + r];
+    src[c][e % RB] = v;
+  }
+  __syncthreads();
+  constexpr int H = RB / 32;
+  double2 acc[4][H];
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int h = 0; h < H; ++h) acc[u][h] = make_double2(0.0, 0.0);
+#pragma unroll
+  for (int uc = 0; uc < 4; ++uc) {  // c' in [8 uc, 8 uc + 8): columns c < 8 uc have none
+#pragma unroll 2
+    for (int i = 0; i < 8; ++i) {
+      const int cp = 8 * uc + i;
+      double2 s[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) s[h] = src[cp][lane + 32 * h];
+#pragma unroll
+      for (int u = uc; u < 4; ++u) {  // z is zero above its diagonal
+        const double2 f = z[w + 8 * u][cp];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          acc[u][h].x = fma(s[h].x, f.x, fma(-s[h].y, f.y, acc[u][h].x));
+          acc[u][h].y = fma(s[h].x, f.y, fma(s[h].y, f.x, acc[u][h].y));
+        }
+      }
     }
   }
-  if (own) Xb[static_cast<long long>(j) * M + row] = v;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int h = 0; h < H; ++h) W[w + 8 * u][lane + 32 * h] = acc[u][h];
 }
 
-// Tile updates over 64 x 64 output tiles (grid: tiles x scenes), depth in
-// chunks of kDk staged in shared memory; thread (ti, tj) of 16 x 16 owns the
-// rows i0 + ti + 16 a and columns j0 + tj + 16 b (a, b < 4), so that stores
-// of consecutive threads are consecutive in a column.
-//   MODE 0  Cholesky trailing update, lower tiles of rows/cols [k1, M):
-//           Q[i][j] -= sum_{c in [k0, k1)} Q[i][c] conj(Q[j][c])
-//   MODE 1  inverse update, rows [k1, M) x columns [0, k1):
-//           X[i][j] -= sum_{c in [k0, k1)} L[i][c] X[c][j]
-//   MODE 2  R = X^H X, lower tiles of [0, M), stored in both triangles:
-//           R[i][j] = sum_{r >= i0} conj(X[r][i]) X[r][j]
-template <int MODE>
-__global__ void __launch_bounds__(256) dense_tile_kernel(double2* C, const double2* A, const double2* Xm, int M,
-                                                         int k0, int k1) {
-  __shared__ double2 As[kDk][kTile];
-  __shared__ double2 Bs[kDk][kTile];
-  const long long MM = static_cast<long long>(M) * M;
+// Sweep k of scene blockIdx.y: block 0 the next diagonal block, the others
+// one 64 x 64 tile of the lower triangle each; thread (ri, rj) of 16 x 16
+// owns the rows i0 + ri + 16 a and columns j0 + rj + 16 b (a, b < 4), so that
+// stores of consecutive threads are consecutive in a column.  P: this
+// sweep's panel [c][r], Pn: the next one's, Z: this sweep's diagonal
+// inverse, Zn: the next one's.  The last sweep stores both triangles.
+__global__ void __launch_bounds__(256) dense_sweep_kernel(double2* Sm, const double2* Pm, double2* Pn, const double2* Zm,
+                                                          double2* Zn, int M, int k, int* status) {
+  extern __shared__ double2 sweep_shm[];
+  SweepUnion& sh = *reinterpret_cast<SweepUnion*>(sweep_shm);
   const int scene = blockIdx.y;
-  C += scene * MM;
-  A += scene * MM;
-  if (Xm) Xm += scene * MM;
-  // tile coordinates
-  int ti, tj, base_i, base_j;
-  const int t = blockIdx.x;
-  if (MODE == 1) {
-    const int tcols = (k1 + kTile - 1) / kTile;
-    ti = t / tcols;
-    tj = t - ti * tcols;
-    base_i = k1;
-    base_j = 0;
-  } else {
-    ti = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-    while (ti * (ti + 1) / 2 > t) --ti;
-    tj = t - ti * (ti + 1) / 2;
-    base_i = base_j = MODE == 0 ? k1 : 0;
+  double2* S = Sm + static_cast<long long>(scene) * M * M;
+  const double2* P = Pm + static_cast<long long>(scene) * kPanel * M;
+  const double2* Z = Zm + scene * kPanel * kPanel;
+  const int tid = threadIdx.x;
+  const int k1 = k + kPanel < M ? k + kPanel : M, nb = k1 - k;
+  auto load_z = [&](double2 (*z)[kPanel]) {
+    for (int e = tid; e < kPanel * kPanel; e += 256) {
+      const int c = e / kPanel, cp = e % kPanel;
+      const double2 v = (c < nb && cp <= c) ? Z[e] : make_double2(0.0, 0.0);
+      z[c][cp] = make_double2(v.x, -v.y);
+    }
+  };
+  if (blockIdx.x == 0) {
+    if (k1 >= M) return;
+    const int nn = M - k1 < kPanel ? M - k1 : kPanel, lane = tid & 31, w = tid >> 5;
+    double2 v[kDiagCols];  // the block's entries, loaded ahead of their update
+#pragma unroll
+    for (int u = 0; u < kDiagCols; ++u) {
+      const int j = w + kDiagWarps * u;
+      v[u] = (lane < nn && j < nn && lane >= j) ? S[static_cast<long long>(k1 + j) * M + k1 + lane]
+                                                : make_double2(0.0, 0.0);
+    }
+    load_z(sh.g.z);
+    sweep_rows<kPanel>(P, M, k, nb, k1, sh.g.src, sh.g.z, sh.g.W);
+    __syncthreads();
+#pragma unroll 4
+    for (int c = 0; c < kPanel; ++c) {
+      const double2 a = sh.g.W[c][lane];
+#pragma unroll
+      for (int u = 0; u < kDiagCols; ++u) {
+        const double2 b = sh.g.W[c][w + kDiagWarps * u];
+        v[u].x -= a.x * b.x + a.y * b.y;
+        v[u].y -= a.y * b.x - a.x * b.y;
+      }
+    }
+    diag_factor(sh.g.d, v, nn, Zn + scene * kPanel * kPanel, status ? status + scene : nullptr);
+    return;
   }
-  const int i0 = base_i + ti * kTile, j0 = base_j + tj * kTile;
-  const int tid = threadIdx.x, ri = tid & 15, rj = tid >> 4;
+  const int t = blockIdx.x - 1;
+  int ti = static_cast<int>((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
+  while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+  while (ti * (ti + 1) / 2 > t) --ti;
+  const int tj = t - ti * (ti + 1) / 2;
+  const int i0 = ti * kTile, j0 = tj * kTile;
+  const int ri = tid & 15, rj = tid >> 4;
+  load_z(sh.s.z);
+  sweep_rows<kTile>(P, M, k, nb, i0, sh.s.src[0], sh.s.z, sh.s.W[0]);
+  if (ti != tj) sweep_rows<kTile>(P, M, k, nb, j0, sh.s.src[1], sh.s.z, sh.s.W[1]);
+  __syncthreads();
+  const double2(*Wi)[kTile] = sh.s.W[0];
+  const double2(*Wj)[kTile] = ti != tj ? sh.s.W[1] : sh.s.W[0];
   double2 acc[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) acc[a][b] = make_double2(0.0, 0.0);
-  const int d_begin = MODE == 2 ? i0 : k0;
-  const int d_end = MODE == 2 ? M : (k1 < M ? k1 : M);
-  for (int d0 = d_begin; d0 < d_end; d0 += kDk) {
-    for (int u = tid; u < kDk * kTile; u += 256) {
-      if (MODE == 2) {  // both operands read along a column of X (d fastest)
-        const int d = u % kDk, e = u / kDk;
-        const int r = d0 + d;
-        const int i = i0 + e, j = j0 + e;
-        double2 av = make_double2(0.0, 0.0), bv = make_double2(0.0, 0.0);
-        // X is lower triangular; its upper part is never written
-        if (r < d_end && i < M && r >= i) {
-          const double2 x = Xm[static_cast<long long>(i) * M + r];
-          av = make_double2(x.x, -x.y);
-        }
-        if (r < d_end && j < M && r >= j) bv = Xm[static_cast<long long>(j) * M + r];
-        As[d][e] = av;
-        Bs[d][e] = bv;
-      } else {
-        const int e = u % kTile, d = u / kTile;
-        const int c = d0 + d;
-        const int i = i0 + e;
-        As[d][e] = (c < d_end && i < M) ? A[static_cast<long long>(c) * M + i] : make_double2(0.0, 0.0);
-        if (MODE == 0) {
-          const int j = j0 + e;
-          double2 bv = make_double2(0.0, 0.0);
-          if (c < d_end && j < M) {
-            const double2 q = A[static_cast<long long>(c) * M + j];
-            bv = make_double2(q.x, -q.y);
-          }
-          Bs[d][e] = bv;
-        }
-      }
-    }
-    if (MODE == 1) {  // X[c][j]: along a column of X (d fastest)
-      for (int u = tid; u < kDk * kTile; u += 256) {
-        const int d = u % kDk, e = u / kDk;
-        const int c = d0 + d, j = j0 + e;
-        Bs[d][e] = (c < d_end && j < M && c >= j) ? Xm[static_cast<long long>(j) * M + c] : make_double2(0.0, 0.0);
-      }
-    }
-    __syncthreads();
 #pragma unroll 4
-    for (int d = 0; d < kDk; ++d) {
-      double2 av[4], bv[4];
+  for (int d = 0; d < kPanel; ++d) {
+    double2 av[4], bv[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[d][ri + 16 * a];
+    for (int a = 0; a < 4; ++a) av[a] = Wi[d][ri + 16 * a];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = Bs[d][rj + 16 * b];
+    for (int b = 0; b < 4; ++b) bv[b] = Wj[d][rj + 16 * b];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          acc[a][b].x = fma(av[a].x, bv[b].x, fma(-av[a].y, bv[b].y, acc[a][b].x));
-          acc[a][b].y = fma(av[a].x, bv[b].y, fma(av[a].y, bv[b].x, acc[a][b].y));
-        }
-    }
-    __syncthreads();
+      for (int b = 0; b < 4; ++b) {  // W_i conj(W_j)
+        acc[a][b].x = fma(av[a].x, bv[b].x, fma(av[a].y, bv[b].y, acc[a][b].x));
+        acc[a][b].y = fma(-av[a].x, bv[b].y, fma(av[a].y, bv[b].x, acc[a][b].y));
+      }
   }
+  double2* Pnext = Pn + static_cast<long long>(scene) * kPanel * M;
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int j = j0 + rj + 16 * b;
@@ -320,26 +417,20 @@ __global__ void __launch_bounds__(256) dense_tile_kernel(double2* C, const doubl
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
       const int i = i0 + ri + 16 * a;
-      if (i >= M || (MODE != 1 && i < j)) continue;
-      double2* dst = C + static_cast<long long>(j) * M + i;
-      if (MODE == 2) {  // R is stored in full (both triangles)
-        *dst = acc[a][b];
-        if (i != j) C[static_cast<long long>(i) * M + j] = make_double2(acc[a][b].x, -acc[a][b].y);
-      } else {
-        *dst = make_double2(dst->x - acc[a][b].x, dst->y - acc[a][b].y);
-      }
+      // the next diagonal block is block 0's, which reads it meanwhile
+      if (i >= M || i < j || (j >= k1 && i < k1 + kPanel)) continue;
+      double2* dst = S + static_cast<long long>(j) * M + i;
+      const bool below = i >= k1;
+      // the panel's own rows and columns start from zero
+      const bool fresh = below ? (j >= k && j < k1) : i >= k;
+      const double2 old = fresh ? make_double2(0.0, 0.0) : *dst;
+      const double2 v = below ? make_double2(old.x - acc[a][b].x, old.y - acc[a][b].y) : zadd(old, acc[a][b]);
+      // what the next sweep takes as its panel goes there alone
+      if (j >= k1 && j < k1 + kPanel) Pnext[static_cast<long long>(j - k1) * M + i] = v;
+      else if (i >= k1 && i < k1 + kPanel) Pnext[static_cast<long long>(i - k1) * M + j] = make_double2(v.x, -v.y);
+      else *dst = v;
+      if (k1 == M && i != j) S[static_cast<long long>(i) * M + j] = make_double2(v.x, -v.y);
     }
-  }
-}
-
-// X = I (lower triangle) before the blocked inversion.
-__global__ void dense_identity_kernel(double2* X, int B, int M) {
-  const long long MM = static_cast<long long>(M) * M, total = B * MM;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long r = t % MM;
-    const int j = static_cast<int>(r / M), i = static_cast<int>(r - static_cast<long long>(j) * M);
-    if (i >= j) X[t] = make_double2(i == j ? 1.0 : 0.0, 0.0);
   }
 }
 
@@ -412,8 +503,8 @@ __global__ void dense_inv1_kernel(const double2* S, int B, int W1, int W2, int o
     const long long r = t / n2;  // b * W1 + e1
     const double2* row = S + r * W2;
     double2 acc = make_double2(0.0, 0.0);
-    for (int e2 = 0; e2 < W2; ++e2)
-      acc = zadd(acc, zmul(row[e2], twid(tw2, n2, static_cast<long long>(e2 + o2) * k2, +1)));
+    TwidStep tw(tw2, n2, static_cast<long long>(o2) * k2, k2);
+    for (int e2 = 0; e2 < W2; ++e2) acc = zadd(acc, zmul(row[e2], tw.next(+1)));
     U[t] = acc;
   }
 }
@@ -428,8 +519,8 @@ __global__ void dense_inv2_kernel(const double2* U, int B, int W1, int o1, int n
     const int k1 = static_cast<int>(r % n1), b = static_cast<int>(r / n1);
     const double2* ub = U + static_cast<long long>(b) * W1 * n2 + k2;
     double2 acc = make_double2(0.0, 0.0);
-    for (int e1 = 0; e1 < W1; ++e1)
-      acc = zadd(acc, zmul(twid(tw1, n1, static_cast<long long>(e1 + o1) * k1, +1), ub[static_cast<long long>(e1) * n2]));
+    TwidStep tw(tw1, n1, static_cast<long long>(o1) * k1, k1);
+    for (int e1 = 0; e1 < W1; ++e1) acc = zadd(acc, zmul(tw.next(+1), ub[static_cast<long long>(e1) * n2]));
     if (REAL)
       out_re[t] = acc.x;
     else
@@ -496,8 +587,8 @@ int grid_of(long long n) {
 
 }  // namespace
 
-// Workspace of the dense posterior: [Q / L / R][X] per scene (FP64
-// complex M x M each), lags, pass buffers, Q^-1 y, lift, data diagonal and
+// Workspace of the dense posterior: Q, swept in place to Q^-1, per scene (FP64
+// complex M x M), the sweeps' panels and diagonal inverses (two each), lags, pass buffers, Q^-1 y, lift, data diagonal and
 // the FP64 twiddle tables.
 size_t dense_bytes(const BatchShape& s) {
   const size_t B = s.B, M = s.m(), N = s.n();
@@ -505,7 +596,8 @@ size_t dense_bytes(const BatchShape& s) {
   auto up = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
   const size_t pass = std::max(std::max(static_cast<size_t>(s.n1) * W2, W1 * static_cast<size_t>(s.n2)),
                                static_cast<size_t>(s.m1) * s.n2);
-  return 2 * up(B * M * M * sizeof(double2)) + 2 * up(B * W1 * W2 * sizeof(double2)) +
+  return up(B * M * M * sizeof(double2)) + 2 * up(B * kPanel * M * sizeof(double2)) +
+         2 * up(B * kPanel * kPanel * sizeof(double2)) + 2 * up(B * W1 * W2 * sizeof(double2)) +
          up(B * pass * sizeof(double2)) + up(B * M * sizeof(double2)) + up(B * N * sizeof(double2)) +
          up(B * N * sizeof(double)) + up(s.n1 * sizeof(double2)) + up(s.n2 * sizeof(double2));
 }
@@ -524,7 +616,8 @@ DenseBufs dense_bind(uint8_t* w, const BatchShape& s, cudaStream_t st) {
     return p;
   };
   d.Q = reinterpret_cast<double2*>(take(B * M * M * sizeof(double2)));
-  d.X = reinterpret_cast<double2*>(take(B * M * M * sizeof(double2)));
+  for (int i = 0; i < 2; ++i) d.P[i] = reinterpret_cast<double2*>(take(B * kPanel * M * sizeof(double2)));
+  for (int i = 0; i < 2; ++i) d.Z[i] = reinterpret_cast<double2*>(take(B * kPanel * kPanel * sizeof(double2)));
   d.lag = reinterpret_cast<double2*>(take(B * W1 * W2 * sizeof(double2)));
   d.lsum = reinterpret_cast<double2*>(take(B * W1 * W2 * sizeof(double2)));
   d.pass = reinterpret_cast<double2*>(take(B * pass * sizeof(double2)));
@@ -535,6 +628,8 @@ DenseBufs dense_bind(uint8_t* w, const BatchShape& s, cudaStream_t st) {
   d.tw2 = reinterpret_cast<double2*>(take(s.n2 * sizeof(double2)));
   dense_twiddle_kernel<<<(s.n1 + 255) / 256, 256, 0, st>>>(d.tw1, s.n1);
   dense_twiddle_kernel<<<(s.n2 + 255) / 256, 256, 0, st>>>(d.tw2, s.n2);
+  cudaFuncSetAttribute(dense_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       static_cast<int>(sizeof(SweepUnion)));
   return d;
 }
 
@@ -547,31 +642,15 @@ void dense_posterior(const BatchShape& s, const DenseBufs& d, const float* gamma
   dense_lag1_kernel<<<grid_of(1LL * B * n1 * W2), 256, 0, st>>>(gamma, B, n1, n2, m2, d.tw2, d.pass);
   dense_lag2_kernel<<<grid_of(1LL * B * W1 * W2), 256, 0, st>>>(d.pass, B, n1, m1, m2, d.tw1, d.lag);
   dense_build_q_kernel<<<grid_of(1LL * B * M * M), 256, 0, st>>>(d.lag, B, m1, m2, noise, jitter, d.Q);
-  // Cholesky
-  for (int k = 0; k < M; k += kPanel) {
-    dense_diag_chol_kernel<<<B, 32, 0, st>>>(d.Q, M, k, status);
-    const int k1 = k + kPanel;
-    if (k1 < M) {
-      dense_panel_trsm_kernel<<<dim3((M - k1 + 7) / 8, B), 256, 0, st>>>(d.Q, M, k);
-      const int T = (M - k1 + kTile - 1) / kTile;
-      dense_tile_kernel<0><<<dim3(T * (T + 1) / 2, B), 256, 0, st>>>(d.Q, d.Q, nullptr, M, k, k1);
-    }
-  }
-  // X = L^-1
-  dense_identity_kernel<<<grid_of(1LL * B * M * M), 256, 0, st>>>(d.X, B, M);
-  for (int k = 0; k < M; k += kPanel) {
-    dense_inv_panel_kernel<<<dim3((std::min(k + kPanel, M) + 7) / 8, B), 256, 0, st>>>(d.Q, d.X, M, k);
-    const int k1 = k + kPanel;
-    if (k1 < M) {
-      const int TI = (M - k1 + kTile - 1) / kTile, TJ = (k1 + kTile - 1) / kTile;
-      dense_tile_kernel<1><<<dim3(TI * TJ, B), 256, 0, st>>>(d.X, d.Q, d.X, M, k, k1);
-    }
-  }
-  // Q^-1 = X^H X into the factor's storage
-  {
-    const int T = (M + kTile - 1) / kTile;
-    dense_tile_kernel<2><<<dim3(T * (T + 1) / 2, B), 256, 0, st>>>(d.Q, d.Q, d.X, M, 0, 0);
-  }
+  // Q^-1 in place; the first panel is Q's first columns
+  const int T = (M + kTile - 1) / kTile;
+  dense_diag_kernel<<<B, 32 * kDiagWarps, 0, st>>>(d.Q, d.Z[0], M, status);
+  const size_t panel = sizeof(double2) * kPanel * M;
+  cudaMemcpy2DAsync(d.P[0], panel, d.Q, sizeof(double2) * M * M, sizeof(double2) * std::min(kPanel, M) * M, B,
+                    cudaMemcpyDeviceToDevice, st);
+  for (int k = 0, i = 0; k < M; k += kPanel, i ^= 1)
+    dense_sweep_kernel<<<dim3(1 + T * (T + 1) / 2, B), 256, sizeof(SweepUnion), st>>>(
+        d.Q, d.P[i], d.P[i ^ 1], d.Z[i], d.Z[i ^ 1], M, k, status);
   dense_qinv_y_kernel<<<dim3((M + 7) / 8, B), 256, 0, st>>>(d.Q, y, B, M, d.z);
   dense_energy_kernel<<<B, 256, 0, st>>>(d.z, d.lag, noise, jitter, m1, m2, part);
   // data diagonal: Re N ifft2 of the lag sums

@@ -307,7 +307,9 @@ void cg_active_posterior(const ActiveArgs& a, cudaStream_t st);
 // mode="dense": the exact posterior through the M x M data covariance in
 // FP64 (dense.cu).
 struct DenseBufs {
-  double2 *Q, *X;      // [B][M][M] Cholesky factor, then Q^-1 / L^-1 (column-major)
+  double2* Q;          // [B][M][M] the data covariance, swept in place to its inverse (column-major)
+  double2* P[2];       // [B][32][M] panel of a sweep, and of the next
+  double2* Z[2];       // [B][32][32] inverse factors of their diagonal blocks
   double2 *lag, *lsum; // [B][2M1-1][2M2-1] lags of the prior, lag sums of Q^-1
   double2* pass;       // separable-transform pass buffer
   double2* z;          // [B][M] Q^-1 y
