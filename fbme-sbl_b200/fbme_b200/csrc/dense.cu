@@ -45,8 +45,10 @@ __device__ __forceinline__ double2 zadd(double2 a, double2 b) { return make_doub
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ double2 zmulc(double2 a, double2 b) {  // a * conj(b)
-  return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+__device__ __forceinline__ double2 warp_sum2(double2 v) {
+  v.x = warp_sum(v.x);
+  v.y = warp_sum(v.y);
+  return v;
 }
 
 // exp(-2 pi i k / L), k < L, FP64
@@ -78,46 +80,45 @@ struct TwidStep {
   }
 };
 
+// One output of a separable pass on one warp: sum_k in(k) w^(sign (e0 +
+// step k)), k < count, lanes over k (a thread per output left 16 blocks
+// walking 64 terms each: 27 us a pass at 64 x 64, 6 us so).
+template <typename F>
+__device__ __forceinline__ double2 warp_dft(F in, int count, const double2* tw, int L, long long e0, long long step,
+                                            int sign) {
+  const int lane = threadIdx.x & 31;
+  TwidStep t(tw, L, e0 + step * lane, 32 * step);
+  double2 acc = make_double2(0.0, 0.0);
+  for (int k = lane; k < count; k += 32) acc = zadd(acc, zmul(in(k), t.next(sign)));
+  return warp_sum2(acc);
+}
+// Outputs t of a pass, one per warp.
+#define FBME_WARP_OUTPUTS(total)                                                              \
+  for (long long t = blockIdx.x * 8LL + (threadIdx.x >> 5); t < (total); t += gridDim.x * 8LL)
+
 // Lag pass 1: T[b][n1][e2] = sum_n2 gamma[b][n1][n2] w2^(d2 n2), d2 = e2 - (M2 - 1)
-__global__ void dense_lag1_kernel(const float* gamma, int B, int n1, int n2, int m2, const double2* tw2,
-                                  double2* T) {
+__global__ void __launch_bounds__(256) dense_lag1_kernel(const float* gamma, int B, int n1, int n2, int m2,
+                                                         const double2* tw2, double2* T) {
   const int W2 = 2 * m2 - 1;
-  const long long total = static_cast<long long>(B) * n1 * W2;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int e2 = static_cast<int>(t % W2);
-    const long long r = t / W2;  // b * n1 + row
-    const int d2 = e2 - (m2 - 1);
-    const float* g = gamma + r * n2;
-    double2 acc = make_double2(0.0, 0.0);
-    TwidStep tw(tw2, n2, 0, d2);
-    for (int k = 0; k < n2; ++k) {
-      const double2 w = tw.next(-1);
-      const double v = g[k];
-      acc.x += v * w.x;
-      acc.y += v * w.y;
-    }
-    T[t] = acc;
+  FBME_WARP_OUTPUTS(static_cast<long long>(B) * n1 * W2) {
+    const int d2 = static_cast<int>(t % W2) - (m2 - 1);
+    const float* g = gamma + t / W2 * n2;  // b * n1 + row
+    const double2 v = warp_dft([&](int k) { return make_double2(g[k], 0.0); }, n2, tw2, n2, 0, d2, -1);
+    if ((threadIdx.x & 31) == 0) T[t] = v;
   }
 }
 
 // Lag pass 2: lag[b][e1][e2] = sum_n1 w1^(d1 n1) T[b][n1][e2], d1 = e1 - (M1 - 1)
-__global__ void dense_lag2_kernel(const double2* T, int B, int n1, int m1, int m2, const double2* tw1,
-                                  double2* lag) {
+__global__ void __launch_bounds__(256) dense_lag2_kernel(const double2* T, int B, int n1, int m1, int m2,
+                                                         const double2* tw1, double2* lag) {
   const int W1 = 2 * m1 - 1, W2 = 2 * m2 - 1;
-  const long long total = static_cast<long long>(B) * W1 * W2;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+  FBME_WARP_OUTPUTS(static_cast<long long>(B) * W1 * W2) {
     const int e2 = static_cast<int>(t % W2);
     const long long r = t / W2;
-    const int e1 = static_cast<int>(r % W1);
-    const int b = static_cast<int>(r / W1);
-    const int d1 = e1 - (m1 - 1);
-    const double2* tb = T + static_cast<long long>(b) * n1 * W2 + e2;
-    double2 acc = make_double2(0.0, 0.0);
-    TwidStep tw(tw1, n1, 0, d1);
-    for (int k = 0; k < n1; ++k) acc = zadd(acc, zmul(tw.next(-1), tb[k * W2]));
-    lag[t] = acc;
+    const int d1 = static_cast<int>(r % W1) - (m1 - 1);
+    const double2* tb = T + r / W1 * n1 * W2 + e2;
+    const double2 v = warp_dft([&](int k) { return tb[static_cast<long long>(k) * W2]; }, n1, tw1, n1, 0, d1, -1);
+    if ((threadIdx.x & 31) == 0) lag[t] = v;
   }
 }
 
@@ -169,7 +170,7 @@ __global__ void dense_build_q_kernel(const double2* lag, int B, int m1, int m2, 
 // block meanwhile.  What sets the time is that block's chain of 32 square
 // roots.  Separate factor, inverse and product passes took five launches a
 // panel, with 32-column triangular solves and a one-warp factorisation in
-// series between them: 4.9 ms an EM iteration at M = 1024, REPLACEME so.
+// series between them: 4.9 ms an EM iteration at M = 1024, 0.8 ms so.
 
 // Factor and invert an nb x nb diagonal block on 256 threads: lane i owns
 // row i, warp w columns w, w + 8, w + 16, w + 24 (r: its entries).  An
@@ -202,7 +203,10 @@ __device__ __forceinline__ void diag_factor(DiagShared& S, double2 (&r)[kDiagCol
     failed |= d > 0.0 ? 0 : isfinite(d) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;
   };
   auto sub_c = [](double2 v, double2 a, double2 b) {  // v - a conj(b)
-    return make_double2(v.x - (a.x * b.x + a.y * b.y), v.y - (a.y * b.x - a.x * b.y));
+    return make_double2(fma(-a.x, b.x, fma(-a.y, b.y, v.x)), fma(-a.y, b.x, fma(a.x, b.y, v.y)));
+  };
+  auto add_m = [](double2 v, double2 a, double2 b) {  // v + a b
+    return make_double2(fma(a.x, b.x, fma(-a.y, b.y, v.x)), fma(a.x, b.y, fma(a.y, b.x, v.y)));
   };
   if (w == 0) post(0, r[0]);
 #pragma unroll
@@ -238,7 +242,7 @@ __device__ __forceinline__ void diag_factor(DiagShared& S, double2 (&r)[kDiagCol
         if (u <= uq) {
           double2 xq = make_double2(__shfl_sync(0xffffffffu, r[u].x, q), __shfl_sync(0xffffffffu, r[u].y, q));
           xq = j == q ? make_double2(rlq, 0.0) : make_double2(-xq.x * rlq, -xq.y * rlq);
-          const double2 t = zadd(r[u], zmul(a, xq));
+          const double2 t = add_m(r[u], a, xq);
           if (!right) {
             if (lane > q) v = t;
             if (lane == 0) Z[q * kPanel + j] = xq;
@@ -282,20 +286,33 @@ union SweepUnion {
   } g;
 };
 
-// Rows r0 .. r0 + RB of W (RB = 32 or 64) from the panel P: lane = row
-// (and row + 32), warp w the columns w, w + 8, w + 16, w + 24.
+// The panel's rows r0 .. r0 + RB (RB = 32 or 64) into shared memory,
+// asynchronous copies (the caller waits); the panel's own rows are the
+// identity's.
 template <int RB>
-__device__ __forceinline__ void sweep_rows(const double2* P, int M, int k, int nb, int r0, double2 (*src)[RB],
-                                           const double2 (*z)[kPanel], double2 (*W)[RB]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int e = threadIdx.x; e < kPanel * RB; e += 256) {
+__device__ __forceinline__ void sweep_load(const double2* P, int M, int k, int nb, int r0, double2 (*src)[RB]) {
+#pragma unroll
+  for (int i = 0; i < kPanel * RB / 256; ++i) {
+    const int e = threadIdx.x + 256 * i;
     const int c = e / RB, r = r0 + e % RB;
-    double2 v = make_double2(0.0, 0.0);
-    if (r >= k && r < k + kPanel) v.x = r - k == c ? 1.0 : 0.0;  // the panel's own rows: the identity
-    else if (c < nb && r < M) v = P[static_cast<long long>(c) * M + r];
-    src[c][e % RB] = v;
+    double2* dst = &src[c][e % RB];
+    if (!(r >= k && r < k + kPanel) && c < nb && r < M)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)),
+                   "l"(P + static_cast<long long>(c) * M + r) : "memory");
+    else
+      *dst = make_double2(r - k == c ? 1.0 : 0.0, 0.0);
   }
+}
+__device__ __forceinline__ void sweep_wait() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+}
+
+// Rows of W from the panel's: lane = row (and row + 32), warp w the columns
+// w, w + 8, w + 16, w + 24.
+template <int RB>
+__device__ __forceinline__ void sweep_rows(const double2 (*src)[RB], const double2 (*z)[kPanel], double2 (*W)[RB]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int H = RB / 32;
   double2 acc[4][H];
 #pragma unroll
@@ -304,7 +321,7 @@ __device__ __forceinline__ void sweep_rows(const double2* P, int M, int k, int n
     for (int h = 0; h < H; ++h) acc[u][h] = make_double2(0.0, 0.0);
 #pragma unroll
   for (int uc = 0; uc < 4; ++uc) {  // c' in [8 uc, 8 uc + 8): columns c < 8 uc have none
-#pragma unroll 2
+#pragma unroll 4
     for (int i = 0; i < 8; ++i) {
       const int cp = 8 * uc + i;
       double2 s[H];
@@ -360,17 +377,19 @@ __global__ void __launch_bounds__(256) dense_sweep_kernel(double2* Sm, const dou
       v[u] = (lane < nn && j < nn && lane >= j) ? S[static_cast<long long>(k1 + j) * M + k1 + lane]
                                                 : make_double2(0.0, 0.0);
     }
+    sweep_load<kPanel>(P, M, k, nb, k1, sh.g.src);
     load_z(sh.g.z);
-    sweep_rows<kPanel>(P, M, k, nb, k1, sh.g.src, sh.g.z, sh.g.W);
+    sweep_wait();
+    sweep_rows<kPanel>(sh.g.src, sh.g.z, sh.g.W);
     __syncthreads();
-#pragma unroll 4
+#pragma unroll 8
     for (int c = 0; c < kPanel; ++c) {
       const double2 a = sh.g.W[c][lane];
 #pragma unroll
       for (int u = 0; u < kDiagCols; ++u) {
         const double2 b = sh.g.W[c][w + kDiagWarps * u];
-        v[u].x -= a.x * b.x + a.y * b.y;
-        v[u].y -= a.y * b.x - a.x * b.y;
+        v[u].x = fma(-a.x, b.x, fma(-a.y, b.y, v[u].x));
+        v[u].y = fma(-a.y, b.x, fma(a.x, b.y, v[u].y));
       }
     }
     diag_factor(sh.g.d, v, nn, Zn + scene * kPanel * kPanel, status ? status + scene : nullptr);
@@ -383,9 +402,23 @@ __global__ void __launch_bounds__(256) dense_sweep_kernel(double2* Sm, const dou
   const int tj = t - ti * (ti + 1) / 2;
   const int i0 = ti * kTile, j0 = tj * kTile;
   const int ri = tid & 15, rj = tid >> 4;
+  sweep_load<kTile>(P, M, k, nb, i0, sh.s.src[0]);
+  if (ti != tj) sweep_load<kTile>(P, M, k, nb, j0, sh.s.src[1]);
+  // the tile's entries, loaded ahead of the products; the panel's own rows
+  // and columns start from zero
+  double2 old[4][4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+      const int i = i0 + ri + 16 * a, j = j0 + rj + 16 * b;
+      const bool fresh = i >= k1 ? (j >= k && j < k1) : i >= k;
+      old[a][b] = (i < M && i >= j && !fresh) ? S[static_cast<long long>(j) * M + i] : make_double2(0.0, 0.0);
+    }
   load_z(sh.s.z);
-  sweep_rows<kTile>(P, M, k, nb, i0, sh.s.src[0], sh.s.z, sh.s.W[0]);
-  if (ti != tj) sweep_rows<kTile>(P, M, k, nb, j0, sh.s.src[1], sh.s.z, sh.s.W[1]);
+  sweep_wait();
+  sweep_rows<kTile>(sh.s.src[0], sh.s.z, sh.s.W[0]);
+  if (ti != tj) sweep_rows<kTile>(sh.s.src[1], sh.s.z, sh.s.W[1]);
   __syncthreads();
   const double2(*Wi)[kTile] = sh.s.W[0];
   const double2(*Wj)[kTile] = ti != tj ? sh.s.W[1] : sh.s.W[0];
@@ -420,11 +453,8 @@ __global__ void __launch_bounds__(256) dense_sweep_kernel(double2* Sm, const dou
       // the next diagonal block is block 0's, which reads it meanwhile
       if (i >= M || i < j || (j >= k1 && i < k1 + kPanel)) continue;
       double2* dst = S + static_cast<long long>(j) * M + i;
-      const bool below = i >= k1;
-      // the panel's own rows and columns start from zero
-      const bool fresh = below ? (j >= k && j < k1) : i >= k;
-      const double2 old = fresh ? make_double2(0.0, 0.0) : *dst;
-      const double2 v = below ? make_double2(old.x - acc[a][b].x, old.y - acc[a][b].y) : zadd(old, acc[a][b]);
+      const double2 o = old[a][b];
+      const double2 v = i >= k1 ? make_double2(o.x - acc[a][b].x, o.y - acc[a][b].y) : zadd(o, acc[a][b]);
       // what the next sweep takes as its panel goes there alone
       if (j >= k1 && j < k1 + kPanel) Pnext[static_cast<long long>(j - k1) * M + i] = v;
       else if (i >= k1 && i < k1 + kPanel) Pnext[static_cast<long long>(i - k1) * M + j] = make_double2(v.x, -v.y);
@@ -434,12 +464,6 @@ __global__ void __launch_bounds__(256) dense_sweep_kernel(double2* Sm, const dou
   }
 }
 
-
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-  v.x = warp_sum(v.x);
-  v.y = warp_sum(v.y);
-  return v;
-}
 
 // z = Q^-1 y (y complex64 [B][M]): one warp per row i, over column i of the
 // Hermitian R (z_i = sum_j conj(R[j][i]) y_j), coalesced.
@@ -494,37 +518,31 @@ __global__ void __launch_bounds__(256) dense_lag_sum_kernel(const double2* R, in
 // (offsets o1, o2) to the N1 x N2 grid:
 //   out[n1][n2] = sum_{e1,e2} S[e1][e2] exp(+2 pi i ((e1+o1) n1 / N1 + (e2+o2) n2 / N2))
 // pass 1: U[b][e1][n2]; pass 2: out (complex, or its real part).
-__global__ void dense_inv1_kernel(const double2* S, int B, int W1, int W2, int o2, int n2, const double2* tw2,
-                                  double2* U) {
-  const long long total = static_cast<long long>(B) * W1 * n2;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+__global__ void __launch_bounds__(256) dense_inv1_kernel(const double2* S, int B, int W1, int W2, int o2, int n2,
+                                                         const double2* tw2, double2* U) {
+  FBME_WARP_OUTPUTS(static_cast<long long>(B) * W1 * n2) {
     const int k2 = static_cast<int>(t % n2);
-    const long long r = t / n2;  // b * W1 + e1
-    const double2* row = S + r * W2;
-    double2 acc = make_double2(0.0, 0.0);
-    TwidStep tw(tw2, n2, static_cast<long long>(o2) * k2, k2);
-    for (int e2 = 0; e2 < W2; ++e2) acc = zadd(acc, zmul(row[e2], tw.next(+1)));
-    U[t] = acc;
+    const double2* row = S + t / n2 * W2;  // b * W1 + e1
+    const double2 v = warp_dft([&](int e) { return row[e]; }, W2, tw2, n2, static_cast<long long>(o2) * k2, k2, +1);
+    if ((threadIdx.x & 31) == 0) U[t] = v;
   }
 }
 template <bool REAL>
-__global__ void dense_inv2_kernel(const double2* U, int B, int W1, int o1, int n1, int n2, const double2* tw1,
-                                  double2* out, double* out_re) {
-  const long long total = static_cast<long long>(B) * n1 * n2;
-  for (long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; t < total;
-       t += static_cast<long long>(gridDim.x) * blockDim.x) {
+__global__ void __launch_bounds__(256) dense_inv2_kernel(const double2* U, int B, int W1, int o1, int n1, int n2,
+                                                         const double2* tw1, double2* out, double* out_re) {
+  FBME_WARP_OUTPUTS(static_cast<long long>(B) * n1 * n2) {
     const int k2 = static_cast<int>(t % n2);
     const long long r = t / n2;
-    const int k1 = static_cast<int>(r % n1), b = static_cast<int>(r / n1);
-    const double2* ub = U + static_cast<long long>(b) * W1 * n2 + k2;
-    double2 acc = make_double2(0.0, 0.0);
-    TwidStep tw(tw1, n1, static_cast<long long>(o1) * k1, k1);
-    for (int e1 = 0; e1 < W1; ++e1) acc = zadd(acc, zmul(tw.next(+1), ub[static_cast<long long>(e1) * n2]));
-    if (REAL)
-      out_re[t] = acc.x;
-    else
-      out[t] = acc;
+    const int k1 = static_cast<int>(r % n1);
+    const double2* ub = U + r / n1 * W1 * n2 + k2;
+    const double2 v = warp_dft([&](int e) { return ub[static_cast<long long>(e) * n2]; }, W1, tw1, n1,
+                               static_cast<long long>(o1) * k1, k1, +1);
+    if ((threadIdx.x & 31) == 0) {
+      if (REAL)
+        out_re[t] = v.x;
+      else
+        out[t] = v;
+    }
   }
 }
 
@@ -580,6 +598,11 @@ dense_finish_kernel(BatchShape s, const float* gamma, const double2* lift, const
   write_block_partial(acc, red, part, b, blockIdx.x, 0 * kPartWarps);
 }
 
+// Blocks of eight warps, one warp an output.
+int warp_grid(long long n) {
+  const long long g = (n + 7) / 8;
+  return static_cast<int>(g < 148 * 64 ? (g > 0 ? g : 1) : 148 * 64);
+}
 int grid_of(long long n) {
   const long long g = (n + 255) / 256;
   return static_cast<int>(g < 148 * 16 ? (g > 0 ? g : 1) : 148 * 16);
@@ -639,8 +662,8 @@ void dense_posterior(const BatchShape& s, const DenseBufs& d, const float* gamma
   const int B = s.B, M = static_cast<int>(s.m()), m1 = s.m1, m2 = s.m2, n1 = s.n1, n2 = s.n2;
   const int W1 = 2 * m1 - 1, W2 = 2 * m2 - 1;
   // lags of the prior and the data covariance
-  dense_lag1_kernel<<<grid_of(1LL * B * n1 * W2), 256, 0, st>>>(gamma, B, n1, n2, m2, d.tw2, d.pass);
-  dense_lag2_kernel<<<grid_of(1LL * B * W1 * W2), 256, 0, st>>>(d.pass, B, n1, m1, m2, d.tw1, d.lag);
+  dense_lag1_kernel<<<warp_grid(1LL * B * n1 * W2), 256, 0, st>>>(gamma, B, n1, n2, m2, d.tw2, d.pass);
+  dense_lag2_kernel<<<warp_grid(1LL * B * W1 * W2), 256, 0, st>>>(d.pass, B, n1, m1, m2, d.tw1, d.lag);
   dense_build_q_kernel<<<grid_of(1LL * B * M * M), 256, 0, st>>>(d.lag, B, m1, m2, noise, jitter, d.Q);
   // Q^-1 in place; the first panel is Q's first columns
   const int T = (M + kTile - 1) / kTile;
@@ -655,12 +678,12 @@ void dense_posterior(const BatchShape& s, const DenseBufs& d, const float* gamma
   dense_energy_kernel<<<B, 256, 0, st>>>(d.z, d.lag, noise, jitter, m1, m2, part);
   // data diagonal: Re N ifft2 of the lag sums
   dense_lag_sum_kernel<<<static_cast<int>((1LL * B * W1 * W2 + 7) / 8), 256, 0, st>>>(d.Q, B, m1, m2, d.lsum);
-  dense_inv1_kernel<<<grid_of(1LL * B * W1 * n2), 256, 0, st>>>(d.lsum, B, W1, W2, -(m2 - 1), n2, d.tw2, d.pass);
-  dense_inv2_kernel<true><<<grid_of(1LL * B * n1 * n2), 256, 0, st>>>(d.pass, B, W1, -(m1 - 1), n1, n2, d.tw1,
+  dense_inv1_kernel<<<warp_grid(1LL * B * W1 * n2), 256, 0, st>>>(d.lsum, B, W1, W2, -(m2 - 1), n2, d.tw2, d.pass);
+  dense_inv2_kernel<true><<<warp_grid(1LL * B * n1 * n2), 256, 0, st>>>(d.pass, B, W1, -(m1 - 1), n1, n2, d.tw1,
                                                                          nullptr, d.dd);
   // A^H Q^-1 y: the same transform of the M1 x M2 block
-  dense_inv1_kernel<<<grid_of(1LL * B * m1 * n2), 256, 0, st>>>(d.z, B, m1, m2, 0, n2, d.tw2, d.pass);
-  dense_inv2_kernel<false><<<grid_of(1LL * B * n1 * n2), 256, 0, st>>>(d.pass, B, m1, 0, n1, n2, d.tw1, d.lift,
+  dense_inv1_kernel<<<warp_grid(1LL * B * m1 * n2), 256, 0, st>>>(d.z, B, m1, m2, 0, n2, d.tw2, d.pass);
+  dense_inv2_kernel<false><<<warp_grid(1LL * B * n1 * n2), 256, 0, st>>>(d.pass, B, m1, 0, n1, n2, d.tw1, d.lift,
                                                                           nullptr);
   dense_finish_kernel<<<dim3(nb, B), kEwThreads, 0, st>>>(s, gamma, d.lift, d.dd, mean, relc, pv_out, part);
 }
