@@ -43,6 +43,7 @@
 #include <new>
 #include <string>
 #include <map>
+#include <type_traits>
 #include <vector>
 
 #include "dft_umma.cuh"
@@ -54,7 +55,11 @@ namespace fbme {
 constexpr int kCgRankMax = 32;
 constexpr int kCgSlice = 256;   // samples per block in the PCG vector kernels
 constexpr int kCgThreads = 256;
-constexpr int kCgChunk = 16;    // right-hand sides staged together in shared memory
+// Most right-hand sides staged together in shared memory: 17 takes the data
+// and 16 probes in one group, the data and 32 probes in two even ones (groups
+// of 16 left a third group of one, which staged a whole atom slice for it)
+constexpr int kCgChunk = 17;
+constexpr int kCgBatch = 4;     // right-hand sides whose loads a thread has in flight
 constexpr int kDSlots = 4;      // FP64 partials per (block, unit): rho', |r|^2, |b|^2
 constexpr int kFsLd = 33;       // padded row of the staged atom slice
 
@@ -166,43 +171,80 @@ struct ProDirection {
   FBME_DEV void tile_done(const TileCtx&, int, int) {}
 };
 
-// Adjoint-2 epilogue: prior[b] * (A^H v) into [unit][N1][N2].
+// The epilogues' operands (prior, direction, right-hand side) are loaded a
+// step of eight columns ahead of the accumulator they meet.
+
+// Adjoint-2 epilogue: prior[b] * (A^H v), the forward transform's input:
+// stored [unit][N1][N2] (EpiGamma), or as forward stage 1's A operand, split
+// into BF16 parts and swizzled (EpiGammaSplit, 3-term products).
+struct GammaPre {
+  float g[8];
+};
+FBME_DEV void gamma_prefetch(const TileCtx& t, int row, int c0, const float* gamma, int R, GammaPre& p) {
+  const DftGeom& g = *t.g;
+  const int r = t.row0() + row;
+  const float* gm = gamma + (t.scene / R) * g.out_stride + r;
+  const int jb = t.col0() + (c0 >> 1);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    p.g[i] = (r < g.rows && jb + i < g.cols) ? __ldg(gm + (jb + i) * g.out_ld) : 0.f;
+}
+
 struct EpiGamma {
-  using Pre = NoPre;
+  using Pre = GammaPre;
   float2* out;
   const float* gamma;
   int R;
-  FBME_DEV void prefetch(const TileCtx&, int, int, Pre&) const {}
-  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre&) const {
+  FBME_DEV void prefetch(const TileCtx& t, int row, int c0, Pre& p) const { gamma_prefetch(t, row, c0, gamma, R, p); }
+  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre& p) const {
     const DftGeom& g = *t.g;
     const int r = t.row0() + row;
     if (r >= g.rows) return;
-    const int b = t.scene / R;
     float2* o = out + t.scene * g.out_stride + r;
-    const float* gm = gamma + b * g.out_stride + r;
     const int jb = t.col0() + (c0 >> 1);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (jb + i < g.cols) {
-        const float gg = gm[(jb + i) * g.out_ld];
-        o[(jb + i) * g.out_ld] = make_float2(gg * v[2 * i], gg * v[2 * i + 1]);
-      }
-    }
+    for (int i = 0; i < 8; ++i)
+      if (jb + i < g.cols) o[(jb + i) * g.out_ld] = make_float2(p.g[i] * v[2 * i], p.g[i] * v[2 * i + 1]);
+  }
+  FBME_DEV void tile_done(const TileCtx&, int, int) {}
+};
+
+struct EpiGammaSplit {
+  using Pre = GammaPre;
+  EpiSplitT split;
+  const float* gamma;
+  int R;
+  FBME_DEV void prefetch(const TileCtx& t, int row, int c0, Pre& p) const { gamma_prefetch(t, row, c0, gamma, R, p); }
+  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre& p) const {
+    float s[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s[i] = p.g[i >> 1] * v[i];
+    split.consume(t, row, c0, s, NoPre());
   }
   FBME_DEV void tile_done(const TileCtx&, int, int) {}
 };
 
 // Forward-2 epilogue of Q d: q = acc + noise * d, partial Re(d^H q).
 struct EpiCurv {
-  using Pre = NoPre;
+  struct Pre {
+    float2 d[8];
+  };
   float2* q;
   const float2* d;
   const float* noise;
   double* part;
   int R;
   double acc;
-  FBME_DEV void prefetch(const TileCtx&, int, int, Pre&) const {}
-  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre&) {
+  FBME_DEV void prefetch(const TileCtx& t, int row, int c0, Pre& p) const {
+    const DftGeom& g = *t.g;
+    const int r = t.row0() + row, jb = t.col0() + (c0 >> 1);
+    const long long base = t.scene * g.out_stride + r;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      p.d[i] = (r < g.rows && jb + i < g.cols) ? d[base + static_cast<long long>(jb + i) * g.out_ld]
+                                               : make_float2(0.f, 0.f);
+  }
+  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre& p) {
     const DftGeom& g = *t.g;
     const int r = t.row0() + row;
     if (r >= g.rows) return;
@@ -213,7 +255,7 @@ struct EpiCurv {
     for (int i = 0; i < 8; ++i) {
       if (jb + i < g.cols) {
         const long long e = base + static_cast<long long>(jb + i) * g.out_ld;
-        const float2 dv = d[e];
+        const float2 dv = p.d[i];
         const float2 qq = make_float2(v[2 * i] + nv * dv.x, v[2 * i + 1] + nv * dv.y);
         q[e] = qq;
         acc += static_cast<double>(dv.x) * qq.x + static_cast<double>(dv.y) * qq.y;
@@ -228,14 +270,27 @@ struct EpiCurv {
 
 // Forward-2 epilogue of the true residual r = rhs - (acc + noise * x).
 struct EpiResid {
-  using Pre = NoPre;
+  struct Pre {
+    float2 x[8], b[8];
+  };
   float2* r;
   const float2* rhs;
   const float2* x;
   const float* noise;
   int R;
-  FBME_DEV void prefetch(const TileCtx&, int, int, Pre&) const {}
-  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre&) const {
+  FBME_DEV void prefetch(const TileCtx& t, int row, int c0, Pre& p) const {
+    const DftGeom& g = *t.g;
+    const int rr = t.row0() + row, jb = t.col0() + (c0 >> 1);
+    const long long base = t.scene * g.out_stride + rr;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const long long e = base + static_cast<long long>(jb + i) * g.out_ld;
+      const bool in = rr < g.rows && jb + i < g.cols;
+      p.x[i] = in ? x[e] : make_float2(0.f, 0.f);
+      p.b[i] = in ? rhs[e] : make_float2(0.f, 0.f);
+    }
+  }
+  FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre& p) const {
     const DftGeom& g = *t.g;
     const int rr = t.row0() + row;
     if (rr >= g.rows) return;
@@ -246,9 +301,8 @@ struct EpiResid {
     for (int i = 0; i < 8; ++i) {
       if (jb + i < g.cols) {
         const long long e = base + static_cast<long long>(jb + i) * g.out_ld;
-        const float2 xv = x[e], bv = rhs[e];
-        const float qx = v[2 * i] + nv * xv.x, qy = v[2 * i + 1] + nv * xv.y;
-        r[e] = make_float2(bv.x - qx, bv.y - qy);
+        const float qx = v[2 * i] + nv * p.x[i].x, qy = v[2 * i + 1] + nv * p.x[i].y;
+        r[e] = make_float2(p.b[i].x - qx, p.b[i].y - qy);
       }
     }
   }
@@ -315,13 +369,20 @@ __global__ void __launch_bounds__(256) cg_atoms_kernel(BatchShape s, int K, cons
   F[static_cast<long long>(b) * M * kCgRankMax + i] = f;
 }
 
-// Vector kernels: grid (sample blocks, scenes, groups of kCgChunk units).
+// Right-hand sides [c0, c0 + nc) of a vector kernel's group: the R of a scene
+// in gridDim.z even groups of at most kCgChunk.
+FBME_DEV int group_first(int R, int z, int groups) { return z * (R / groups) + min(z, R % groups); }
+
+// Vector kernels: grid (sample blocks, scenes, groups of units).
 // STEP: x += alpha d (and r -= alpha q when PROJ) with alpha of this
 // iteration; PROJ: per-block partials of F^H r; NORMS: partials of |r|^2
 // and |rhs|^2.  Block 0 of each scene and group records valid
-// (solver.py:5656-5663).
+// (solver.py:5656-5663).  A thread's loads of kCgBatch units are issued
+// together, and a warp's projections of its units share each atom entry (one
+// unit at a time, every load and every shared-memory read was waited for:
+// 151 us a step of 264 units of 128 x 128 samples, 92 us so).
 template <bool STEP, bool PROJ, bool NORMS>
-__global__ void __launch_bounds__(kCgThreads) cg_vector_kernel(const __grid_constant__ CgArgs A) {
+__global__ void __launch_bounds__(kCgThreads, 2) cg_vector_kernel(const __grid_constant__ CgArgs A) {
   extern __shared__ float2 cg_smem[];
   float2* Fs = cg_smem;                      // [kCgSlice][kFsLd]
   float2* Rs = cg_smem + kCgSlice * kFsLd;   // [kCgChunk][kCgSlice]
@@ -329,65 +390,82 @@ __global__ void __launch_bounds__(kCgThreads) cg_vector_kernel(const __grid_cons
   __shared__ double s_red[kCgThreads / 32][kCgChunk][2];
   const int b = blockIdx.y, blk = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.z * kCgChunk;
-  const int nc = min(kCgChunk, A.R - c0);
+  const int c0 = group_first(A.R, blockIdx.z, gridDim.z);
+  const int nc = group_first(A.R, blockIdx.z + 1, gridDim.z) - c0;
   const long long M = A.s.m();
   const long long m0 = static_cast<long long>(blk) * kCgSlice;
   const long long m = m0 + tid;
   const bool inb = m < M;
-  if (STEP && tid < nc) {
-    int ok = 0;
-    s_alpha[tid] = unit_alpha(A, b * A.R + c0 + tid, &ok);
-    if (blk == 0) A.valid[b * A.R + c0 + tid] = ok;
-  }
   if (PROJ && A.K > 0) {
+    // the atom slice, asynchronous; its rows past M are zero
     const float2* Fb = A.F + (static_cast<long long>(b) * M + m0) * kCgRankMax;
     const long long rows = min(static_cast<long long>(kCgSlice), M - m0);
     for (int e = tid; e < kCgSlice * kCgRankMax; e += kCgThreads) {
       const int row = e / kCgRankMax, k = e % kCgRankMax;
-      Fs[row * kFsLd + k] = row < rows ? Fb[e] : make_float2(0.f, 0.f);
+      float2* dst = Fs + row * kFsLd + k;
+      if (row < rows)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(Fb + e) : "memory");
+      else
+        *dst = make_float2(0.f, 0.f);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  __syncthreads();
-  for (int j = 0; j < nc; ++j) {
-    const long long unit = static_cast<long long>(b) * A.R + c0 + j;
-    const long long e = unit * M + m;
-    float2 rv = make_float2(0.f, 0.f);
-    if (inb) {
-      if (STEP) {
-        const float al = s_alpha[j];
-        const float2 dv = A.d[e];
-        float2 xv = A.x[e];
-        xv.x += al * dv.x;
-        xv.y += al * dv.y;
-        A.x[e] = xv;
-        if (PROJ) {
-          const float2 qv = A.q[e];
-          rv = A.r[e];
-          rv.x -= al * qv.x;
-          rv.y -= al * qv.y;
-          A.r[e] = rv;
+  if (STEP) {
+    if (tid < nc) {
+      int ok = 0;
+      s_alpha[tid] = unit_alpha(A, b * A.R + c0 + tid, &ok);
+      if (blk == 0) A.valid[b * A.R + c0 + tid] = ok;
+    }
+    __syncthreads();
+  }
+  const long long e0 = (static_cast<long long>(b) * A.R + c0) * M + m;
+  for (int j0 = 0; j0 < nc; j0 += kCgBatch) {
+    float2 dv[kCgBatch], xv[kCgBatch], qv[kCgBatch], rv[kCgBatch], bv[kCgBatch];
+#pragma unroll
+    for (int i = 0; i < kCgBatch; ++i) {
+      dv[i] = xv[i] = qv[i] = rv[i] = bv[i] = make_float2(0.f, 0.f);
+      if (inb && j0 + i < nc) {
+        const long long e = e0 + (j0 + i) * M;
+        if (STEP) {
+          dv[i] = A.d[e];
+          xv[i] = A.x[e];
+          if (PROJ) qv[i] = A.q[e];
         }
-      } else if (PROJ || NORMS) {
-        rv = A.r[e];
+        if (PROJ || NORMS) rv[i] = A.r[e];
+        if (NORMS) bv[i] = A.rhs[e];
       }
     }
-    if (PROJ) Rs[j * kCgSlice + tid] = rv;
-    if (NORMS) {
-      double rr = static_cast<double>(rv.x) * rv.x + static_cast<double>(rv.y) * rv.y;
-      double bb = 0.0;
-      if (inb) {
-        const float2 bv = A.rhs[e];
-        bb = static_cast<double>(bv.x) * bv.x + static_cast<double>(bv.y) * bv.y;
-      }
-      rr = warp_sum(rr);
-      bb = warp_sum(bb);
-      if (lane == 0) {
-        s_red[warp][j][0] = rr;
-        s_red[warp][j][1] = bb;
+#pragma unroll
+    for (int i = 0; i < kCgBatch; ++i) {
+      const int j = j0 + i;
+      if (j < nc) {
+        if (STEP && inb) {
+          const long long e = e0 + j * M;
+          const float al = s_alpha[j];
+          xv[i].x += al * dv[i].x;
+          xv[i].y += al * dv[i].y;
+          A.x[e] = xv[i];
+          if (PROJ) {
+            rv[i].x -= al * qv[i].x;
+            rv[i].y -= al * qv[i].y;
+            A.r[e] = rv[i];
+          }
+        }
+        if (PROJ) Rs[j * kCgSlice + tid] = rv[i];
+        if (NORMS) {
+          double rr = static_cast<double>(rv[i].x) * rv[i].x + static_cast<double>(rv[i].y) * rv[i].y;
+          double bb = static_cast<double>(bv[i].x) * bv[i].x + static_cast<double>(bv[i].y) * bv[i].y;
+          rr = warp_sum(rr);
+          bb = warp_sum(bb);
+          if (lane == 0) {
+            s_red[warp][j][0] = rr;
+            s_red[warp][j][1] = bb;
+          }
+        }
       }
     }
   }
+  if (PROJ) asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   if (NORMS && tid < nc) {
     double rr = 0.0, bb = 0.0;
@@ -400,20 +478,37 @@ __global__ void __launch_bounds__(kCgThreads) cg_vector_kernel(const __grid_cons
     dp[2] = bb;
   }
   if (PROJ && lane < A.K) {
-    // thread (k = lane, warp): units warp, warp + 8 of the group
-    for (int j = warp; j < nc; j += kCgThreads / 32) {
-      float ax = 0.f, ay = 0.f;
-      const float2* rs = Rs + j * kCgSlice;
-#pragma unroll 8
-      for (int tt = 0; tt < kCgSlice; ++tt) {
-        const float2 f = Fs[tt * kFsLd + lane];
-        const float2 rv = rs[tt];
-        ax += f.x * rv.x + f.y * rv.y;  // conj(f) * r
-        ay += f.x * rv.y - f.y * rv.x;
+    // thread (k = lane, warp): units warp, warp + 8, ... of the group, all
+    // of them against each atom entry; a unit's sum runs over the slice in
+    // order, its terms rounded one by one
+    constexpr int W = kCgThreads / 32, NU = (kCgChunk + W - 1) / W;
+    auto project = [&](auto count) {
+      constexpr int C = decltype(count)::value;
+      float ax[C], ay[C];
+#pragma unroll
+      for (int i = 0; i < C; ++i) ax[i] = ay[i] = 0.f;
+#pragma unroll 4
+      for (int tt = 0; tt < kCgSlice; tt += 2) {
+        const float2 f0 = Fs[tt * kFsLd + lane], f1 = Fs[(tt + 1) * kFsLd + lane];
+#pragma unroll
+        for (int i = 0; i < C; ++i) {
+          const float4 r2 = *reinterpret_cast<const float4*>(Rs + (warp + W * i) * kCgSlice + tt);
+          ax[i] = __fadd_rn(ax[i], fmaf(f0.x, r2.x, __fmul_rn(f0.y, r2.y)));  // conj(f) * r
+          ay[i] = __fadd_rn(ay[i], fmaf(f0.x, r2.y, -__fmul_rn(f0.y, r2.x)));
+          ax[i] = __fadd_rn(ax[i], fmaf(f1.x, r2.z, __fmul_rn(f1.y, r2.w)));
+          ay[i] = __fadd_rn(ay[i], fmaf(f1.x, r2.w, -__fmul_rn(f1.y, r2.z)));
+        }
       }
-      A.ppart[((static_cast<long long>(b) * A.nblk + blk) * A.R + c0 + j) * A.K + lane] =
-          make_float2(ax, ay);
-    }
+#pragma unroll
+      for (int i = 0; i < C; ++i)
+        A.ppart[((static_cast<long long>(b) * A.nblk + blk) * A.R + c0 + warp + W * i) * A.K + lane] =
+            make_float2(ax[i], ay[i]);
+    };
+    const int mine = nc > warp ? (nc - warp + W - 1) / W : 0;
+    static_assert(NU == 3, "one case per unit count");
+    if (mine == 3) project(std::integral_constant<int, 3>());
+    else if (mine == 2) project(std::integral_constant<int, 2>());
+    else if (mine == 1) project(std::integral_constant<int, 1>());
   }
 }
 
@@ -458,19 +553,27 @@ __global__ void __launch_bounds__(256) cg_weights_kernel(const __grid_constant__
 }
 
 // z = r / b - F w / b and partials of Re(r^H z) (solver.py:5836-5848);
-// grid as the vector kernels.
-__global__ void __launch_bounds__(kCgThreads) cg_precond_kernel(const __grid_constant__ CgArgs A) {
-  __shared__ float2 Ws[kCgChunk][kCgRankMax];
+// grid as the vector kernels.  A thread keeps its sample's atoms in
+// registers and takes kCgBatch units at a time: their residuals loaded
+// together, their sums over the atoms independent chains on shared weights
+// read in 16-byte pairs (one unit at a time 129 us for 264 units of 128 x 128
+// samples, 72 us so).  The terms' rounding is spelled out (a solve stopped at
+// a tolerance shows every changed bit).
+__global__ void __launch_bounds__(kCgThreads, 2) cg_precond_kernel(const __grid_constant__ CgArgs A) {
+  __shared__ __align__(16) float2 Ws[kCgChunk + kCgBatch - 1][kCgRankMax];
   __shared__ double s_red[kCgThreads / 32][kCgChunk];
   const int b = blockIdx.y, blk = blockIdx.x, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.z * kCgChunk;
-  const int nc = min(kCgChunk, A.R - c0);
+  const int c0 = group_first(A.R, blockIdx.z, gridDim.z);
+  const int nc = group_first(A.R, blockIdx.z + 1, gridDim.z) - c0;
   const long long M = A.s.m();
   const long long m = static_cast<long long>(blk) * kCgSlice + tid;
   const bool inb = m < M;
-  for (int i = tid; i < nc * A.K; i += blockDim.x)
-    Ws[i / A.K][i % A.K] = A.w[(static_cast<long long>(b) * A.R + c0) * A.K + i];
+  // weights past K and past the group are zero: their terms add +-0
+  for (int i = tid; i < (kCgChunk + kCgBatch - 1) * kCgRankMax; i += blockDim.x) {
+    const int j = i / kCgRankMax, k = i % kCgRankMax;
+    Ws[j][k] = (j < nc && k < A.K) ? A.w[(static_cast<long long>(b) * A.R + c0 + j) * A.K + k] : make_float2(0.f, 0.f);
+  }
   float2 f[kCgRankMax];
   if (A.K > 0 && inb) {
     const float4* fr = reinterpret_cast<const float4*>(A.F + (static_cast<long long>(b) * M + m) * kCgRankMax);
@@ -486,27 +589,43 @@ __global__ void __launch_bounds__(kCgThreads) cg_precond_kernel(const __grid_con
   }
   __syncthreads();
   const float bgv = A.bg[b];
-  for (int j = 0; j < nc; ++j) {
-    const long long unit = static_cast<long long>(b) * A.R + c0 + j;
-    const long long e = unit * M + m;
-    double rz = 0.0;
-    if (inb) {
-      const float2 rv = A.r[e];
-      float cx = 0.f, cy = 0.f;
+  const long long e0 = (static_cast<long long>(b) * A.R + c0) * M + m;
+  for (int j0 = 0; j0 < nc; j0 += kCgBatch) {
+    float2 rv[kCgBatch];
+    float cx[kCgBatch], cy[kCgBatch];
 #pragma unroll
-      for (int k = 0; k < kCgRankMax; ++k) {
-        if (k < A.K) {
-          const float2 ww = Ws[j][k];
-          cx += f[k].x * ww.x - f[k].y * ww.y;
-          cy += f[k].x * ww.y + f[k].y * ww.x;
-        }
-      }
-      const float2 zv = make_float2(rv.x / bgv - cx / bgv, rv.y / bgv - cy / bgv);
-      A.z[e] = zv;
-      rz = static_cast<double>(rv.x) * zv.x + static_cast<double>(rv.y) * zv.y;
+    for (int i = 0; i < kCgBatch; ++i) {
+      rv[i] = inb && j0 + i < nc ? A.r[e0 + (j0 + i) * M] : make_float2(0.f, 0.f);
+      cx[i] = cy[i] = 0.f;
     }
-    rz = warp_sum(rz);
-    if (lane == 0) s_red[warp][j] = rz;
+#pragma unroll
+    for (int k = 0; k < kCgRankMax; k += 2) {
+#pragma unroll
+      for (int i = 0; i < kCgBatch; ++i) {
+        const float4 w2 = *reinterpret_cast<const float4*>(&Ws[j0 + i][k]);
+        cx[i] = __fadd_rn(cx[i], fmaf(f[k].x, w2.x, -__fmul_rn(f[k].y, w2.y)));
+        cy[i] = __fadd_rn(cy[i], fmaf(f[k].y, w2.x, __fmul_rn(f[k].x, w2.y)));
+        cx[i] = __fadd_rn(cx[i], fmaf(f[k + 1].x, w2.z, -__fmul_rn(f[k + 1].y, w2.w)));
+        cy[i] = __fadd_rn(cy[i], fmaf(f[k + 1].y, w2.z, __fmul_rn(f[k + 1].x, w2.w)));
+      }
+    }
+    double rz[kCgBatch];
+#pragma unroll
+    for (int i = 0; i < kCgBatch; ++i) {
+      const float2 zv = make_float2(rv[i].x / bgv - cx[i] / bgv, rv[i].y / bgv - cy[i] / bgv);
+      rz[i] = 0.0;
+      if (inb && j0 + i < nc) {
+        A.z[e0 + (j0 + i) * M] = zv;
+        rz[i] = static_cast<double>(rv[i].x) * zv.x + static_cast<double>(rv[i].y) * zv.y;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kCgBatch; ++i) rz[i] = warp_sum(rz[i]);
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < kCgBatch; ++i)
+        if (j0 + i < nc) s_red[warp][j0 + i] = rz[i];
+    }
   }
   __syncthreads();
   if (tid < nc) {
@@ -954,6 +1073,12 @@ cudaError_t set_cg_attributes() {
   if ((e = set_attr_both<ProPlain, EpiCurv>()) != cudaSuccess) return e;
   if ((e = set_attr_both<ProPlain, EpiResid>()) != cudaSuccess) return e;
   if ((e = set_attr_both<ProPlain, EpiEnergy>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProPlain, EpiSplitT>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProDirection, EpiSplitT>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProSplit, EpiSplitT>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProSplit, EpiGammaSplit>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProSplit, EpiCurv>()) != cudaSuccess) return e;
+  if ((e = set_attr_both<ProSplit, EpiResid>()) != cudaSuccess) return e;
   const int vec_smem = (kCgSlice * kFsLd + kCgChunk * kCgSlice) * static_cast<int>(sizeof(float2));
   if ((e = cudaFuncSetAttribute(cg_vector_kernel<true, true, false>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize, vec_smem)) != cudaSuccess)
@@ -1068,9 +1193,14 @@ size_t CgBuffers::layout(const BatchShape& s, int pmax, int rank, int max_iter, 
   take(B * pmax * M * sizeof(float2) + 16);  // 6 pz
   take(B * pmax * N * sizeof(float2) + 16);  // 7 lp
   for (int v = 0; v < 8; ++v) take(U * M * sizeof(float2));  // 8..15 rhs x r z q d0 d1 best
-  take(U * static_cast<size_t>(s.n2) * s.m1 * sizeof(float2));  // 16 t1
-  take(U * N * sizeof(float2));              // 17 wide (prior-scaled / lifted)
-  take(U * static_cast<size_t>(s.m2) * s.n1 * sizeof(float2));  // 18 t2
+  // intermediates, FP32 or as the next stage's split operand (tile-padded)
+  auto mid = [](size_t rows, size_t k) {
+    return std::max(rows * k * sizeof(float2),
+                    static_cast<size_t>(split_unit_bytes(static_cast<int>(rows), static_cast<int>(k))));
+  };
+  take(U * mid(s.n2, s.m1));                 // 16 t1
+  take(U * mid(s.n1, s.n2));                 // 17 wide (prior-scaled / lifted)
+  take(U * mid(s.m2, s.n1));                 // 18 t2
   take(B * N * sizeof(float2));              // 19 mean
   take(B * N * sizeof(float2));              // 20 prev
   take(B * N * sizeof(float));               // 21 relc
@@ -1210,23 +1340,43 @@ void CgEngine::matvec(int R, const float2* v, bool direction, float2* out, bool 
   const DftGeom a2 = stage_geom_units(kAdj2, s, t, nt, U, R);
   const DftGeom f1 = stage_geom_units(kFwd1, s, t, nt, U, R);
   const DftGeom f2 = stage_geom_units(kFwd2, s, t, nt, U, R);
+  // 3-term products: every intermediate goes straight into the next stage's
+  // operand form (EpiSplitT / ProSplit), the prior-scaled lift included, whose
+  // rows are forward stage 1's contracted index; the values split are the
+  // same, so the results are too (264 units of 256^2 / 128^2: adjoint 2 148 ->
+  // 83 us with the prior loaded ahead, forward 1 66 -> 52, forward 2 92 -> 44)
+  const bool split = c.terms == 3;
+  auto split_of = [](float2* p, const DftGeom& g2) {
+    return EpiSplitT{reinterpret_cast<uint8_t*>(p), split_unit_bytes(g2.rows, g2.kcplx), g2.kchunks};
+  };
+  auto from = [](const float2* p, const DftGeom& g2) {
+    return ProSplit{reinterpret_cast<const uint8_t*>(p), split_unit_bytes(g2.rows, g2.kcplx)};
+  };
   const float2* src = v;
   if (direction) {
-    run_stage(c.terms, a1,
-              ProDirection{buf.z, buf.d[dcur], buf.d[dcur ^ 1], buf.beta, buf.dmask},
-              EpiStoreT{buf.t1}, buf.status, st);
+    const ProDirection pro{buf.z, buf.d[dcur], buf.d[dcur ^ 1], buf.beta, buf.dmask};
+    if (split) run_stage(c.terms, a1, pro, split_of(buf.t1, a2), buf.status, st);
+    else run_stage(c.terms, a1, pro, EpiStoreT{buf.t1}, buf.status, st);
     dcur ^= 1;
     src = buf.d[dcur];
+  } else if (split) {
+    run_stage(c.terms, a1, ProPlain{v}, split_of(buf.t1, a2), buf.status, st);
   } else {
     run_stage(c.terms, a1, ProPlain{v}, EpiStoreT{buf.t1}, buf.status, st);
   }
+  const EpiResid er{buf.r, buf.rhs, src, noise, R};
+  const EpiCurv ec{out, src, noise, buf.cpart, R, 0.0};
+  if (split) {
+    run_stage(c.terms, a2, from(buf.t1, a2), EpiGammaSplit{split_of(buf.wide, f1), prior, R}, buf.status, st);
+    run_stage(c.terms, f1, from(buf.wide, f1), split_of(buf.t2, f2), buf.status, st);
+    if (residual) run_stage(c.terms, f2, from(buf.t2, f2), er, buf.status, st);
+    else run_stage(c.terms, f2, from(buf.t2, f2), ec, buf.status, st);
+    return;
+  }
   run_stage(c.terms, a2, ProPlain{buf.t1}, EpiGamma{buf.wide, prior, R}, buf.status, st);
   run_stage(c.terms, f1, ProPlain{buf.wide}, EpiStoreT{buf.t2}, buf.status, st);
-  if (residual)
-    run_stage(c.terms, f2, ProPlain{buf.t2}, EpiResid{buf.r, buf.rhs, src, noise, R}, buf.status, st);
-  else
-    run_stage(c.terms, f2, ProPlain{buf.t2}, EpiCurv{out, src, noise, buf.cpart, R, 0.0}, buf.status,
-              st);
+  if (residual) run_stage(c.terms, f2, ProPlain{buf.t2}, er, buf.status, st);
+  else run_stage(c.terms, f2, ProPlain{buf.t2}, ec, buf.status, st);
 }
 
 void CgEngine::precond_build(cudaStream_t st) {

@@ -581,6 +581,10 @@ struct EpiSplitT {
     const DftGeom& g = *t.g;
     const int r = t.row0() + row;
     if (r >= kchunks2 * 32) return;
+    // rows past this stage's are zeros of the next stage's contraction; the
+    // accumulators there come from operand rows that nothing wrote when this
+    // stage's own operand was pre-split
+    const bool in = r < g.rows;
     const int kc = r >> 5, w = r & 31;
     uint8_t* base = out + t.scene * unit_bytes + static_cast<size_t>(kc) * 2 * kPartBytesA;
     const int jb = t.col0() + (c0 >> 1);
@@ -588,7 +592,7 @@ struct EpiSplitT {
     for (int i = 0; i < 8; ++i) {
       const int c = jb + i;
       if (c >= g.cols) continue;
-      const float2 x = make_float2(v[2 * i], v[2 * i + 1]);
+      const float2 x = in ? make_float2(v[2 * i], v[2 * i + 1]) : make_float2(0.f, 0.f);
       const __nv_bfloat162 hi = __float22bfloat162_rn(x);
       const float2 h = __bfloat1622float2(hi);
       const __nv_bfloat162 lo = __float22bfloat162_rn(make_float2(x.x - h.x, x.y - h.y));
