@@ -381,6 +381,7 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, int n,
 // start of x8 -- the network's first layer takes f1 from the partials.
 __global__ void __launch_bounds__(256) features_kernel(int pass, const float2* bp, int B, long long N,
                                                        __nv_bfloat16* x8, double* part, bool compact = false) {
+  dep_sync();
   __shared__ double red[32];
   const int b = blockIdx.y;
   double acc = 0.0;
@@ -502,6 +503,7 @@ FBME_DEV void prior_strip(const float (&o)[kFStrip], float base, float fl, float
 __global__ void __launch_bounds__(kFThreads) warm_map_kernel(const float* map, int H, int W,
                                                             const float* data_power, const float* floor_,
                                                             float* gamma, double* upart, int nslots) {
+  dep_sync();
   __shared__ double red[32];
   const int b = blockIdx.y;
   const long long img = static_cast<long long>(b) * H * W;
@@ -574,6 +576,7 @@ static_assert(kF1N % 16 == 0, "layer 1: every fragment row is a region pixel");
 
 template <bool TRAIN, int CSTR>
 __global__ void __launch_bounds__(kFThreads, 3) net_tile_kernel(NetArgs a) {
+  dep_sync();
   extern __shared__ __align__(16) uint8_t fsm[];
   __shared__ double red[32];
   float* z = reinterpret_cast<float*>(fsm);         // [9][kF2N]
@@ -908,6 +911,7 @@ int feature_parts(int H, int W) {
 // initialisation's sum of the backprojection power): partial 0 holds it,
 // the other partials of the pass zero.
 __global__ void seed_feature_sum_kernel(const float* ebp, int B, int parts, double* part) {
+  dep_sync();
   const int b = blockIdx.x, k = threadIdx.x;
   if (b < B && k < parts) part[b * 128 + k] = k == 0 ? static_cast<double>(ebp[b]) : 0.0;
 }
@@ -920,7 +924,7 @@ void features_passes(const float2* bp, int B, int H, int W, void* ws, int passes
   auto* x8 = reinterpret_cast<__nv_bfloat16*>(w + L.x8);
   auto* fpart = reinterpret_cast<double*>(w + L.fpart);
   for (int pass = first; pass < passes; ++pass)
-    features_kernel<<<dim3(feature_parts(H, W), B), 256, 0, st>>>(pass, bp, B, static_cast<long long>(H) * W,
+    launch_dep(features_kernel, dim3(feature_parts(H, W), B), 256, 0, st, pass, bp, B, static_cast<long long>(H) * W,
                                                                   x8, fpart, compact);
 }
 }  // namespace
@@ -1014,7 +1018,7 @@ void cnn_warm_prior(const float* params, const float2* bp, int B, int H, int W, 
   // f0 alone, one BF16 per pixel (the network takes f1 from the partials);
   // with the backprojection power `ebp` the statistics pass is not repeated
   if (ebp) {
-    seed_feature_sum_kernel<<<B, 64, 0, st>>>(ebp, B, feature_parts(H, W), fpart);
+    launch_dep(seed_feature_sum_kernel, B, 64, 0, st, ebp, B, feature_parts(H, W), fpart);
     features_passes(bp, B, H, W, ws, 2, st, true, 1);
   } else {
     features_passes(bp, B, H, W, ws, 2, st, true);
@@ -1031,13 +1035,13 @@ void cnn_warm_prior(const float* params, const float2* bp, int B, int H, int W, 
   na.gamma = gamma;
   na.upart = upart;
   na.nslots = nblocks;
-  net_tile_kernel<false, 1><<<dim3(warm_ctas(H, W, nblocks), B), kFThreads, kFSmem, st>>>(na);
+  launch_dep(net_tile_kernel<false, 1>, dim3(warm_ctas(H, W, nblocks), B), kFThreads, kFSmem, st, na);
 }
 
 void warm_prior_from_map(const float* map, int B, int H, int W, const float* data_power, const float* floor_,
                          float* gamma, double* upart, int nblocks, cudaStream_t st) {
   using namespace cnn;
-  warm_map_kernel<<<dim3(warm_ctas(H, W, nblocks), B), kFThreads, 0, st>>>(map, H, W, data_power, floor_, gamma,
+  launch_dep(warm_map_kernel, dim3(warm_ctas(H, W, nblocks), B), kFThreads, 0, st, map, H, W, data_power, floor_, gamma,
                                                                           upart, nblocks);
 }
 

@@ -30,6 +30,38 @@ static inline int sm_count() {
 }
 
 // ---------------------------------------------------------------------------
+// dependent launches
+// ---------------------------------------------------------------------------
+// A replay is a chain of 20-40 kernels, each of a few microseconds for small
+// batches, so the gap between two kernels counts: launch_dep lets a kernel's
+// launch overlap the completion of its predecessor in the stream.  Every
+// kernel launched so begins with dep_sync in all its threads, which waits
+// until the predecessor has completed and its writes are visible; because
+// every kernel of the chain waits, completion stays ordered along the whole
+// chain.  Kernels launched the plain way pass dep_sync at once.  Measured
+// (B200, captured replays, us): one 256x256 Fast scene 176 -> 162, 16 masked
+// scenes 330 -> 308, one 40x32 Stable scene 222 -> 220, 512 scenes 3165 -> 3160.
+// No kernel allows the next one's launch before its own end
+// (griddepcontrol.launch_dependents): the waiting blocks then settle beside
+// the running ones, and the same replays took 204, 349, 234 and 3199 us.
+FBME_DEV void dep_sync() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline void launch_dep(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// ---------------------------------------------------------------------------
 // complex helpers (interleaved complex64 as float2)
 // ---------------------------------------------------------------------------
 FBME_DEV float2 cmul(float2 a, float2 b) {

@@ -216,6 +216,7 @@ dft_stage_kernel(const __grid_constant__ StageSet<Pro, Epi, NI> set) {
     fence_mbar_init();
   }
   if (warp == kMmaWarp) tmem_alloc(tmem_slot, 2 * N_TILE);
+  dep_sync();  // the set-up above reads nothing of the predecessor's
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

@@ -177,6 +177,7 @@ FBME_DEV int fft_set_item(const FftSet<NMAX>& set, int t) {
 }
 
 __global__ void __launch_bounds__(kFftThreads) fft_stage_kernel(const FftStage S, const FftIo io) {
+  dep_sync();
   extern __shared__ float2 fsm[];
   const int unit = blockIdx.y, tile = blockIdx.x;
   const int rt = S.p.rows_per_cta, L = S.p.L, pitch = L + 1;
@@ -427,6 +428,7 @@ FBME_DEV void fast_issue(const FftStage& st, const FftIo& io, int t, float2* buf
 // EPI: 0 store (modes 0 and 1), 1 residual (mode 2), 2 denoiser (mode 3)
 template <int L, int S, int EPI>
 __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage st, const FftIo io) {
+  dep_sync();
   constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P;
   constexpr int J = (Q + P - 1) / P;     // output columns k1 per thread in pass 2
   constexpr int A = fast_row_area(L);    // row stride of a buffer
@@ -653,6 +655,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
 // kernel, so that the single-stage kernel keeps its code.
 template <int L, int S, int EPI, int NMAX>
 __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftSet<NMAX> set) {
+  dep_sync();
   constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P;
   constexpr int J = (Q + P - 1) / P;     // output columns k1 per thread in pass 2
   constexpr int A = fast_row_area(L);    // row stride of a buffer
@@ -894,7 +897,7 @@ void launch_fast_as(const FftStage& S_, const FftIo& io, cudaStream_t st) {
   const long long total = static_cast<long long>(S_.tiles) * S_.units;
   const long long cap = static_cast<long long>(sm_count()) * per_sm;
   const int grid = static_cast<int>(total < cap ? total : cap);
-  if (grid > 0) kern<<<grid, kFftThreads, fast_smem_bytes(L), st>>>(S_, io);
+  if (grid > 0) launch_dep(kern, grid, kFftThreads, fast_smem_bytes(L), st, S_, io);
 }
 
 template <int L, int S, int EPI>
@@ -1072,7 +1075,7 @@ void fft_stage(const DftGeom& g, int L, int sign, const float2* tw, const float2
     case 32: launch_fast<32>(S, io, sign, st); return;
     default: break;
   }
-  fft_stage_kernel<<<dim3(S.tiles, g.n_scenes), kFftThreads, fft_smem_bytes(L), st>>>(S, io);
+  launch_dep(fft_stage_kernel, dim3(S.tiles, g.n_scenes), kFftThreads, fft_smem_bytes(L), st, S, io);
 }
 
 // The same-length stages of several shape buckets in one launch of the

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(256) gram_pass2_kernel(const double2* r, int m
 // Masked copy of the caller's data: out[b][m] = mask[m] ? y[b][m] : 0.
 __global__ void __launch_bounds__(256) mask_data_kernel(const float2* y, const uint8_t* mask, long long m,
                                                         float2* out) {
+  dep_sync();
   const long long scene = blockIdx.y;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < m;
        i += static_cast<long long>(gridDim.x) * blockDim.x)
@@ -116,7 +117,7 @@ cudaError_t mask_setup(const BatchShape& s, const uint8_t* mask_in, uint8_t* mas
 void mask_data(const BatchShape& s, const float2* y, const uint8_t* mask, float2* out, cudaStream_t st) {
   const long long m = s.m();
   const long long blocks = (m + 255) / 256;
-  mask_data_kernel<<<dim3(static_cast<unsigned>(blocks < 256 ? blocks : 256), s.B), 256, 0, st>>>(y, mask, m, out);
+  launch_dep(mask_data_kernel, dim3(static_cast<unsigned>(blocks < 256 ? blocks : 256), s.B), 256, 0, st, y, mask, m, out);
 }
 
 }  // namespace fbme

@@ -568,6 +568,7 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int s
   if (threadIdx.x == 0 && S.status) atomicOr(&A.p.status[scene], S.status);
 }
 __global__ void __launch_bounds__(kPolishThreads) polish_kernel(PolishArgs A, int phase) {
+  dep_sync();
   __shared__ PolishShared S;
   polish_body(A, S, phase, blockIdx.x);
 }
@@ -754,6 +755,7 @@ FBME_DEV void exchange_body(const PolishArgs& A, uint32_t* cand_key, int* cand_i
 template <typename T>
 __global__ void __launch_bounds__(T::threads, 2)
 exchange_kernel(PolishArgs A, uint32_t* cand_key, int* cand_idx) {
+  dep_sync();
   exchange_body<T>(A, cand_key, cand_idx, blockIdx.y, blockIdx.x, gridDim.x);
 }
 
@@ -838,6 +840,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, PolishShared& S, const Fbm
   }
 }
 __global__ void __launch_bounds__(kPolishThreads) polish_finish_kernel(PolishArgs A, FbmeOutputs out) {
+  dep_sync();
   __shared__ PolishShared S;
   polish_finish_body(A, S, out, blockIdx.x);
 }
@@ -1098,6 +1101,7 @@ FBME_DEV CertBest cert_merge(void* ws, int B, int scene, int nblk) {
 // final certificate (solver.py:4851-4870, 5388-5460).
 __global__ void __launch_bounds__(kPolishThreads) cert_step_kernel(PolishArgs A, FbmeCertificate C, void* ws,
                                                                    int nblk, int t) {
+  dep_sync();
   __shared__ PolishShared S;
   extern __shared__ float2 dtab[];
   const int scene = blockIdx.x;
@@ -1214,6 +1218,7 @@ __global__ void __launch_bounds__(kPolishThreads) cert_step_kernel(PolishArgs A,
 // Block (bx, scene) scores atoms [bx chunk, (bx + 1) chunk) against the
 // staged model and writes its best to the scene's partials.
 __global__ void __launch_bounds__(kCertThreads, 3) cert_scan_kernel(PolishArgs A, void* ws) {
+  dep_sync();
   __shared__ __align__(16) float2 M[32][34];
   __shared__ CertModel model;
   __shared__ CertBest red[kCertThreads / 32];
@@ -1289,6 +1294,7 @@ FBME_DEV void output_body(const PolishArgs& A, const FbmeOutputs& out, int scene
   }
 }
 __global__ void __launch_bounds__(256) output_kernel(PolishArgs A, FbmeOutputs out) {
+  dep_sync();
   output_body(A, out, blockIdx.y, blockIdx.x, gridDim.x);
 }
 
@@ -1312,6 +1318,7 @@ static_assert(sizeof(PolishSet) <= 32764, "kernel parameter limit");
 FBME_DEV bool has_exchange(const DevConfig& c) { return c.exchange > 0 && c.polish_iters > 1; }
 
 __global__ void __launch_bounds__(kPolishThreads) polish_set_kernel(const PolishSet set, int phase) {
+  dep_sync();
   __shared__ PolishShared S;
   const PolishArgs& A = set.a[blockIdx.z];
   if (phase == 1 && !has_exchange(A.c)) return;
@@ -1320,6 +1327,7 @@ __global__ void __launch_bounds__(kPolishThreads) polish_set_kernel(const Polish
 
 template <typename T>
 __global__ void __launch_bounds__(T::threads, 2) exchange_set_kernel(const PolishSet S) {
+  dep_sync();
   const PolishArgs& A = S.a[blockIdx.z];
   const int nbx = S.ex_blocks[blockIdx.z];
   if (static_cast<int>(blockIdx.x) >= nbx || static_cast<int>(blockIdx.y) >= A.s.B) return;
@@ -1327,11 +1335,13 @@ __global__ void __launch_bounds__(T::threads, 2) exchange_set_kernel(const Polis
 }
 
 __global__ void __launch_bounds__(kPolishThreads) polish_finish_set_kernel(const PolishSet set) {
+  dep_sync();
   __shared__ PolishShared S;
   polish_finish_body(set.a[blockIdx.z], S, set.out[blockIdx.z], blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256) output_set_kernel(const PolishSet S) {
+  dep_sync();
   const int nbx = S.out_blocks[blockIdx.z];
   if (static_cast<int>(blockIdx.x) >= nbx || static_cast<int>(blockIdx.y) >= S.a[blockIdx.z].s.B) return;
   output_body(S.a[blockIdx.z], S.out[blockIdx.z], blockIdx.y, blockIdx.x, nbx);
@@ -1370,6 +1380,7 @@ cudaError_t set_polish_attributes() {
 // top-E selection; active atoms get key 0 (the reference's -inf).  One
 // thread per grid point; the table lookups hit L2.
 __global__ void __launch_bounds__(256) exchange_masked_kernel(PolishArgs A) {
+  dep_sync();
   __shared__ int atom1[kMaxPolish], atom2[kMaxPolish], atom[kMaxPolish];
   __shared__ float2 amu[kMaxPolish];
   const int scene = blockIdx.y;
@@ -1404,7 +1415,7 @@ __global__ void __launch_bounds__(256) exchange_masked_kernel(PolishArgs A) {
 template <typename T>
 static void launch_exchange(const PolishArgs& A, const PolishBuffers& p, cudaStream_t st) {
   const dim3 grid(exchange_blocks(A.s), A.s.B);
-  exchange_kernel<T><<<grid, T::threads, T::smem_bytes(A.s.n2), st>>>(A, p.cand_key, p.cand_idx);
+  launch_dep(exchange_kernel<T>, grid, T::threads, T::smem_bytes(A.s.n2), st, A, p.cand_key, p.cand_idx);
 }
 
 void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
@@ -1416,17 +1427,17 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
   FBME_TIMED(prof, FBME_GROUP_TOPK,
              launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * K, K, s.B, p.active, p.score, st));
   const size_t dsm = (s.n1 + s.n2) * sizeof(float2);
-  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 0)));
+  FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 0)));
   if (c.exchange > 0 && c.polish_iters > 1 && p.gram2d) {
     const long long nblk = (s.n() + 255) / 256;
     FBME_TIMED(prof, FBME_GROUP_EXCHANGE,
-               (exchange_masked_kernel<<<dim3(static_cast<unsigned>(nblk < 1024 ? nblk : 1024), s.B), 256, 0, st>>>(A)));
+               (launch_dep(exchange_masked_kernel, dim3(static_cast<unsigned>(nblk < 1024 ? nblk : 1024), s.B), 256, 0, st, A)));
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_blocks(p.keys, s.n(), c.exchange, s.B, p.cand_key, p.cand_idx, st));
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * c.exchange, c.exchange, s.B,
                                  p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1)));
   } else if (c.exchange > 0 && c.polish_iters > 1) {
     const int nb = exchange_blocks(s);
     if (s.n2 <= 64)
@@ -1440,7 +1451,7 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_merge(p.cand_key, p.cand_idx, nb * c.exchange, c.exchange, s.B,
                                  p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1)));
   }
   if (cert) {  // model, scan, (decide + model, scan) per repair, final
     int resident = 1;
@@ -1450,15 +1461,15 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     const int nblk = cert_blocks(s, resident);
     for (int t = 0; t <= c.repairs + 1; ++t) {
       FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
-                 (cert_step_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, *cert, cert->workspace, nblk, t)));
+                 (launch_dep(cert_step_kernel, s.B, kPolishThreads, dsm, st, A, *cert, cert->workspace, nblk, t)));
       if (t <= c.repairs)
         FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
-                   (cert_scan_kernel<<<dim3(nblk, s.B), kCertThreads, dsm, st>>>(A, cert->workspace)));
+                   (launch_dep(cert_scan_kernel, dim3(nblk, s.B), kCertThreads, dsm, st, A, cert->workspace)));
     }
   }
-  FBME_TIMED(prof, FBME_GROUP_POLISH, (polish_finish_kernel<<<s.B, kPolishThreads, dsm, st>>>(A, out)));
+  FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_finish_kernel, s.B, kPolishThreads, dsm, st, A, out)));
   const int fb = static_cast<int>((s.n() + 2047) / 2048);
-  FBME_TIMED(prof, FBME_GROUP_OUTPUT, (output_kernel<<<dim3(fb < 64 ? fb : 64, s.B), 256, 0, st>>>(A, out)));
+  FBME_TIMED(prof, FBME_GROUP_OUTPUT, (launch_dep(output_kernel, dim3(fb < 64 ? fb : 64, s.B), 256, 0, st, A, out)));
 }
 
 // The polish of an uneven plan's buckets, one launch per step over all of
@@ -1468,7 +1479,7 @@ static int exchange_class(int n2) { return n2 <= 64 ? 0 : n2 <= 128 ? 1 : n2 <= 
 
 template <typename T>
 static void launch_exchange_set(const PolishSet& S, int max_blocks, int max_b, int max_n2, cudaStream_t st) {
-  exchange_set_kernel<T><<<dim3(max_blocks, max_b, S.n), T::threads, T::smem_bytes(max_n2), st>>>(S);
+  launch_dep(exchange_set_kernel<T>, dim3(max_blocks, max_b, S.n), T::threads, T::smem_bytes(max_n2), st, S);
 }
 
 void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
@@ -1511,7 +1522,7 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
     }
     launch_topk_blocks_multi(tj, max_slices, max_b, st);
     launch_topk_merge_multi(tm, max_b, st);
-    polish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S, 0);
+    launch_dep(polish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S, 0);
     // the exchange, one launch per row-tile class, then its candidates' merge
     bool any = false;
     for (int cls = 0; cls < 4; ++cls) {
@@ -1547,10 +1558,10 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
                                     A.p.xcand_val};
       }
       launch_topk_merge_multi(tx, max_b, st);
-      polish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S, 1);
+      launch_dep(polish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S, 1);
     }
-    polish_finish_set_kernel<<<dim3(max_b, 1, m), kPolishThreads, dsm, st>>>(*S);
-    output_set_kernel<<<dim3(max_out, max_b, m), 256, 0, st>>>(*S);
+    launch_dep(polish_finish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S);
+    launch_dep(output_set_kernel, dim3(max_out, max_b, m), 256, 0, st, *S);
     for (int i = 0; i < m; ++i) {
       const PolishBucket& k = b[plain[i]];
       if (k.out.status && k.out.status != k.p.status)

@@ -161,8 +161,12 @@ static cudaError_t set_attr() {
 template <int A_PARTS, int N_TILE, class Pro, class Epi, int NI>
 static void launch_set(const StageSet<Pro, Epi, NI>& set, cudaStream_t st) {
   const int t = set.tile0[set.n], s = sm_count();
-  dft_stage_kernel<A_PARTS, N_TILE, Pro, Epi, NI>
-      <<<t < s ? t : s, kDftPersistThreads, DftCfg<A_PARTS, N_TILE>::kSmemBytes, st>>>(set);
+  if constexpr (NI == 1)
+    launch_dep(dft_stage_kernel<A_PARTS, N_TILE, Pro, Epi, NI>, t < s ? t : s, kDftPersistThreads,
+               DftCfg<A_PARTS, N_TILE>::kSmemBytes, st, set);
+  else
+    dft_stage_kernel<A_PARTS, N_TILE, Pro, Epi, NI>
+        <<<t < s ? t : s, kDftPersistThreads, DftCfg<A_PARTS, N_TILE>::kSmemBytes, st>>>(set);
 }
 
 template <int A_PARTS, int N_TILE, class Pro, class Epi>

@@ -51,12 +51,14 @@ FBME_DEV void topk_blocks_body(const void* in, long long n, int k, uint32_t* can
 template <bool FROM_SCORES>
 __global__ void __launch_bounds__(kTopkBlockThreads, 2)
 topk_blocks_kernel(const void* in, long long n, int k, uint32_t* cand_key, int* cand_idx) {
+  dep_sync();
   topk_blocks_body<FROM_SCORES>(in, n, k, cand_key, cand_idx, blockIdx.y, blockIdx.x, gridDim.x);
 }
 
 // Several shape buckets' slices in one launch (blockIdx.z: the bucket;
 // blocks past a bucket's own slices or scenes return).
 __global__ void __launch_bounds__(kTopkBlockThreads, 2) topk_blocks_multi_kernel(const TopkJobs J) {
+  dep_sync();
   const TopkJob& j = J.j[blockIdx.z];
   const int nblk = topk_slices_dev(j.n);
   if (static_cast<int>(blockIdx.x) >= nblk || static_cast<int>(blockIdx.y) >= j.B) return;
@@ -106,10 +108,12 @@ template <typename Idx>
 __global__ void __launch_bounds__(1024)
 topk_merge_kernel(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, Idx* out_idx,
                   float* out_val) {
+  dep_sync();
   topk_merge_body<Idx>(cand_key, cand_idx, ncand, k, out_idx, out_val, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(1024) topk_merge_multi_kernel(const TopkMergeJobs J) {
+  dep_sync();
   const TopkMergeJob& j = J.j[blockIdx.z];
   if (static_cast<int>(blockIdx.x) >= j.B) return;
   topk_merge_body<int>(j.cand_key, j.cand_idx, j.ncand, j.k, j.out_idx, j.out_val, blockIdx.x);
@@ -118,27 +122,26 @@ __global__ void __launch_bounds__(1024) topk_merge_multi_kernel(const TopkMergeJ
 int topk_slices(long long n) { return static_cast<int>((n + kTopkSlice - 1) / kTopkSlice); }
 
 void launch_topk_blocks_multi(const TopkJobs& J, int max_slices, int max_b, cudaStream_t st) {
-  topk_blocks_multi_kernel<<<dim3(max_slices, max_b, J.n), kTopkBlockThreads, 0, st>>>(J);
+  launch_dep(topk_blocks_multi_kernel, dim3(max_slices, max_b, J.n), kTopkBlockThreads, 0, st, J);
 }
 void launch_topk_merge_multi(const TopkMergeJobs& J, int max_b, cudaStream_t st) {
-  topk_merge_multi_kernel<<<dim3(max_b, 1, J.n), 1024, 0, st>>>(J);
+  launch_dep(topk_merge_multi_kernel, dim3(max_b, 1, J.n), 1024, 0, st, J);
 }
 
 void launch_topk_blocks(const uint32_t* keys, long long n, int k, int B, uint32_t* cand_key, int* cand_idx,
                         cudaStream_t st) {
-  topk_blocks_kernel<false>
-      <<<dim3(topk_slices(n), B), kTopkBlockThreads, 0, st>>>(keys, n, k, cand_key, cand_idx);
+  launch_dep(topk_blocks_kernel<false>, dim3(topk_slices(n), B), kTopkBlockThreads, 0, st, keys, n, k, cand_key, cand_idx);
 }
 
 void launch_topk(const uint32_t* keys, long long n, int k, int B, uint32_t* cand_key, int* cand_idx,
                  int* out_idx, float* out_val, cudaStream_t st) {
   launch_topk_blocks(keys, n, k, B, cand_key, cand_idx, st);
-  topk_merge_kernel<int><<<B, 1024, 0, st>>>(cand_key, cand_idx, topk_slices(n) * k, k, out_idx, out_val);
+  launch_dep(topk_merge_kernel<int>, B, 1024, 0, st, cand_key, cand_idx, topk_slices(n) * k, k, out_idx, out_val);
 }
 
 void launch_topk_merge(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, int B,
                        int* out_idx, float* out_val, cudaStream_t st) {
-  topk_merge_kernel<int><<<B, 1024, 0, st>>>(cand_key, cand_idx, ncand, k, out_idx, out_val);
+  launch_dep(topk_merge_kernel<int>, B, 1024, 0, st, cand_key, cand_idx, ncand, k, out_idx, out_val);
 }
 
 // Candidate scratch of the score top-k: per row, one k-list per 8192-score slice.
@@ -163,8 +166,8 @@ void topk_scores(const float* scores, long long n, int k, int batch, void* scrat
   const int nblk = topk_slices(n);
   uint32_t* ck = static_cast<uint32_t*>(scratch);
   int* ci = reinterpret_cast<int*>(ck + static_cast<size_t>(batch) * nblk * k);
-  topk_blocks_kernel<true><<<dim3(nblk, batch), kTopkBlockThreads, 0, st>>>(scores, n, k, ck, ci);
-  topk_merge_kernel<int64_t><<<batch, 1024, 0, st>>>(ck, ci, nblk * k, k, indices, values);
+  launch_dep(topk_blocks_kernel<true>, dim3(nblk, batch), kTopkBlockThreads, 0, st, scores, n, k, ck, ci);
+  launch_dep(topk_merge_kernel<int64_t>, batch, 1024, 0, st, ck, ci, nblk * k, k, indices, values);
 }
 
 }  // namespace fbme

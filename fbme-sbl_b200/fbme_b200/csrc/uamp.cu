@@ -184,6 +184,7 @@ FBME_DEV void gamma0_body(Blk k, BatchShape s, DevConfig c, Scalars sc, const fl
 __global__ void __launch_bounds__(kEwThreads) gamma0_kernel(BatchShape s, DevConfig c, Scalars sc,
                                                             const float2* bp, float* gamma,
                                                             double* part) {
+  dep_sync();
   gamma0_body(blk_here(), s, c, sc, bp, gamma, part);
 }
 
@@ -239,6 +240,7 @@ FBME_DEV void denoise_body(Blk k, BatchShape s, DenoiseArgs a, const float2* lif
   write_block_partial(sv, red, a.part, scene, k.x, 1 * kPartWarps);
 }
 __global__ void __launch_bounds__(kEwThreads) denoise_kernel(BatchShape s, DenoiseArgs a, const float2* lift) {
+  dep_sync();
   denoise_body(blk_here(), s, a, lift);
 }
 
@@ -287,6 +289,7 @@ FBME_DEV void message_body(Blk k, BatchShape s, const float2* y, const float2* p
 __global__ void __launch_bounds__(kEwThreads)
 message_kernel(BatchShape s, const float2* y, const float2* pred, const float2* msg_in, float2* msg_out,
                const float* prec, const float* dvar, float damping, const uint8_t* mask) {
+  dep_sync();
   message_body(blk_here(), s, y, pred, msg_in, msg_out, prec, dvar, damping, mask);
 }
 
@@ -350,6 +353,7 @@ __global__ void __launch_bounds__(kEwThreads) sweep1_kernel(BatchShape s, DevCon
                                                             DenoiseArgs a, const float2* bp,
                                                             const float2* y, float2* msg,
                                                             int nblk_n) {
+  dep_sync();
   sweep1_body(blk_here(), s, c, sc, a, bp, y, msg, nblk_n);
 }
 
@@ -426,6 +430,7 @@ FBME_DEV void scalars_body(Blk k, int mode, BatchShape s, DevConfig c, Scalars s
 __global__ void __launch_bounds__(32 * kScalarScenesPerBlock)
 scalars_kernel(int mode, BatchShape s, DevConfig c, Scalars sc, const double* part, PartSrc p0, PartSrc p1,
                PartSrc p2) {
+  dep_sync();
   scalars_body(blk_here(), mode, s, c, sc, part, p0, p1, p2);
 }
 
@@ -655,15 +660,15 @@ void sbl_init(const BatchShape& s, const DftTables& t, const DevConfig& c, const
                stage2(c.terms, split, a2, u.tmp, EpiBackprojection{u.bp, u.part, 0.f}, u.status, st));
   }
   FBME_TIMED(prof, FBME_GROUP_INIT,
-             (scalars_kernel<<<sc_blocks, 32 * kScalarScenesPerBlock, 0, st>>>(
+             (launch_dep(scalars_kernel, sc_blocks, 32 * kScalarScenesPerBlock, 0, st, 
                  kScalarInit1, s, c, u.sc, u.part, src_y, src_bp, PartSrc{0, 0})));
   if (!plain_prior) return;
   const int bn = ew_blocks_host(s.n());
   FBME_TIMED(prof, FBME_GROUP_INIT,
-             (gamma0_kernel<<<dim3(bn, s.B), kEwThreads, 0, st>>>(s, c, u.sc, u.bp, u.gamma,
+             (launch_dep(gamma0_kernel, dim3(bn, s.B), kEwThreads, 0, st, s, c, u.sc, u.bp, u.gamma,
                                                                   u.part)));
   FBME_TIMED(prof, FBME_GROUP_INIT,
-             (scalars_kernel<<<sc_blocks, 32 * kScalarScenesPerBlock, 0, st>>>(kScalarInit2, s, c, u.sc, u.part,
+             (launch_dep(scalars_kernel, sc_blocks, 32 * kScalarScenesPerBlock, 0, st, kScalarInit2, s, c, u.sc, u.part,
                                                         PartSrc{bn, 1}, PartSrc{0, 0},
                                                         PartSrc{0, 0})));
 }
@@ -697,7 +702,7 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
                  warm_prior_from_map(u.warm_map, s.B, s.n1, s.n2, u.sc.data_power, u.sc.floor_, u.gamma, u.part, bn,
                                      st));
     FBME_TIMED(prof, FBME_GROUP_INIT,
-               (scalars_kernel<<<sc_blocks, 32 * kScalarScenesPerBlock, 0, st>>>(
+               (launch_dep(scalars_kernel, sc_blocks, 32 * kScalarScenesPerBlock, 0, st, 
                    kScalarInit2, s, c, u.sc, u.part, PartSrc{bn, 1}, PartSrc{0, 0}, PartSrc{0, 0})));
   }
   DenoiseArgs da = denoise_args(c, u);
@@ -732,12 +737,12 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
     PartSrc src_dof;
     if (it == 1) {
       FBME_TIMED(prof, FBME_GROUP_SWEEP1,
-                 (sweep1_kernel<<<dim3(bn + bm, s.B), kEwThreads, 0, st>>>(s, c, u.sc, da, u.bp,
+                 (launch_dep(sweep1_kernel, dim3(bn + bm, s.B), kEwThreads, 0, st, s, c, u.sc, da, u.bp,
                                                                            u.y, msg[cur], bn)));
       src_dof = PartSrc{bn, 1};
     } else {
       FBME_TIMED(prof, FBME_GROUP_MESSAGE,
-                 (message_kernel<<<dim3(bm, s.B), kEwThreads, 0, st>>>(s, u.y, u.pred, msg[cur], msg[cur ^ 1],
+                 (launch_dep(message_kernel, dim3(bm, s.B), kEwThreads, 0, st, s, u.y, u.pred, msg[cur], msg[cur ^ 1],
                                                                       u.sc.prec, u.sc.dvar, c.uamp_damping, u.mask)));
       FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, adj1(msg[cur ^ 1]));
       cur ^= 1;
@@ -747,20 +752,20 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
       } else {
         FBME_TIMED(prof, FBME_GROUP_ADJ_2, adj2());
         FBME_TIMED(prof, FBME_GROUP_ADJ_DENOISE,
-                   (denoise_kernel<<<dim3(bn, s.B), kEwThreads, 0, st>>>(s, da, u.lift)));
+                   (launch_dep(denoise_kernel, dim3(bn, s.B), kEwThreads, 0, st, s, da, u.lift)));
         src_dof = PartSrc{bn, 1};
       }
     }
     FBME_TIMED(prof, FBME_GROUP_FWD_1, fwd1());
     FBME_TIMED(prof, FBME_GROUP_FWD_RESIDUAL, fwd2());
     FBME_TIMED(prof, FBME_GROUP_SCALARS,
-               (scalars_kernel<<<sc_blocks, 32 * kScalarScenesPerBlock, 0, st>>>(
+               (launch_dep(scalars_kernel, sc_blocks, 32 * kScalarScenesPerBlock, 0, st, 
                    kScalarSweep, s, c, u.sc, u.part, src_dof, src_dof, src_res)));
   }
 
   // --- final E-step (no prior update, no prediction), score keys ---
   FBME_TIMED(prof, FBME_GROUP_MESSAGE,
-             (message_kernel<<<dim3(bm, s.B), kEwThreads, 0, st>>>(s, u.y, u.pred, msg[cur], msg[cur ^ 1],
+             (launch_dep(message_kernel, dim3(bm, s.B), kEwThreads, 0, st, s, u.y, u.pred, msg[cur], msg[cur ^ 1],
                                                                   u.sc.prec, u.sc.dvar, c.uamp_damping, u.mask)));
   FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, adj1(msg[cur ^ 1]));
   da.update_prior = 0;
@@ -770,7 +775,7 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
   } else {
     FBME_TIMED(prof, FBME_GROUP_ADJ_2, adj2());
     FBME_TIMED(prof, FBME_GROUP_ADJ_DENOISE,
-               (denoise_kernel<<<dim3(bn, s.B), kEwThreads, 0, st>>>(s, da, u.lift)));
+               (launch_dep(denoise_kernel, dim3(bn, s.B), kEwThreads, 0, st, s, da, u.lift)));
   }
 }
 
