@@ -247,93 +247,175 @@ FBME_DEV void ldmatrix_x2(uint32_t addr, uint32_t& a0, uint32_t& a1) {
 
 
 
-// Weight gradient of one layer: dW[tap][ci][co] = sum_p x[p + shift(tap)][ci]
-// * g[p][co] (g masked by mask > 0 when a mask is given) and db[co] =
-// sum_p g[p][co].  Each block loops over tiles and writes its partial sums;
-// grad_reduce_kernel adds them in block order.
-template <typename TX, int CIN, int COUT>
-__global__ void __launch_bounds__(256)
-wgrad_kernel(const TX* x, const float* gin, const __nv_bfloat16* mask, int B, int H, int W,
+// Weight gradient of one layer with 8 input and 8 output channels:
+// dW[tap][ci][co] = sum_p x[p + shift(tap)][ci] g[p][co] (g masked by mask > 0
+// when a mask is given) and db[co] = sum_p g[p][co], as a contraction over
+// the pixels on the tensor cores: M = (tap, ci) and a row of ones for db, N =
+// co, K = 16 pixels of a row.  x is BF16 as it is; the FP32 gradient goes in
+// as three BF16 parts (8 + 8 + 8 bits of its significand), so the products
+// are exact and only the FP32 sums round, over shorter chains than one per
+// output (a warp's sum takes 4 runs of 16 pixels a tile).  Both operands lie
+// pixel-major in shared memory and are read transposed by ldmatrix.  The
+// products on the CUDA cores, one output a thread, took 293 us for 16 x 256 x
+// 256 pixels, bound by two shared-memory reads a product; 23 us so.  A
+// block loops over 16 x 32 tiles, the next one's loads in flight, and writes
+// its partial sums; grad_reduce_kernel adds them.
+constexpr int kGtH = 16, kGtW = 32, kGtPix = kGtH * kGtW;
+constexpr int kGtHaloW = kGtW + 2, kGtHalo = (kGtH + 2) * kGtHaloW;
+constexpr int kWgradOut = 9 * kHid * kHid + kHid;
+constexpr int kGtHaloIt = (kGtHalo + 255) / 256, kGtPixIt = kGtPix / 256;
+
+FBME_DEV void ldmatrix_x4_t(uint32_t addr, uint32_t& a0, uint32_t& a1, uint32_t& a2, uint32_t& a3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3)
+               : "r"(addr));
+}
+FBME_DEV void ldmatrix_x2_t(uint32_t addr, uint32_t& a0, uint32_t& a1) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(a0), "=r"(a1) : "r"(addr));
+}
+
+__global__ void __launch_bounds__(256, 3)
+wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask, int B, int H, int W,
              float* partial) {
-  constexpr int NW = 9 * CIN * COUT;
-  constexpr int NOUT = NW + COUT;
-  constexpr int PER = (NOUT + 255) / 256;
-  constexpr int HW = kTileH + 2, WW = kTileW + 2;
-  __shared__ float xs[HW * WW * CIN];
-  __shared__ float gs[kTileH * kTileW * COUT];
-  const int tid = threadIdx.x;
-  float acc[PER];
-#pragma unroll
-  for (int j = 0; j < PER; ++j) acc[j] = 0.f;
-  const int tx_n = W / kTileW, ty_n = H / kTileH;
+  static_assert(kHid == 8 && kInP == 8, "one ldmatrix row is a pixel's 8 channels");
+  __shared__ uint4 xs[kGtHalo + 1];       // the tile with its halo; the last row is ones
+  __shared__ uint4 gs[3][kGtPix];         // the gradient's parts
+  static_assert(8 * kWgradOut * sizeof(float) <= sizeof(gs), "the warps' sums reuse the gradient's parts");
+  float(*red)[kWgradOut] = reinterpret_cast<float(*)[kWgradOut]>(gs);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tx_n = (W + kGtW - 1) / kGtW, ty_n = (H + kGtH - 1) / kGtH;
   const long long ntiles = static_cast<long long>(B) * tx_n * ty_n;
-  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int b = static_cast<int>(tile / (tx_n * ty_n));
-    const int rem = static_cast<int>(tile % (tx_n * ty_n));
-    const int y0 = (rem / tx_n) * kTileH, x0 = (rem % tx_n) * kTileW;
+  uint4 hx[kGtHaloIt], hm[kGtPixIt];
+  float4 hg[kGtPixIt][2];
+  auto fetch = [&](long long tile) {
+    const int b = static_cast<int>(tile / (tx_n * ty_n)), rem = static_cast<int>(tile % (tx_n * ty_n));
+    const int y0 = (rem / tx_n) * kGtH, x0 = (rem % tx_n) * kGtW;
     const long long img = static_cast<long long>(b) * H * W;
-    __syncthreads();
-    for (int i = tid; i < HW * WW * CIN; i += 256) {
-      const int pix = i / CIN, c = i % CIN;
-      const int gy = y0 - 1 + pix / WW, gx = x0 - 1 + pix % WW;
-      float v = 0.f;
-      if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
-        const long long e = (img + static_cast<long long>(gy) * W + gx) * CIN + c;
-        if constexpr (sizeof(TX) == 2) v = __bfloat162float(x[e]);
-        else v = x[e];
-      }
-      xs[i] = v;
-    }
-    for (int i = tid; i < kTileH * kTileW * COUT; i += 256) {
-      const int pix = i / COUT, c = i % COUT;
-      const long long e = (img + static_cast<long long>(y0 + pix / kTileW) * W + x0 + pix % kTileW) * COUT + c;
-      float v = gin[e];
-      if (mask && !(__bfloat162float(mask[e]) > 0.f)) v = 0.f;
-      gs[i] = v;
-    }
-    __syncthreads();
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const int o = tid + j * 256;
-      if (o >= NOUT) continue;
-      float a = 0.f;
-      if (o < NW) {
-        const int co = o % COUT, ci = (o / COUT) % CIN, tap = o / (COUT * CIN);
-        const int dy = tap / 3, dx = tap % 3;
-        for (int py = 0; py < kTileH; ++py)
-#pragma unroll 4
-          for (int px = 0; px < kTileW; ++px)
-            a += xs[((py + dy) * WW + px + dx) * CIN + ci] * gs[(py * kTileW + px) * COUT + co];
-      } else {
-        const int co = o - NW;
-        for (int p = 0; p < kTileH * kTileW; ++p) a += gs[p * COUT + co];
+    for (int j = 0; j < kGtHaloIt; ++j) {
+      const int i = tid + 256 * j;
+      const int gy = y0 - 1 + i / kGtHaloW, gx = x0 - 1 + i % kGtHaloW;
+      hx[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (i < kGtHalo && gy >= 0 && gy < H && gx >= 0 && gx < W)
+        hx[j] = __ldg(reinterpret_cast<const uint4*>(x + (img + static_cast<long long>(gy) * W + gx) * kHid));
+    }
+#pragma unroll
+    for (int j = 0; j < kGtPixIt; ++j) {
+      const int i = tid + 256 * j;
+      const int gy = y0 + i / kGtW, gx = x0 + i % kGtW;
+      hg[j][0] = hg[j][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      hm[j] = make_uint4(0u, 0u, 0u, 0u);
+      if (gy < H && gx < W) {
+        const long long e = (img + static_cast<long long>(gy) * W + gx) * kHid;
+        hg[j][0] = __ldg(reinterpret_cast<const float4*>(gin + e));
+        hg[j][1] = __ldg(reinterpret_cast<const float4*>(gin + e) + 1);
+        if (mask) hm[j] = __ldg(reinterpret_cast<const uint4*>(mask + e));
       }
-      acc[j] += a;
+    }
+  };
+  float acc[5][4];
+#pragma unroll
+  for (int m = 0; m < 5; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[m][j] = 0.f;
+  if (tid == 0) xs[kGtHalo] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+  // this lane's ldmatrix rows: of A, matrix mi = (tap of the pair, pixel half);
+  // of B, matrix mi = (part of the pair, pixel half)
+  const int mi = lane >> 3, r8 = lane & 7;
+  const int pa = r8 + (mi >> 1) * 8, second = mi & 1;
+  const uint32_t xbase = smem_u32(xs), gbase = smem_u32(gs);
+  long long tile = blockIdx.x;
+  if (tile < ntiles) fetch(tile);
+  for (; tile < ntiles; tile += gridDim.x) {
+    __syncthreads();  // the previous tile's operands have been read
+#pragma unroll
+    for (int j = 0; j < kGtHaloIt; ++j)
+      if (tid + 256 * j < kGtHalo) xs[tid + 256 * j] = hx[j];
+#pragma unroll
+    for (int j = 0; j < kGtPixIt; ++j) {
+      float v[8] = {hg[j][0].x, hg[j][0].y, hg[j][0].z, hg[j][0].w, hg[j][1].x, hg[j][1].y, hg[j][1].z, hg[j][1].w};
+      if (mask) {
+        const uint32_t mw[4] = {hm[j].x, hm[j].y, hm[j].z, hm[j].w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float2 mf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mw[c]));
+          if (!(mf.x > 0.f)) v[2 * c] = 0.f;
+          if (!(mf.y > 0.f)) v[2 * c + 1] = 0.f;
+        }
+      }
+      uint32_t w[4];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const __nv_bfloat162 h = __float22bfloat162_rn(make_float2(v[2 * c], v[2 * c + 1]));
+          const float2 f = __bfloat1622float2(h);
+          v[2 * c] -= f.x;
+          v[2 * c + 1] -= f.y;
+          w[c] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        gs[p][tid + 256 * j] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+    __syncthreads();
+    if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
+#pragma unroll
+    for (int run = 0; run < kGtPix / 16 / 8; ++run) {  // a warp's two rows of two runs
+      const int py = 2 * warp + (run >> 1), px = (run & 1) * 16;
+      const uint32_t gp = gbase + 16u * (py * kGtW + px);
+      uint32_t bh[4], bl[2];  // parts 0 and 1, part 2
+      ldmatrix_x4_t(gp + 16u * ((mi >> 1) * kGtPix + r8 + (mi & 1) * 8), bh[0], bh[1], bh[2], bh[3]);
+      ldmatrix_x2_t(gp + 16u * (2 * kGtPix + r8 + (mi & 1) * 8), bl[0], bl[1]);
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {  // taps 2m and 2m + 1; tap 9 is the ones
+        const int tap = 2 * m + second;
+        const uint32_t row = tap < 9 ? (py + tap / 3) * kGtHaloW + px + pa + tap % 3 : kGtHalo;
+        uint32_t a[4];
+        ldmatrix_x4_t(xbase + 16u * row, a[0], a[1], a[2], a[3]);
+        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bl[0], bl[1]);
+        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bh[2], bh[3]);
+        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bh[0], bh[1]);
+      }
     }
   }
+  // block partials: the warps' sums added in order
+  __syncthreads();
+  const int g = lane >> 2, t2 = 2 * (lane & 3);
 #pragma unroll
-  for (int j = 0; j < PER; ++j) {
-    const int o = tid + j * 256;
-    if (o < NOUT) partial[static_cast<long long>(blockIdx.x) * NOUT + o] = acc[j];
+  for (int m = 0; m < 5; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int tap = 2 * m + (j >> 1), co = t2 + (j & 1);
+      if (tap < 9) red[warp][(tap * kHid + g) * kHid + co] = acc[m][j];
+      else if (g == 0) red[warp][9 * kHid * kHid + co] = acc[m][j];
+    }
+  __syncthreads();
+  for (int o = tid; o < kWgradOut; o += 256) {
+    float s = 0.f;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) s += red[v][o];
+    partial[static_cast<long long>(blockIdx.x) * kWgradOut + o] = s;
   }
 }
 
-// Sum the block partials of a layer into the flat gradient (FP64 sums in
-// block order).  `cin_used` drops padded input channels; weights land at
-// flat offset woff as [tap][ci][co], biases at boff.
-__global__ void grad_reduce_kernel(const float* partial, int nblocks, int cin, int cin_used, int cout,
-                                   int cout_used, int woff, int boff, float* grad) {
-  const int nw = 9 * cin * cout;
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nw + cout) return;
+// Sum the block partials of a layer into the flat gradient (FP64, one warp
+// an output, lanes over the blocks in a fixed order).  `cin_used` and
+// `cout_used` drop padded channels; weights land at flat offset woff as
+// [tap][ci][co], biases at boff.
+__global__ void __launch_bounds__(256) grad_reduce_kernel(const float* partial, int nblocks, int cin_used,
+                                                          int cout_used, int woff, int boff, float* grad) {
+  const int o = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (o >= kWgradOut) return;
   double s = 0.0;
-  for (int k = 0; k < nblocks; ++k) s += partial[static_cast<long long>(k) * (nw + cout) + o];
-  if (o < nw) {
-    const int co = o % cout, ci = (o / cout) % cin, tap = o / (cout * cin);
+  for (int k = lane; k < nblocks; k += 32) s += partial[static_cast<long long>(k) * kWgradOut + o];
+  s = warp_sum(s);
+  if (lane != 0) return;
+  const int co = o % kHid;
+  if (o < kWgradOut - kHid) {
+    const int ci = (o / kHid) % kHid, tap = o / (kHid * kHid);
     if (ci < cin_used && co < cout_used) grad[woff + (tap * cin_used + ci) * cout_used + co] = static_cast<float>(s);
-  } else {
-    const int co = o - nw;
-    if (co < cout_used) grad[boff + co] = static_cast<float>(s);
+  } else if (co < cout_used) {
+    grad[boff + co] = static_cast<float>(s);
   }
 }
 
@@ -356,10 +438,12 @@ __global__ void __launch_bounds__(256) loss_kernel(const float* out, const float
   if (threadIdx.x == 0) lpart[blockIdx.x] = s;
 }
 
-__global__ void loss_sum_kernel(const double* lpart, int n, double scale, double* loss_out) {
+__global__ void __launch_bounds__(256) loss_sum_kernel(const double* lpart, int n, double scale, double* loss_out) {
+  __shared__ double red[32];
   double s = 0.0;
-  for (int i = 0; i < n; ++i) s += lpart[i];
-  *loss_out = s * scale;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) s += lpart[i];
+  s = block_sum(s, red);
+  if (threadIdx.x == 0) *loss_out = s * scale;
 }
 
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, int n, float lr, float b1,
@@ -953,6 +1037,7 @@ void cnn_forward(const float* params, int B, int H, int W, void* ws, float* out,
   na.h2 = reinterpret_cast<__nv_bfloat16*>(w + L.h2);
   na.out = wout;
   const int ntiles = ((H + kFT - 1) / kFT) * ((W + kFT - 1) / kFT);
+  set_cnn_attributes();  // a process may train without ever creating a plan
   net_tile_kernel<true, kInP><<<dim3(ntiles, B), kFThreads, kFSmem, st>>>(na);
   if (out && out != wout)
     cudaMemcpyAsync(out, wout, static_cast<size_t>(B) * H * W * sizeof(float), cudaMemcpyDeviceToDevice, st);
@@ -978,23 +1063,23 @@ void cnn_backward(const float* target, int B, int H, int W, void* ws, float* gra
   auto* lpart = reinterpret_cast<double*>(w + L.lpart);
   loss_kernel<<<1024, 256, 0, st>>>(out, target, n, dout8, lpart);
   const dim3 grid(W / kTileW, H / kTileH, B);
-  // layer 3
-  wgrad_kernel<__nv_bfloat16, kHid, 8><<<kWgradBlocks, 256, 0, st>>>(h2, dout8, nullptr, B, H, W, partial);
-  grad_reduce_kernel<<<(9 * kHid * 8 + 8 + 255) / 256, 256, 0, st>>>(partial, kWgradBlocks, kHid, kHid, 8, 1,
-                                                                       kOffW3, kOffB3, grad);
+  // per layer: the weight gradient's block partials and their sum, then the
+  // input gradient (layer 2: d a2 = d h2 masked by h2 > 0, layer 1 likewise)
+  const long long tiles = static_cast<long long>(B) * ((H + kGtH - 1) / kGtH) * ((W + kGtW - 1) / kGtW);
+  const int blocks = static_cast<int>(tiles < kWgradBlocks ? tiles : kWgradBlocks);
+  auto wgrad = [&](const __nv_bfloat16* x, const float* g, const __nv_bfloat16* mask, int cin, int cout, int woff,
+                   int boff) {
+    wgrad_kernel<<<blocks, 256, 0, st>>>(x, g, mask, B, H, W, partial);
+    grad_reduce_kernel<<<(kWgradOut + 7) / 8, 256, 0, st>>>(partial, blocks, cin, cout, woff, boff, grad);
+  };
+  wgrad(h2, dout8, nullptr, kHid, 1, kOffW3, kOffB3);
   conv3x3_kernel<float, 8, kHid, kOutF32All><<<grid, kConvThreads, 0, st>>>(dout8, nullptr, P.wb3, nullptr,
                                                                             dh2, H, W);
-  // layer 2 (d a2 = d h2 masked by h2 > 0)
-  wgrad_kernel<__nv_bfloat16, kHid, kHid><<<kWgradBlocks, 256, 0, st>>>(h1, dh2, h2, B, H, W, partial);
-  grad_reduce_kernel<<<(9 * kHid * kHid + kHid + 255) / 256, 256, 0, st>>>(
-      partial, kWgradBlocks, kHid, kHid, kHid, kHid, kOffW2, kOffB2, grad);
+  wgrad(h1, dh2, h2, kHid, kHid, kOffW2, kOffB2);
   conv3x3_kernel<float, kHid, kHid, kOutF32All><<<grid, kConvThreads, 0, st>>>(dh2, h2, P.wb2, nullptr, dh1,
                                                                                H, W);
-  // layer 1 (d a1 = d h1 masked by h1 > 0)
-  wgrad_kernel<__nv_bfloat16, kInP, kHid><<<kWgradBlocks, 256, 0, st>>>(x8, dh1, h1, B, H, W, partial);
-  grad_reduce_kernel<<<(9 * kInP * kHid + kHid + 255) / 256, 256, 0, st>>>(
-      partial, kWgradBlocks, kInP, kIn, kHid, kHid, kOffW1, kOffB1, grad);
-  if (loss_out) loss_sum_kernel<<<1, 1, 0, st>>>(lpart, 1024, 1.0 / static_cast<double>(n), loss_out);
+  wgrad(x8, dh1, h1, kIn, kHid, kOffW1, kOffB1);
+  if (loss_out) loss_sum_kernel<<<1, 256, 0, st>>>(lpart, 1024, 1.0 / static_cast<double>(n), loss_out);
 }
 
 void cnn_adam(float* params, const float* grad, float* m, float* v, int step, float lr, cudaStream_t st) {
