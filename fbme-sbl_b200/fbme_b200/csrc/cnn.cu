@@ -253,11 +253,15 @@ FBME_DEV void ldmatrix_x2(uint32_t addr, uint32_t& a0, uint32_t& a1) {
 // the pixels on the tensor cores: M = (tap, ci) and a row of ones for db, N =
 // co, K = 16 pixels of a row.  x is BF16 as it is; the FP32 gradient goes in
 // as three BF16 parts (8 + 8 + 8 bits of its significand), so the products
-// are exact and only the FP32 sums round, over shorter chains than one per
-// output (a warp's sum takes 4 runs of 16 pixels a tile).  Both operands lie
+// are exact.  The tensor core truncates its sums, which biases long ones, so
+// each run of 16 pixels starts from zero, the upper part apart from the two
+// lower (its 16-bit products leave room for the run's sum), and the runs are
+// added with rounding.  Error of db3 against the 64-bit sum of its own FP32
+// terms: 2e-9 to 3e-8 (one output a thread the same, one running
+// accumulator 2e-7 to 6e-7).  Both operands lie
 // pixel-major in shared memory and are read transposed by ldmatrix.  The
 // products on the CUDA cores, one output a thread, took 293 us for 16 x 256 x
-// 256 pixels, bound by two shared-memory reads a product; 23 us so.  A
+// 256 pixels, bound by two shared-memory reads a product; 27 us so.  A
 // block loops over 16 x 32 tiles, the next one's loads in flight, and writes
 // its partial sums; grad_reduce_kernel adds them.
 constexpr int kGtH = 16, kGtW = 32, kGtPix = kGtH * kGtW;
@@ -372,9 +376,12 @@ wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask
         const uint32_t row = tap < 9 ? (py + tap / 3) * kGtHaloW + px + pa + tap % 3 : kGtHalo;
         uint32_t a[4];
         ldmatrix_x4_t(xbase + 16u * row, a[0], a[1], a[2], a[3]);
-        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bl[0], bl[1]);
-        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bh[2], bh[3]);
-        mma_bf16_16816(acc[m], a[0], a[1], a[2], a[3], bh[0], bh[1]);
+        float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_bf16_16816(lo, a[0], a[1], a[2], a[3], bl[0], bl[1]);
+        mma_bf16_16816(lo, a[0], a[1], a[2], a[3], bh[2], bh[3]);
+        mma_bf16_16816(hi, a[0], a[1], a[2], a[3], bh[0], bh[1]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[m][j] += hi[j] + lo[j];
       }
     }
   }
