@@ -887,69 +887,127 @@ struct CertModel {
   float inv_d[kMaxPolish], inv_l[kMaxPolish];
 };
 
-// Largest one-coordinate ratio over the atoms [j0, j1) of the grid (first
-// index on ties, as torch's max), with its atom precision s_j; the block's
-// best, in every thread.
-FBME_DEV CertBest cert_scan(const PolishArgs& A, const float2 (*L)[34], const CertModel& m, int K, float nu,
-                            const float2* bp, const float2* d1, const float2* d2, long long j0, long long j1,
-                            CertBest* red) {
+// Shared memory of a scan: the model's constants and factor, every value
+// doubled (and where it is needed with both signs) as an operand of the
+// paired FP32 instructions, and the Dirichlet table D2 split into re and im,
+// unrolled past the wrap, at even and at odd offset (as the exchange's).
+struct CertShared {
+  float4 mu[kMaxPolish];    // mu.x, mu.x, mu.y, mu.y
+  float4 scale[kMaxPolish]; // -mu.y, -mu.y, 1/d, 1/d
+  float4 inv[kMaxPolish];   // -1/d, -1/d, 1/l, 1/l
+  // row i's entries k < i in pairs (k, k + 1) of three float4s:
+  // -Lx, -Lx, Ly, Ly | -Ly, -Ly, -Lx', -Lx' | Ly', Ly', -Ly', -Ly'
+  float4 l[kMaxPolish * kMaxPolish / 4][3];
+  int idx[kMaxPolish], a1[kMaxPolish], a2[kMaxPolish];
+  CertBest red[kCertThreads / 32];
+};
+__host__ __device__ constexpr int cert_table_len(int n2) { return 2 * n2; }  // a pair ends at 2 n2 - 1 at most
+static size_t cert_scan_smem(const BatchShape& s) {
+  return s.n1 * sizeof(float2) + 4ull * cert_table_len(s.n2) * sizeof(float);
+}
+
+FBME_DEV float2 dup(float v) { return make_float2(v, v); }
+FBME_DEV float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+FBME_DEV float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
+
+// Largest one-coordinate ratio over the atoms of the pairs [p0, p1) (pair p:
+// columns 2c, 2c + 1 of row p / ppr, ppr pairs a row; first index on ties, as
+// torch's max), with its atom precision s_j; the block's best, in every
+// thread.  A thread carries its pair through the substitution in the paired
+// FP32 instructions, each element with the rounding sequence of one atom
+// alone (products and sums spelled out); the factor's entries are broadcast
+// reads, three 16-byte ones for two entries and two atoms.  One block of
+// eight warps with the whole register file an SM, its warps kept together by
+// a barrier a pair: the unrolled substitution is longer than the instruction
+// cache, and warps at different places of it wait for its refills (two blocks
+// of four warps 2.24 ms, this block without the barrier 1.84 ms).  One atom at
+// a time took 2.14 ms for two scans of 64 scenes of 256 x 256, this 1.78 ms,
+// about a quarter of it in the hypotenuses.
+template <bool MASKED>
+FBME_DEV CertBest cert_scan(const PolishArgs& A, CertShared& S, int K, float nu, const float2* bp, const float2* d1,
+                            const float* tab, long long p0, long long p1) {
   const BatchShape& s = A.s;
+  const int n2 = s.n2, ppr = (n2 + 1) / 2, len = cert_table_len(n2);
   const float Mf = static_cast<float>(observed_samples(s, A.c));
   const float nu2 = nu * nu;
   CertBest b{-1.f, 1.f, 0x7fffffff};
-  for (long long j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-    const int j1i = static_cast<int>(j / s.n2);
-    const int j2i = static_cast<int>(j - static_cast<long long>(j1i) * s.n2);
-    float2 q = __ldg(bp + j);
-    bool act = false;
-    float2 v[kMaxPolish];
-    float red2 = 0.f;
+  for (long long pb = p0; pb < p1; pb += kCertThreads) {
+    __syncthreads();
+    const long long p = min(pb + threadIdx.x, p1 - 1);
+    const int j1 = static_cast<int>(p / ppr), j2 = 2 * static_cast<int>(p - static_cast<long long>(j1) * ppr);
+    const int j = j1 * n2 + j2;
+    const bool two = j2 + 1 < n2;
+    const float2 b0 = __ldg(bp + j), b1 = two ? __ldg(bp + j + 1) : make_float2(0.f, 0.f);
+    float2 qx = make_float2(-b0.x, -b1.x), qy = make_float2(-b0.y, -b1.y);  // minus q of the pair
+    unsigned act = 0u;
+    float2 vx[kMaxPolish], vy[kMaxPolish];
+    float2 red2 = make_float2(0.f, 0.f);
 #pragma unroll
     for (int i = 0; i < kMaxPolish; ++i) {
       if (i < K) {
-        act |= m.idx[i] == j;
-        const float2 g = gram_at(A, d1, d2, j1i, j2i, m.a1[i], m.a2[i]);
-        const float2 mu = m.mu[i];
-        q.x -= g.x * mu.x - g.y * mu.y;
-        q.y -= g.x * mu.y + g.y * mu.x;
-        float2 c = make_float2(g.x * m.inv_d[i], -g.y * m.inv_d[i]);
-        // Row i of L in 16-byte pairs (rows start 16-byte aligned), same
-        // order of the multiply-adds as one entry at a time.
+        const unsigned dj = static_cast<unsigned>(S.idx[i] - j);
+        act |= dj < 2u ? 1u << dj : 0u;
+        int i1 = j1 - S.a1[i], i2 = j2 - S.a2[i];
+        if (i1 < 0) i1 += s.n1;
+        float2 gx, gy;
+        if constexpr (MASKED) {
+          if (i2 < 0) i2 += n2;
+          const float2* row = A.p.gram2d + static_cast<long long>(i1) * n2;
+          const float2 g0 = __ldg(row + i2), g1 = __ldg(row + (i2 + 1 < n2 ? i2 + 1 : 0));
+          gx = make_float2(g0.x, g1.x);
+          gy = make_float2(g0.y, g1.y);
+        } else {
+          const int e = i2 + n2, odd = e & 1;  // e in [1, 2 n2)
+          const float* base = tab + odd * 2 * len + (e - odd);
+          const float2 yx = *reinterpret_cast<const float2*>(base);
+          const float2 yy = *reinterpret_cast<const float2*>(base + len);
+          const float2 x = d1[i1];
+          gx = __ffma2_rn(dup(x.x), yx, __fmul2_rn(dup(-x.y), yy));
+          gy = __ffma2_rn(dup(x.y), yx, __fmul2_rn(dup(x.x), yy));
+        }
+        const float4 cm = S.mu[i], cs = S.scale[i], ci = S.inv[i];
+        qx = __fadd2_rn(qx, __ffma2_rn(gx, lo2(cm), __fmul2_rn(gy, lo2(cs))));
+        qy = __fadd2_rn(qy, __ffma2_rn(gy, lo2(cm), __fmul2_rn(gx, hi2(cm))));
+        float2 cx, cy;
+        if (i == 0) {
+          cx = __fmul2_rn(gx, hi2(cs));
+          cy = __fmul2_rn(gy, lo2(ci));
+        }
+        // minus the terms L[i][k] v[k], k ascending; the first one is fused
+        // with the scaling of conj(g)
 #pragma unroll
-        for (int k = 0; k + 1 < i; k += 2) {
-          const float4 l2 = *reinterpret_cast<const float4*>(&L[i][k]);
-          c.x -= l2.x * v[k].x - l2.y * v[k].y;
-          c.y -= l2.x * v[k].y + l2.y * v[k].x;
-          c.x -= l2.z * v[k + 1].x - l2.w * v[k + 1].y;
-          c.y -= l2.z * v[k + 1].y + l2.w * v[k + 1].x;
+        for (int k = 0; k < i; k += 2) {
+          const float4* e = S.l[i * i / 4 + k / 2];
+          const float4 e0 = e[0], e1 = e[1], e2 = e[2];
+          const float2 tx = __ffma2_rn(lo2(e0), vx[k], __fmul2_rn(hi2(e0), vy[k]));
+          const float2 ty = __ffma2_rn(lo2(e0), vy[k], __fmul2_rn(lo2(e1), vx[k]));
+          cx = k == 0 ? __ffma2_rn(gx, hi2(cs), tx) : __fadd2_rn(cx, tx);
+          cy = k == 0 ? __ffma2_rn(gy, lo2(ci), ty) : __fadd2_rn(cy, ty);
+          if (k + 1 < i) {
+            cx = __fadd2_rn(cx, __ffma2_rn(hi2(e1), vx[k + 1], __fmul2_rn(lo2(e2), vy[k + 1])));
+            cy = __fadd2_rn(cy, __ffma2_rn(hi2(e1), vy[k + 1], __fmul2_rn(hi2(e2), vx[k + 1])));
+          }
         }
-        if (i & 1) {
-          const float2 l = L[i][i - 1];
-          c.x -= l.x * v[i - 1].x - l.y * v[i - 1].y;
-          c.y -= l.x * v[i - 1].y + l.y * v[i - 1].x;
-        }
-        v[i] = make_float2(c.x * m.inv_l[i], c.y * m.inv_l[i]);
-        red2 += abs_sq(v[i]);
+        vx[i] = __fmul2_rn(cx, hi2(ci));
+        vy[i] = __fmul2_rn(cy, hi2(ci));
+        const float2 h = make_float2(hypotf(vx[i].x, vy[i].x), hypotf(vx[i].y, vy[i].y));
+        red2 = __ffma2_rn(h, h, red2);
       }
     }
-    const float prec = fmaxf(Mf / nu - red2 / nu2, kTinyP);
-    const float2 qn = make_float2(q.x / nu, q.y / nu);
-    cert_pick(b, act ? 0.f : abs_sq(qn) / prec, prec, static_cast<int>(j));
+    auto pick = [&](float qxj, float qyj, float r2, bool active, int jj) {
+      const float prec = fmaxf(Mf / nu - r2 / nu2, kTinyP);
+      const float2 qn = make_float2(qxj / nu, qyj / nu);
+      cert_pick(b, active ? 0.f : abs_sq(qn) / prec, prec, jj);
+    };
+    pick(qx.x, qy.x, red2.x, act & 1u, j);
+    if (two) pick(qx.y, qy.y, red2.y, (act >> 1) & 1u, j + 1);
   }
   b = cert_warp_best(b);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) red[w] = b;
+  if (lane == 0) S.red[w] = b;
   __syncthreads();
-  if (w == 0) {
-    b = lane < static_cast<int>(blockDim.x >> 5) ? red[lane] : CertBest{-1.f, 1.f, 0x7fffffff};
-    b = cert_warp_best(b);
-    __syncwarp();
-    if (lane == 0) red[0] = b;
-  }
-  __syncthreads();
-  b = red[0];
-  __syncthreads();
-  return b;
+  b = lane < kCertThreads / 32 ? S.red[lane] : CertBest{-1.f, 1.f, 0x7fffffff};
+  return cert_warp_best(b);
 }
 
 // Inactive certificate of the best atom (solver.py:3568-3588).
@@ -1215,42 +1273,58 @@ __global__ void __launch_bounds__(kPolishThreads) cert_step_kernel(PolishArgs A,
   if (threadIdx.x == 0 && S.status) atomicOr(&A.p.status[scene], S.status);
 }
 
-// Block (bx, scene) scores atoms [bx chunk, (bx + 1) chunk) against the
-// staged model and writes its best to the scene's partials.
-__global__ void __launch_bounds__(kCertThreads, 3) cert_scan_kernel(PolishArgs A, void* ws) {
+// Block (bx, scene) scores the atom pairs [bx chunk, (bx + 1) chunk) against
+// the staged model and writes its best to the scene's partials.
+template <bool MASKED>
+__global__ void __launch_bounds__(kCertThreads, 1) cert_scan_kernel(PolishArgs A, void* ws) {
   dep_sync();
-  __shared__ __align__(16) float2 M[32][34];
-  __shared__ CertModel model;
-  __shared__ CertBest red[kCertThreads / 32];
-  extern __shared__ float2 dtab[];
+  __shared__ CertShared S;
+  extern __shared__ float2 dtab[];  // D1 (n1), then the four D2 tables
   const int scene = blockIdx.y;
   if (scene >= A.s.B) return;
   const BatchShape& s = A.s;
-  const int K = A.c.polish_size;
+  const int K = A.c.polish_size, tid = threadIdx.x;
   const CertScratch* cs = cert_scene(ws, scene);
-  float2* d1 = dtab;
-  float2* d2 = dtab + s.n1;
-  load_dirichlet(A, d1, d2);
-  for (int e = threadIdx.x; e < K * K; e += blockDim.x) {
-    const int i = e / K, k = e - i * K;
-    if (k < i) M[i][k] = cs->L[i][k];
+  float* tab = reinterpret_cast<float*>(dtab + s.n1);
+  if constexpr (!MASKED) {
+    const int len = cert_table_len(s.n2);
+    for (int i = tid; i < s.n1; i += kCertThreads) dtab[i] = __ldg(A.p.dir1 + i);
+    for (int e = tid; e < 2 * s.n2; e += kCertThreads) {
+      const int e0 = e < s.n2 ? e : e - s.n2, e1 = e0 + 1 < s.n2 ? e0 + 1 : 0;
+      const float2 v0 = __ldg(A.p.dir2 + e0), v1 = __ldg(A.p.dir2 + e1);
+      tab[e] = v0.x;
+      tab[len + e] = v0.y;
+      tab[2 * len + e] = v1.x;
+      tab[3 * len + e] = v1.y;
+    }
   }
-  if (threadIdx.x < K) {
-    const int i = threadIdx.x;
-    model.idx[i] = cs->m.idx[i];
-    model.a1[i] = cs->m.a1[i];
-    model.a2[i] = cs->m.a2[i];
-    model.mu[i] = cs->m.mu[i];
-    model.inv_d[i] = cs->m.inv_d[i];
-    model.inv_l[i] = cs->m.inv_l[i];
+  for (int e = tid; e < kMaxPolish * (kMaxPolish / 2); e += kCertThreads) {
+    const int i = e / (kMaxPolish / 2), k = 2 * (e % (kMaxPolish / 2));
+    if (k < i && i < K) {
+      const float2 l0 = cs->L[i][k], l1 = k + 1 < i ? cs->L[i][k + 1] : make_float2(0.f, 0.f);
+      float4* d = S.l[i * i / 4 + k / 2];
+      d[0] = make_float4(-l0.x, -l0.x, l0.y, l0.y);
+      d[1] = make_float4(-l0.y, -l0.y, -l1.x, -l1.x);
+      d[2] = make_float4(l1.y, l1.y, -l1.y, -l1.y);
+    }
+  }
+  if (tid < K) {
+    const float2 mu = cs->m.mu[tid];
+    const float id = cs->m.inv_d[tid], il = cs->m.inv_l[tid];
+    S.idx[tid] = cs->m.idx[tid];
+    S.a1[tid] = cs->m.a1[tid];
+    S.a2[tid] = cs->m.a2[tid];
+    S.mu[tid] = make_float4(mu.x, mu.x, mu.y, mu.y);
+    S.scale[tid] = make_float4(-mu.y, -mu.y, id, id);
+    S.inv[tid] = make_float4(-id, -id, il, il);
   }
   __syncthreads();
   const float nu = __int_as_float(cs->nu_bits);
-  const long long N = s.n();
-  const long long chunk = (N + gridDim.x - 1) / gridDim.x;
-  const long long j0 = blockIdx.x * chunk, j1 = min(N, j0 + chunk);
-  const CertBest b = cert_scan(A, M, model, K, nu, A.p.bp + scene * N, d1, d2, j0, j1, red);
-  if (threadIdx.x == 0) cert_parts(ws, s.B, scene)[blockIdx.x] = b;
+  const long long P = static_cast<long long>(s.n1) * ((s.n2 + 1) / 2);
+  const long long chunk = (P + gridDim.x - 1) / gridDim.x;
+  const long long p0 = blockIdx.x * chunk, p1 = min(P, p0 + chunk);
+  const CertBest b = cert_scan<MASKED>(A, S, K, nu, A.p.bp + scene * s.n(), dtab, tab, p0, p1);
+  if (tid == 0) cert_parts(ws, s.B, scene)[blockIdx.x] = b;
 }
 
 // N-space outputs in one pass: zero mean, floor variance and 1/floor
@@ -1454,17 +1528,17 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
     FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1)));
   }
   if (cert) {  // model, scan, (decide + model, scan) per repair, final
+    auto scan = p.gram2d ? cert_scan_kernel<true> : cert_scan_kernel<false>;
+    const size_t csm = p.gram2d ? 0 : cert_scan_smem(s);
     int resident = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, cert_scan_kernel, kCertThreads, dsm) !=
-        cudaSuccess)
-      resident = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, scan, kCertThreads, csm) != cudaSuccess) resident = 1;
     const int nblk = cert_blocks(s, resident);
     for (int t = 0; t <= c.repairs + 1; ++t) {
       FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
                  (launch_dep(cert_step_kernel, s.B, kPolishThreads, dsm, st, A, *cert, cert->workspace, nblk, t)));
       if (t <= c.repairs)
         FBME_TIMED(prof, FBME_GROUP_CERTIFICATE,
-                   (launch_dep(cert_scan_kernel, dim3(nblk, s.B), kCertThreads, dsm, st, A, cert->workspace)));
+                   (launch_dep(scan, dim3(nblk, s.B), kCertThreads, csm, st, A, cert->workspace)));
     }
   }
   FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_finish_kernel, s.B, kPolishThreads, dsm, st, A, out)));
