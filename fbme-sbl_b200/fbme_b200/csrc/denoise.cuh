@@ -1,6 +1,6 @@
-// The UAMP Gaussian denoiser of one coefficient, shared by the elementwise
-// denoiser (uamp.cu) and the FFT stage that fuses it into its epilogue
-// (fft.cu).
+// The UAMP Gaussian denoiser of one coefficient and message update of one
+// sample, shared by the elementwise kernels (uamp.cu) and the FFT stages that
+// fuse them into their epilogue and prologue (fft.cu).
 #pragma once
 
 #include <stdint.h>
@@ -55,6 +55,24 @@ FBME_DEV DenoiseOut denoise_math(const DenoiseArgs& a, float prior, float2 om, f
   cand = fmaxf(fl, fminf(a.prior_max, cand));
   o.gamma = fmaxf(a.prior_damping * prior + (1.0f - a.prior_damping) * cand, fl);
   return o;
+}
+
+// UAMP message update of one sample (triton_kernels.py:72-84):
+// m' = d m + (1-d) prec (y - (p - dvar m)), its rounding spelled out so that
+// the message kernel and the FFT stage that forms its input this way agree.
+struct MessageArgs {
+  const float2 *y, *pred, *in;
+  float2* out;
+  const float *prec, *dvar;
+  float damping;
+  const uint8_t* mask;  // [M1*M2] observed samples (or nullptr)
+};
+
+FBME_DEV float2 message_step(float2 y, float2 p, float2 m, float prec, float dvar, float damping) {
+  const float upd = 1.0f - damping;
+  const float cx = __fmul_rn(prec, __fsub_rn(y.x, fmaf(-dvar, m.x, p.x)));
+  const float cy = __fmul_rn(prec, __fsub_rn(y.y, fmaf(-dvar, m.y, p.y)));
+  return make_float2(fmaf(damping, m.x, __fmul_rn(upd, cx)), fmaf(damping, m.y, __fmul_rn(upd, cy)));
 }
 
 }  // namespace fbme

@@ -137,6 +137,10 @@ FBME_DEV float2* fft_rows(const FftPlan& p, int rt, int pitch, float2* a, float2
 //           kernel only): mean, variance, prior and score keys updated as
 //           denoise_kernel does, per-tile sums of relevance (slot 0) and
 //           variance (slot 1)
+//   mode 4  store, of the UAMP message update (two-pass kernel only): the
+//           input rows are formed from the observations, the prediction and
+//           the previous message (message_step), and the new message is
+//           written beside the transform
 struct FftIo {
   const float2* in;
   float2* out;
@@ -146,6 +150,7 @@ struct FftIo {
   int mode;
   int ysum;
   DenoiseArgs dn;         // mode 3
+  MessageArgs ms;         // mode 4
 };
 
 // The stages of one launch of the two-pass kernel: item i owns the launch's
@@ -422,10 +427,64 @@ FBME_DEV void fast_issue(const FftStage& st, const FftIo& io, int t, float2* buf
   cp_async_commit();
 }
 
+// The values thread (lr, p) transforms in tile t under mode 4, straight into
+// its registers: the message update of x[p + P q] for p + P q < K, written to
+// the new message as well.  A batch's loads are issued before its stores.
+// The next tile's rows are prefetched into L2, not into shared memory: the two
+// blocks of an SM overlap each other's loads.  512 scenes of 256^2 / 128^2:
+// message kernel and stage 48 + 51 us, fused 87 us; 61 us is the copy rate's
+// time for the bytes that remain.
+FBME_DEV void message_prefetch(const FftStage& st, const MessageArgs& ms, int unit, int r0, int rows) {
+  const int lines = (st.kin * 8 + 127) / 128 + 1;  // 128-byte lines a row touches, at most
+  const long long last = static_cast<long long>(st.rows) * st.in_ld - 1;
+  for (int i = threadIdx.x; i < rows * lines; i += kFftThreads) {
+    const long long in_row = static_cast<long long>(r0 + i / lines) * st.in_ld + (i % lines) * 16;
+    const long long e = unit * st.in_stride + (in_row < last ? in_row : last);
+    prefetch_l2(ms.y + e);
+    prefetch_l2(ms.pred + e);
+    prefetch_l2(ms.in + e);
+  }
+}
+template <int L>
+FBME_DEV void message_rows(const FftStage& st, const MessageArgs& ms, int unit, int r, int p,
+                           float2 (&v)[L / fast_threads_per_row(L)]) {
+  constexpr int P = fast_threads_per_row(L), Q = L / P, NB = Q % 8 == 0 && Q <= 16 ? 8 : Q % 4 == 0 ? 4 : 3;
+  static_assert(Q % NB == 0, "whole batches");
+  const bool live = r < st.rows;
+  const long long e0 = unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
+  const uint8_t* mask = ms.mask ? ms.mask + static_cast<long long>(r) * st.in_ld + p : nullptr;
+  const float pr = ms.prec[unit], dv = ms.dvar[unit];
+#pragma unroll
+  for (int q0 = 0; q0 < Q; q0 += NB) {
+    float2 y[NB], pd[NB], m[NB];
+    bool in[NB], obs[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int k = P * (q0 + i);
+      in[i] = live && p + k < st.kin;
+      y[i] = pd[i] = m[i] = make_float2(0.f, 0.f);
+      obs[i] = true;
+      if (in[i]) {
+        y[i] = __ldg(ms.y + e0 + k);
+        pd[i] = __ldg(ms.pred + e0 + k);
+        m[i] = __ldg(ms.in + e0 + k);
+        if (mask) obs[i] = __ldg(mask + k) != 0;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const float2 o = obs[i] ? message_step(y[i], pd[i], m[i], pr, dv, ms.damping) : make_float2(0.f, 0.f);
+      v[q0 + i] = in[i] ? o : make_float2(0.f, 0.f);
+      if (in[i]) ms.out[e0 + P * (q0 + i)] = o;
+    }
+  }
+}
+
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (tile t = unit x
 // tiles + row tile); the copy of its next tile is in flight while the
 // current one is transformed.
-// EPI: 0 store (modes 0 and 1), 1 residual (mode 2), 2 denoiser (mode 3)
+// EPI: 0 store (modes 0 and 1), 1 residual (mode 2), 2 denoiser (mode 3),
+// 3 store of the message update (mode 4)
 template <int L, int S, int EPI>
 __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage st, const FftIo io) {
   dep_sync();
@@ -437,14 +496,14 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
   const int lr = threadIdx.x / P, p = threadIdx.x % P;
   const int total = st.tiles * st.units;
   int t = blockIdx.x;
-  if (t < total) fast_issue<L>(st, io, t, fsm, lr, p);
+  if (EPI != 3 && t < total) fast_issue<L>(st, io, t, fsm, lr, p);
   for (int it = 0; t < total; ++it, t += gridDim.x) {
     float2* buf = fsm + (it & 1) * BUF;
-    if (t + static_cast<int>(gridDim.x) < total)
+    if (EPI != 3 && t + static_cast<int>(gridDim.x) < total)
       fast_issue<L>(st, io, t + gridDim.x, fsm + ((it + 1) & 1) * BUF, lr, p);
     else
       cp_async_commit();  // empty group: the wait below counts the same
-    if constexpr (EPI != 0) {
+    if constexpr (EPI == 1 || EPI == 2) {
       // the next tile's epilogue operands (observations; prior, mean and
       // variance) into L2, one line per output column and array, so their
       // DRAM reads overlap this tile's transform
@@ -464,6 +523,10 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
         }
       }
     }
+    if constexpr (EPI == 3) {
+      const int tn = t + gridDim.x;
+      if (tn < total) message_prefetch(st, io.ms, tn / st.tiles, (tn % st.tiles) * ROWS, ROWS);
+    }
     cp_async_wait<1>();   // this thread's copies of tile t (it reads only its own)
     const int unit = t / st.tiles, tile = t - unit * st.tiles;
     const int r0 = tile * ROWS;
@@ -472,9 +535,13 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
 
     // pass 1: DFT-Q of x[p + P q] in registers
     float2 v[Q];
+    if constexpr (EPI == 3) {
+      message_rows<L>(st, io.ms, unit, r0 + lr, p, v);
+    } else {
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-      v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+      for (int q = 0; q < Q; ++q)
+        v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+    }
     if (io.ysum) {
       float acc = 0.f;
 #pragma unroll
@@ -540,7 +607,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
     const long long o0 = static_cast<long long>(c0) * st.out_ld + rr;
     const long long step = static_cast<long long>(P) * st.out_ld;
     const float2* sp = buf + row * A + row;
-    if constexpr (EPI == 0) {
+    if constexpr (EPI == 0 || EPI == 3) {
       __syncthreads();
       float acc = 0.f;
       if (live_out) {
@@ -664,7 +731,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
   const int lr = threadIdx.x / P, p = threadIdx.x % P;
   const int total = set.tile0[set.n];
   int t = blockIdx.x;
-  if (t < total) {
+  if (EPI != 3 && t < total) {
     const int i = fft_set_item(set, t);
     fast_issue<L>(set.st[i], set.io[i], t - set.tile0[i], fsm, lr, p);
   }
@@ -674,12 +741,12 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
     const FftIo& io = set.io[item];
     float2* buf = fsm + (it & 1) * BUF;
     const int tn = t + gridDim.x;
-    if (tn < total) {
+    if (EPI != 3 && tn < total) {
       const int in_ = fft_set_item(set, tn);
       const FftStage& sn = set.st[in_];
       const int tl = tn - set.tile0[in_];
       fast_issue<L>(sn, set.io[in_], tl, fsm + ((it + 1) & 1) * BUF, lr, p);
-      if constexpr (EPI != 0) {
+      if constexpr (EPI == 1 || EPI == 2) {
         // the next tile's epilogue operands (observations; prior, mean and
         // variance) into L2, one line per output column and array, so their
         // DRAM reads overlap this tile's transform
@@ -709,9 +776,13 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
 
     // pass 1: DFT-Q of x[p + P q] in registers
     float2 v[Q];
+    if constexpr (EPI == 3) {
+      message_rows<L>(st, io.ms, unit, r0 + lr, p, v);
+    } else {
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-      v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+      for (int q = 0; q < Q; ++q)
+        v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+    }
     if (io.ysum) {
       float acc = 0.f;
 #pragma unroll
@@ -777,7 +848,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
     const long long o0 = static_cast<long long>(c0) * st.out_ld + rr;
     const long long step = static_cast<long long>(P) * st.out_ld;
     const float2* sp = buf + row * A + row;
-    if constexpr (EPI == 0) {
+    if constexpr (EPI == 0 || EPI == 3) {
       __syncthreads();
       float acc = 0.f;
       if (live_out) {
@@ -923,6 +994,7 @@ void launch_fast(const FftStage& S, const FftIo& io, int sign, cudaStream_t st) 
     else launch_fast_as<L, -1, 0>(S, io, st);
   } else {
     if (io.mode == 3) launch_fast_as<L, 1, 2>(S, io, st);
+    else if (io.mode == 4) launch_fast_as<L, 1, 3>(S, io, st);
     else launch_fast_as<L, 1, 0>(S, io, st);
   }
 }
@@ -933,6 +1005,7 @@ void launch_fast_set(const FftSet<kFftSetMax>& set, int sign, int mode, cudaStre
     else launch_fast_set_as<L, -1, 0>(set, st);
   } else {
     if (mode == 3) launch_fast_set_as<L, 1, 2>(set, st);
+    else if (mode == 4) launch_fast_set_as<L, 1, 3>(set, st);
     else launch_fast_set_as<L, 1, 0>(set, st);
   }
 }
@@ -948,10 +1021,12 @@ cudaError_t set_fast_attr() {
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, -1, 1>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 0>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 2>, bytes);
+  if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 3>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 0, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 1, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 0, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 2, kFftSetMax>, bytes);
+  if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 3, kFftSetMax>, bytes);
   return e;
 }
 
@@ -1022,9 +1097,12 @@ cudaError_t set_fft_attributes() {
 
 // One FFT stage of `units` transforms (the geometry of the GEMM stage `g`,
 // whose contracted length K is padded to the transform length L).
-// The fused denoiser epilogue pays where two CTAs fit on an SM; at L = 512
-// (one CTA of 147 KB) its loads find too few warps, and the elementwise
-// denoiser at full occupancy is faster.
+// The fused denoiser epilogue and the message update formed in the load pay
+// where two CTAs fit on an SM; at L = 512 (one CTA of 147 KB) their loads find
+// too few warps, and the elementwise kernels at full occupancy are faster (32
+// scenes of 512^2 / 256^2: message update fused 1.27 ms a replay, by itself
+// 1.25 ms; 512 scenes of 256^2 / 128^2: fused 3.13 ms, by itself 3.17 ms).
+int fft_message_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
 int fft_denoise_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
 
 static FftStage fft_stage_of(const DftGeom& g, int L, int sign, const float2* tw) {
@@ -1059,10 +1137,11 @@ static void launch_fast_set_len(const FftSet<kFftSetMax>& set, int L, int sign, 
 
 void fft_stage(const DftGeom& g, int L, int sign, const float2* tw, const float2* in, float2* out,
                const float2* y, const uint8_t* mask, double* part, int mode, int ysum, cudaStream_t st,
-               const DenoiseArgs* dn) {
+               const DenoiseArgs* dn, const MessageArgs* ms) {
   const FftStage S = fft_stage_of(g, L, sign, tw);
   FftIo io{in, out, y, mask, part, mode, ysum};
   if (dn) io.dn = *dn;
+  if (ms) io.ms = *ms;
   switch (L) {
     case 512: launch_fast<512>(S, io, sign, st); return;
     case 384: launch_fast<384>(S, io, sign, st); return;
@@ -1089,7 +1168,7 @@ void fft_stage_set(const FftSetJob* jobs, int n, int L, int sign, int mode, cuda
     // per bucket, as fft_stage runs it
     for (int i = 0; i < n; ++i) {
       const FftSetJob& j = jobs[i];
-      fft_stage(j.g, L, sign, j.tw, j.in, j.out, j.y, j.mask, j.part, mode, j.ysum, st, j.dn);
+      fft_stage(j.g, L, sign, j.tw, j.in, j.out, j.y, j.mask, j.part, mode, j.ysum, st, j.dn, j.ms);
     }
     return;
   }
@@ -1103,6 +1182,7 @@ void fft_stage_set(const FftSetJob* jobs, int n, int L, int sign, int mode, cuda
       set.st[i] = fft_stage_of(j.g, L, sign, j.tw);
       set.io[i] = FftIo{j.in, j.out, j.y, j.mask, j.part, mode, j.ysum};
       if (mode == 3) set.io[i].dn = *j.dn;
+      if (mode == 4) set.io[i].ms = *j.ms;
       set.tile0[i + 1] = set.tile0[i] + set.st[i].tiles * set.st[i].units;
     }
     launch_fast_set_len(set, L, sign, mode, st);

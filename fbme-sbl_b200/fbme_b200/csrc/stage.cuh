@@ -259,15 +259,18 @@ static cudaError_t set_attr_both() {
 
 namespace fbme {
 struct DenoiseArgs;
+struct MessageArgs;
 // One FP32 FFT stage (fft.cu) with the geometry of the GEMM stage `g`: a
 // length-L transform of sign `sign` per row, input zero-padded from g.kcplx,
 // output truncated to g.cols.  Mode 3 (with `dn`) runs the UAMP denoiser on
-// the outputs instead of storing them; fft_denoise_fused(L) says whether
-// that is built for the length.
+// the outputs instead of storing them, mode 4 (with `ms`) takes the UAMP
+// message update as its input; fft_denoise_fused(L) and fft_message_fused(L)
+// say whether that is built for the length.
 void fft_stage(const DftGeom& g, int L, int sign, const float2* tw, const float2* in, float2* out,
                const float2* y, const uint8_t* mask, double* part, int mode, int ysum, cudaStream_t st,
-               const DenoiseArgs* dn = nullptr);
+               const DenoiseArgs* dn = nullptr, const MessageArgs* ms = nullptr);
 int fft_denoise_fused(int L);
+int fft_message_fused(int L);
 
 // One shape bucket's stage in a merged FFT launch (fft_stage_set): the
 // arguments fft_stage takes, per bucket.
@@ -281,6 +284,7 @@ struct FftSetJob {
   double* part;
   int ysum;
   const DenoiseArgs* dn;  // mode 3
+  const MessageArgs* ms;  // mode 4
 };
 // The stages `jobs[0..n)` of one transform length L, sign and mode: in as
 // few launches of the two-pass kernel as fit (64 buckets each) where L has

@@ -257,12 +257,7 @@ FBME_DEV void message_body(Blk k, BatchShape s, const float2* y, const float2* p
   const int scene = k.y;
   const long long m = s.m();
   const float pr = prec[scene], dv = dvar[scene];
-  const float keep = damping, upd = 1.0f - damping;
-  auto step = [&](float2 yy, float2 pp, float2 mm) {
-    const float2 pseudo = make_float2(pp.x - dv * mm.x, pp.y - dv * mm.y);
-    const float2 cand = make_float2(pr * (yy.x - pseudo.x), pr * (yy.y - pseudo.y));
-    return make_float2(keep * mm.x + upd * cand.x, keep * mm.y + upd * cand.y);
-  };
+  auto step = [&](float2 yy, float2 pp, float2 mm) { return message_step(yy, pp, mm, pr, dv, damping); };
   const long long first = k.x * static_cast<long long>(blockDim.x) + threadIdx.x;
   const long long stride = static_cast<long long>(k.gx) * blockDim.x;
   if ((m & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0) {
@@ -573,10 +568,10 @@ static void stage2(int terms, bool split, const DftGeom& g2, const float2* tmp, 
 // the N2 axis, stages 2 the N1 axis; forward stages take the minus sign.
 static void fft_of(Stage which, const BatchShape& s, const DftTables& t, const DftGeom& g, const float2* in,
                    float2* out, const float2* y, const uint8_t* mask, double* part, int mode, int ysum,
-                   cudaStream_t st, const DenoiseArgs* dn = nullptr) {
+                   cudaStream_t st, const DenoiseArgs* dn = nullptr, const MessageArgs* ms = nullptr) {
   const bool ax2 = which == kFwd1 || which == kAdj1;
   fft_stage(g, ax2 ? s.n2 : s.n1, (which == kFwd1 || which == kFwd2) ? -1 : 1, ax2 ? t.fft_n2 : t.fft_n1, in,
-            out, y, mask, part, mode, ysum, st, dn);
+            out, y, mask, part, mode, ysum, st, dn, ms);
 }
 // Partial-sum source of an FFT stage: its row tiles x 8 warps.
 static PartSrc fft_src(Stage which, const BatchShape& s, const DftGeom& g) {
@@ -713,6 +708,21 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
     if (fft) fft_of(kAdj1, s, t, a1, m, u.tmp, nullptr, nullptr, nullptr, 0, 0, st);
     else stage1(c.terms, split, a1, a2, ProPlain{m}, u.tmp, u.status, st);
   };
+  // the message update, then adjoint stage 1: one launch where the FFT stage
+  // forms its input that way
+  const bool fused_message = fft && fft_message_fused(s.n2);
+  auto message_adj1 = [&](const float2* mi, float2* mo) {
+    if (fused_message) {
+      const MessageArgs ms{u.y, u.pred, mi, mo, u.sc.prec, u.sc.dvar, c.uamp_damping, u.mask};
+      FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
+                 fft_of(kAdj1, s, t, a1, nullptr, u.tmp, nullptr, nullptr, nullptr, 4, 0, st, nullptr, &ms));
+      return;
+    }
+    FBME_TIMED(prof, FBME_GROUP_MESSAGE,
+               (launch_dep(message_kernel, dim3(bm, s.B), kEwThreads, 0, st, s, u.y, u.pred, mi, mo, u.sc.prec,
+                           u.sc.dvar, c.uamp_damping, u.mask)));
+    FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, adj1(mo));
+  };
   auto adj2 = [&]() {
     if (fft) fft_of(kAdj2, s, t, a2, u.tmp, u.lift, nullptr, nullptr, nullptr, 0, 0, st);
     else stage2(c.terms, split, a2, u.tmp, EpiStoreT{u.lift}, u.status, st);
@@ -741,10 +751,7 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
                                                                            u.y, msg[cur], bn)));
       src_dof = PartSrc{bn, 1};
     } else {
-      FBME_TIMED(prof, FBME_GROUP_MESSAGE,
-                 (launch_dep(message_kernel, dim3(bm, s.B), kEwThreads, 0, st, s, u.y, u.pred, msg[cur], msg[cur ^ 1],
-                                                                      u.sc.prec, u.sc.dvar, c.uamp_damping, u.mask)));
-      FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, adj1(msg[cur ^ 1]));
+      message_adj1(msg[cur], msg[cur ^ 1]);
       cur ^= 1;
       if (fused_denoise) {
         FBME_TIMED(prof, FBME_GROUP_ADJ_DENOISE, adj2_denoise());
@@ -764,10 +771,7 @@ void uamp_run(const BatchShape& s, const DftTables& t, const DevConfig& c, const
   }
 
   // --- final E-step (no prior update, no prediction), score keys ---
-  FBME_TIMED(prof, FBME_GROUP_MESSAGE,
-             (launch_dep(message_kernel, dim3(bm, s.B), kEwThreads, 0, st, s, u.y, u.pred, msg[cur], msg[cur ^ 1],
-                                                                  u.sc.prec, u.sc.dvar, c.uamp_damping, u.mask)));
-  FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, adj1(msg[cur ^ 1]));
+  message_adj1(msg[cur], msg[cur ^ 1]);
   da.update_prior = 0;
   da.keys = reinterpret_cast<uint32_t*>(u.keys);
   if (fused_denoise) {
@@ -914,6 +918,39 @@ void uamp_run_multi(const UampJob* J, int nb, cudaStream_t st, Profiler* prof, c
     const bool ax2 = which == kFwd1 || which == kAdj1;
     return PartSrc{fft_stage_tiles(g.rows, ax2 ? J[b].s.n2 : J[b].s.n1), kPartWarps};
   };
+  // FFT buckets whose adjoint stage 1 takes the message update as its input:
+  // the other buckets' updates first, then the stage of all
+  auto fmsg = [&](int b) { return is_fft(b) && fft_message_fused(J[b].s.n2); };
+  std::vector<MessageArgs> mss(nb);
+  auto message_adj1 = [&](const std::vector<int>& bs) {
+    std::vector<MessageJob> jm;
+    std::vector<int> plain, taking;
+    for (int b : bs) {
+      const UampBuffers& u = J[b].u;
+      if (fmsg(b)) {
+        mss[b] = MessageArgs{u.y, u.pred, msg(b, cur[b]), msg(b, cur[b] ^ 1), u.sc.prec, u.sc.dvar,
+                             J[b].c.uamp_damping, nullptr};
+        taking.push_back(b);
+      } else {
+        jm.push_back({bm[b], J[b].s, u.y, u.pred, msg(b, cur[b]), msg(b, cur[b] ^ 1), u.sc.prec, u.sc.dvar,
+                      J[b].c.uamp_damping});
+        plain.push_back(b);
+      }
+    }
+    if (!jm.empty())
+      FBME_TIMED(prof, FBME_GROUP_MESSAGE, ew_launch(jm, [&](const EwJobs<MessageJob>& m, dim3 g) {
+                   message_multi_kernel<<<g, kEwThreads, 0, st>>>(m);
+                 }));
+    FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
+               stage1_m(tens_of(plain), a1, a2, [&](int b) { return ProPlain{msg(b, cur[b] ^ 1)}; }));
+    FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
+               fft_m(kAdj1, plain, a1, 0, [&](int b) { return job(msg(b, cur[b] ^ 1), J[b].u.tmp); }));
+    FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE, fft_m(kAdj1, taking, a1, 4, [&](int b) {
+                 FftSetJob j = job(nullptr, J[b].u.tmp);
+                 j.ms = &mss[b];
+                 return j;
+               }));
+  };
   // FFT buckets whose adjoint stage 2 runs the denoiser in its epilogue
   auto fused = [&](int b) { return is_fft(b) && fft_denoise_fused(J[b].s.n1); };
   std::vector<DenoiseArgs> das(nb);
@@ -975,13 +1012,10 @@ void uamp_run_multi(const UampJob* J, int nb, cudaStream_t st, Profiler* prof, c
                    sweep1_multi_kernel<<<g, kEwThreads, 0, st>>>(m);
                  }));
     } else {
-      std::vector<MessageJob> jm;
       std::vector<DenoiseJob> jd;
       std::vector<int> lifted, fusing;
       for (int b : act) {
         const UampBuffers& u = J[b].u;
-        jm.push_back({bm[b], J[b].s, u.y, u.pred, msg(b, cur[b]), msg(b, cur[b] ^ 1), u.sc.prec, u.sc.dvar,
-                      J[b].c.uamp_damping});
         das[b] = denoise_args(J[b].c, u);
         if (fused(b)) {
           fusing.push_back(b);
@@ -990,13 +1024,7 @@ void uamp_run_multi(const UampJob* J, int nb, cudaStream_t st, Profiler* prof, c
           jd.push_back({bn[b], J[b].s, das[b], u.lift});
         }
       }
-      FBME_TIMED(prof, FBME_GROUP_MESSAGE, ew_launch(jm, [&](const EwJobs<MessageJob>& m, dim3 g) {
-                   message_multi_kernel<<<g, kEwThreads, 0, st>>>(m);
-                 }));
-      FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
-                 stage1_m(tens_of(act), a1, a2, [&](int b) { return ProPlain{msg(b, cur[b] ^ 1)}; }));
-      FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
-                 fft_m(kAdj1, act, a1, 0, [&](int b) { return job(msg(b, cur[b] ^ 1), J[b].u.tmp); }));
+      message_adj1(act);
       for (int b : act) cur[b] ^= 1;
       FBME_TIMED(prof, FBME_GROUP_ADJ_2,
                  stage2_m(tens_of(lifted), a2, [&](int b) { return EpiStoreT{J[b].u.lift}; }));
@@ -1038,13 +1066,10 @@ void uamp_run_multi(const UampJob* J, int nb, cudaStream_t st, Profiler* prof, c
   }
 
   // --- final E-step (no prior update, no prediction), score keys ---
-  std::vector<MessageJob> jm;
   std::vector<DenoiseJob> jd;
   std::vector<int> lifted, fusing;
   for (int b = 0; b < nb; ++b) {
     const UampBuffers& u = J[b].u;
-    jm.push_back({bm[b], J[b].s, u.y, u.pred, msg(b, cur[b]), msg(b, cur[b] ^ 1), u.sc.prec, u.sc.dvar,
-                  J[b].c.uamp_damping});
     das[b] = denoise_args(J[b].c, u);
     das[b].update_prior = 0;
     das[b].keys = reinterpret_cast<uint32_t*>(u.keys);
@@ -1055,13 +1080,7 @@ void uamp_run_multi(const UampJob* J, int nb, cudaStream_t st, Profiler* prof, c
       jd.push_back({bn[b], J[b].s, das[b], u.lift});
     }
   }
-  FBME_TIMED(prof, FBME_GROUP_MESSAGE, ew_launch(jm, [&](const EwJobs<MessageJob>& m, dim3 g) {
-               message_multi_kernel<<<g, kEwThreads, 0, st>>>(m);
-             }));
-  FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
-             stage1_m(tens_of(all), a1, a2, [&](int b) { return ProPlain{msg(b, cur[b] ^ 1)}; }));
-  FBME_TIMED(prof, FBME_GROUP_ADJ_MESSAGE,
-             fft_m(kAdj1, all, a1, 0, [&](int b) { return job(msg(b, cur[b] ^ 1), J[b].u.tmp); }));
+  message_adj1(all);
   FBME_TIMED(prof, FBME_GROUP_ADJ_2, stage2_m(tens_of(lifted), a2, [&](int b) { return EpiStoreT{J[b].u.lift}; }));
   FBME_TIMED(prof, FBME_GROUP_ADJ_2, fft_m(kAdj2, lifted, a2, 0, [&](int b) { return job(J[b].u.tmp, J[b].u.lift); }));
   FBME_TIMED(prof, FBME_GROUP_ADJ_DENOISE, fft_m(kAdj2, fusing, a2, 3, [&](int b) {
