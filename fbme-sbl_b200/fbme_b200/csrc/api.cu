@@ -35,7 +35,7 @@ int default_n_tile(int terms) { return terms == 6 ? 128 : 256; }
 struct Layout {
   size_t tab_f2, tab_f1, tab_a2, tab_a1, dir1, dir2;
   size_t mu, bp, var, gamma, msg, pred, tmp, lift, keys, part, scal;
-  size_t active, score, pstate, xval, xidx, status, ckey, cidx;
+  size_t pstate, status, ckey, cidx;
   size_t mask, ymask, gram, gscr;  // observation mask (fbme_plan_set_observation_mask)
   size_t fft1, fft2;               // FP32 FFT twiddles (dft_terms 0)
   size_t total;
@@ -82,11 +82,7 @@ Layout make_layout(const fbme::BatchShape& s, const FbmeConfig& c, int nt) {
   L.keys = take(B * N * sizeof(uint32_t));
   L.part = take(B * fbme::kMaxTilesPerScene * fbme::kPartSlots * sizeof(double));
   L.scal = take(10 * B * sizeof(float));
-  L.active = take(B * K * sizeof(int));
-  L.score = take(B * K * sizeof(float));
   L.pstate = take(B * fbme::polish_state_bytes());
-  L.xval = take(B * E * sizeof(float));
-  L.xidx = take(B * E * sizeof(int));
   L.status = take(B * sizeof(int));
   const size_t c1 = static_cast<size_t>(fbme::topk_slices(s.n())) * K;
   const size_t c2 = static_cast<size_t>(fbme::exchange_blocks(s)) * E;
@@ -435,11 +431,7 @@ void bind_bucket(Bucket& k, uint8_t* ws, cudaStream_t st) {
   p.var = u.var;
   p.gamma = u.gamma;
   p.sc = u.sc;
-  p.active = reinterpret_cast<int*>(w + L.active);
-  p.score = reinterpret_cast<float*>(w + L.score);
   p.pstate = w + L.pstate;
-  p.xcand_val = reinterpret_cast<float*>(w + L.xval);
-  p.xcand_idx = reinterpret_cast<int*>(w + L.xidx);
   p.keys = u.keys;
   p.cand_key = reinterpret_cast<uint32_t*>(w + L.ckey);
   p.cand_idx = reinterpret_cast<int*>(w + L.cidx);

@@ -177,15 +177,10 @@ struct PolishBuffers {
   const float *var, *gamma;
   Scalars sc;
   // per-scene state
-  int* active;        // [B][K] current active set
-  float* score;       // [B][K] UAMP second moments of the active set
-  float* gamma_init;  // [B][K] prior variances of the active set before reinit
   unsigned char* pstate;  // opaque per-scene polish state
-  float* xcand_val;   // exchange candidates [B][E]
-  int* xcand_idx;
   uint32_t* keys;     // [B][N] score keys scratch
   uint32_t* cand_key; // [B][max candidates] top-k candidate keys
-  int* cand_idx;      // [B][max candidates] their grid indices
+  int* cand_idx;      // [B][max candidates] their grid indices, in lists (topk.cuh)
   int* status;        // [B] per-scene status
 };
 // `cert` (host copy; null: off) adds the global certificate and support
@@ -211,19 +206,7 @@ struct TopkJobs {
   int n;
   TopkJob j[kBucketSetMax];
 };
-struct TopkMergeJob {
-  const uint32_t* cand_key;
-  const int* cand_idx;
-  int ncand, k, B;
-  int* out_idx;
-  float* out_val;
-};
-struct TopkMergeJobs {
-  int n;
-  TopkMergeJob j[kBucketSetMax];
-};
 void launch_topk_blocks_multi(const TopkJobs& J, int max_slices, int max_b, cudaStream_t st);
-void launch_topk_merge_multi(const TopkMergeJobs& J, int max_b, cudaStream_t st);
 // The polish of several equal-config shape buckets (an uneven plan's) as
 // one launch per step: results equal polish_run per bucket.
 struct PolishBucket {

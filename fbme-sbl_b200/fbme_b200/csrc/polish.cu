@@ -405,10 +405,10 @@ FBME_DEV int warp_sort_desc(float val, int pos, float* out_val) {
 
 // Evaluations p in [state.evals, P) until done or an exchange is needed,
 // one block per scene.  phase 0: initialise from the top-K; phase 1: apply
-// the exchange whose candidates are in p.xcand_*, then continue.  Every
+// the exchange whose candidate lists are in p.cand_*, then continue.  Every
 // warp holds the same lane values (active set, variances, best model), so
 // the decisions need no broadcast; warp 0 writes the state.
-FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int scene) {
+FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, TopkMergeShared& T, int phase, int lists, int scene) {
   extern __shared__ float2 dtab[];  // D1 (n1) then D2 (n2)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (scene >= A.s.B) return;
@@ -426,6 +426,16 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int s
   float2* d2 = dtab + s.n1;
   if (threadIdx.x == 0) S.status = 0;
 
+  // the selection this phase starts from: the active set or the exchange's
+  // additions, merged from the candidate lists (S.M and S.L are free here)
+  static_assert(sizeof(S.M) + sizeof(S.L) >= kMergeMax * sizeof(unsigned long long), "merge scratch");
+  const int nsel = phase == 0 ? K : c.exchange;
+  {
+    const size_t off = static_cast<size_t>(scene) * lists * nsel;
+    block_topk_merge<kMergeMax / kPolishThreads>(A.p.cand_key + off, A.p.cand_idx + off, lists, nsel,
+                                                 reinterpret_cast<unsigned long long*>(&S), T);
+  }
+
   // the work set of the next evaluation and the best model so far
   int idx = 0, bidx = 0, pending = 0, exch_acc = 0, has_best = 0, evals = 0;
   float gam = 1.0f, nu = 0.f, bnoise = 0.f, bpv = 0.f, bdd = 0.f, bg = 1.0f;
@@ -434,9 +444,9 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int s
   if (phase == 0) {
     // prune + reinitialise (solver.py:4087-4106)
     if (on) {
-      idx = A.p.active[scene * K + lane];
+      idx = merge_index(T.best[lane]);
       const float g0 = A.p.gamma[scene * N + idx];
-      gam = c.reinit ? fmaxf(A.p.score[scene * K + lane], fl) : g0;
+      gam = c.reinit ? fmaxf(key_to_float(merge_key(T.best[lane])), fl) : g0;
     }
     nu = A.p.sc.noise[scene];
     load_dirichlet(A, d1, d2);
@@ -468,8 +478,8 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int s
     float repl_gamma = 0.f;
     int xmask = 0;
     if (lane < E) {
-      const float add_e = A.p.xcand_val[scene * E + lane];
-      const int add_i = A.p.xcand_idx[scene * E + lane];
+      const float add_e = key_to_float(merge_key(T.best[lane]));
+      const int add_i = merge_index(T.best[lane]);
       const float ce = Mf;
       const float ratio = add_e / fmaxf(bnoise * ce, kTinyP);
       const float add_gain = ratio > 1.0f ? ratio - 1.0f - logf(fmaxf(ratio, kTinyP)) : 0.0f;
@@ -567,10 +577,11 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, int phase, int s
   __syncthreads();
   if (threadIdx.x == 0 && S.status) atomicOr(&A.p.status[scene], S.status);
 }
-__global__ void __launch_bounds__(kPolishThreads) polish_kernel(PolishArgs A, int phase) {
+__global__ void __launch_bounds__(kPolishThreads) polish_kernel(PolishArgs A, int phase, int lists) {
   dep_sync();
   __shared__ PolishShared S;
-  polish_body(A, S, phase, blockIdx.x);
+  __shared__ TopkMergeShared T;
+  polish_body(A, S, T, phase, lists, blockIdx.x);
 }
 
 // Residual exchange scoring (solver.py:4398-4412) without the M-space
@@ -1374,8 +1385,6 @@ __global__ void __launch_bounds__(256) output_kernel(PolishArgs A, FbmeOutputs o
 
 void launch_topk_blocks(const uint32_t* keys, long long n, int k, int B, uint32_t* cand_key, int* cand_idx,
                         cudaStream_t st);
-void launch_topk_merge(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, int B,
-                       int* out_idx, float* out_val, cudaStream_t st);
 
 // The polish steps of several shape buckets (an uneven plan's), one launch
 // each: bucket i is blockIdx.z = i with its own arguments; blocks past its
@@ -1384,6 +1393,7 @@ struct PolishSet {
   int n;
   PolishArgs a[kBucketSetMax];
   FbmeOutputs out[kBucketSetMax];
+  int slices[kBucketSetMax];      // top-k slices per scene
   int ex_blocks[kBucketSetMax];   // exchange row blocks per scene
   int out_blocks[kBucketSetMax];  // output blocks per scene
 };
@@ -1394,9 +1404,10 @@ FBME_DEV bool has_exchange(const DevConfig& c) { return c.exchange > 0 && c.poli
 __global__ void __launch_bounds__(kPolishThreads) polish_set_kernel(const PolishSet set, int phase) {
   dep_sync();
   __shared__ PolishShared S;
+  __shared__ TopkMergeShared T;
   const PolishArgs& A = set.a[blockIdx.z];
   if (phase == 1 && !has_exchange(A.c)) return;
-  polish_body(A, S, phase, blockIdx.x);
+  polish_body(A, S, T, phase, phase == 0 ? set.slices[blockIdx.z] : set.ex_blocks[blockIdx.z], blockIdx.x);
 }
 
 template <typename T>
@@ -1498,20 +1509,16 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
   const int K = c.polish_size;
   // each launch timed on its own, so the profile counts launches
   FBME_TIMED(prof, FBME_GROUP_TOPK, launch_topk_blocks(p.keys, s.n(), K, s.B, p.cand_key, p.cand_idx, st));
-  FBME_TIMED(prof, FBME_GROUP_TOPK,
-             launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * K, K, s.B, p.active, p.score, st));
   const size_t dsm = (s.n1 + s.n2) * sizeof(float2);
-  FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 0)));
+  FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 0, topk_slices(s.n()))));
   if (c.exchange > 0 && c.polish_iters > 1 && p.gram2d) {
     const long long nblk = (s.n() + 255) / 256;
     FBME_TIMED(prof, FBME_GROUP_EXCHANGE,
                (launch_dep(exchange_masked_kernel, dim3(static_cast<unsigned>(nblk < 1024 ? nblk : 1024), s.B), 256, 0, st, A)));
     FBME_TIMED(prof, FBME_GROUP_TOPK,
                launch_topk_blocks(p.keys, s.n(), c.exchange, s.B, p.cand_key, p.cand_idx, st));
-    FBME_TIMED(prof, FBME_GROUP_TOPK,
-               launch_topk_merge(p.cand_key, p.cand_idx, topk_slices(s.n()) * c.exchange, c.exchange, s.B,
-                                 p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH,
+               (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1, topk_slices(s.n()))));
   } else if (c.exchange > 0 && c.polish_iters > 1) {
     const int nb = exchange_blocks(s);
     if (s.n2 <= 64)
@@ -1522,10 +1529,7 @@ void polish_run(const BatchShape& s, const DevConfig& c, const PolishBuffers& p,
       FBME_TIMED(prof, FBME_GROUP_EXCHANGE, (launch_exchange<ExWide>(A, p, st)));
     else
       FBME_TIMED(prof, FBME_GROUP_EXCHANGE, (launch_exchange<ExWidest>(A, p, st)));
-    FBME_TIMED(prof, FBME_GROUP_TOPK,
-               launch_topk_merge(p.cand_key, p.cand_idx, nb * c.exchange, c.exchange, s.B,
-                                 p.xcand_idx, p.xcand_val, st));
-    FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1)));
+    FBME_TIMED(prof, FBME_GROUP_POLISH, (launch_dep(polish_kernel, s.B, kPolishThreads, dsm, st, A, 1, nb)));
   }
   if (cert) {  // model, scan, (decide + model, scan) per repair, final
     auto scan = p.gram2d ? cert_scan_kernel<true> : cert_scan_kernel<false>;
@@ -1574,9 +1578,8 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
     const int m = static_cast<int>(plain.size());
     auto* S = new PolishSet();  // ~31 KB: not on the stack
     TopkJobs tj{};
-    TopkMergeJobs tm{}, tx{};
     S->n = m;
-    tj.n = tm.n = m;
+    tj.n = m;
     int max_b = 1, max_slices = 1, max_out = 1;
     size_t dsm = 0;
     for (int i = 0; i < m; ++i) {
@@ -1584,20 +1587,19 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
       const int K = k.c.polish_size, sl = topk_slices(k.s.n());
       S->a[i] = PolishArgs{k.s, k.c, k.p};
       S->out[i] = k.out;
+      S->slices[i] = sl;
       S->ex_blocks[i] = exchange_blocks(k.s);
       const int fb = static_cast<int>((k.s.n() + 2047) / 2048);
       S->out_blocks[i] = fb < 64 ? fb : 64;
       tj.j[i] = TopkJob{k.p.keys, k.s.n(), K, k.s.B, k.p.cand_key, k.p.cand_idx};
-      tm.j[i] = TopkMergeJob{k.p.cand_key, k.p.cand_idx, sl * K, K, k.s.B, k.p.active, k.p.score};
       max_b = std::max(max_b, k.s.B);
       max_slices = std::max(max_slices, sl);
       max_out = std::max(max_out, S->out_blocks[i]);
       dsm = std::max(dsm, static_cast<size_t>(k.s.n1 + k.s.n2) * sizeof(float2));
     }
     launch_topk_blocks_multi(tj, max_slices, max_b, st);
-    launch_topk_merge_multi(tm, max_b, st);
     launch_dep(polish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S, 0);
-    // the exchange, one launch per row-tile class, then its candidates' merge
+    // the exchange, one launch per row-tile class
     bool any = false;
     for (int cls = 0; cls < 4; ++cls) {
       auto* X = new PolishSet();
@@ -1622,18 +1624,7 @@ void polish_run_multi(const PolishBucket* b, int n, cudaStream_t st) {
       }
       delete X;
     }
-    if (any) {
-      tx.n = 0;
-      for (int i = 0; i < m; ++i) {
-        const PolishArgs& A = S->a[i];
-        if (!(A.c.exchange > 0 && A.c.polish_iters > 1)) continue;
-        const int E = A.c.exchange;
-        tx.j[tx.n++] = TopkMergeJob{A.p.cand_key, A.p.cand_idx, S->ex_blocks[i] * E, E, A.s.B, A.p.xcand_idx,
-                                    A.p.xcand_val};
-      }
-      launch_topk_merge_multi(tx, max_b, st);
-      launch_dep(polish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S, 1);
-    }
+    if (any) launch_dep(polish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S, 1);
     launch_dep(polish_finish_set_kernel, dim3(max_b, 1, m), kPolishThreads, dsm, st, *S);
     launch_dep(output_set_kernel, dim3(max_out, max_b, m), 256, 0, st, *S);
     for (int i = 0; i < m; ++i) {

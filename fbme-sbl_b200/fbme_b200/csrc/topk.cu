@@ -4,12 +4,12 @@
 // and 4410 (residual-exchange additions).  Two launches:
 //   topk_blocks_kernel  each CTA reduces an 8192-key slice of one scene to
 //                       its k best: the keys at or above the k-th largest
-//                       thread maximum, ranked by counting (radix select
+//                       quad maximum, ranked by counting (radix select
 //                       over all register-held keys as the fallback);
-//   topk_merge_kernel   one CTA per scene sorts the candidates as 64-bit
-//                       (key, ~index) words and keeps the k first, so the
-//                       result is the exact top-k, largest first, ties by
-//                       lower index.
+//   topk_merge_kernel   one CTA per scene merges the candidates as 64-bit
+//                       (key, ~index) words, so the result is the exact
+//                       top-k, largest first, ties by lower index.
+// The replay's selections are merged by their reader, the polish kernel.
 #include "kernels.cuh"
 #include "topk.cuh"
 
@@ -18,12 +18,15 @@ namespace fbme {
 constexpr int kTopkBlockThreads = 512;
 constexpr int kTopkKpt = 16;
 constexpr int kTopkSlice = kTopkBlockThreads * kTopkKpt;  // 8192 keys per CTA
-constexpr int kMergeMax = 2048;
+constexpr int kMergeThreads = 256;
 FBME_DEV int topk_slices_dev(long long n) { return static_cast<int>((n + kTopkSlice - 1) / kTopkSlice); }
 
 // FROM_SCORES: `in` holds float scores (converted to keys); else keys.
 // The slice's k best lie among its keys at or above the k-th largest
-// thread maximum (radix bound), typically a few dozen of the 8192.
+// maximum of 64 keys, typically a few dozen of the 8192.  Latency of the
+// loads and the barriers, not bytes, bounds a block: the bound costs three
+// barriers (a radix select over the lane maxima took thirteen, 7.3 -> 6.0 us
+// for one scene of 256^2, whose 8 blocks run alone).
 template <bool FROM_SCORES>
 FBME_DEV void topk_blocks_body(const void* in, long long n, int k, uint32_t* cand_key, int* cand_idx, int scene,
                                int blk, int nblk) {
@@ -43,7 +46,7 @@ FBME_DEV void topk_blocks_body(const void* in, long long n, int k, uint32_t* can
     }
   }
   const size_t off = (static_cast<size_t>(scene) * nblk + blk) * k;
-  block_topk_pruned<kTopkKpt, false, TopkBound::kRadix>(
+  block_topk_pruned<kTopkKpt, false, TopkBound::kQuads>(
       key, valid, [&](int i) { return static_cast<int>(base + static_cast<long long>(i) * kTopkBlockThreads); }, k,
       S, cand_key + off, cand_idx + off);
 }
@@ -66,57 +69,19 @@ __global__ void __launch_bounds__(kTopkBlockThreads, 2) topk_blocks_multi_kernel
 }
 
 template <typename Idx>
-FBME_DEV void topk_merge_body(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, Idx* out_idx,
-                              float* out_val, int scene) {
-  __shared__ unsigned long long s[kMergeMax];
-  int np = 1;
-  while (np < ncand) np <<= 1;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    unsigned long long w = 0ull;
-    if (i < ncand) {
-      const size_t e = static_cast<size_t>(scene) * ncand + i;
-      w = (static_cast<unsigned long long>(cand_key[e]) << 32) |
-          static_cast<unsigned long long>(0xFFFFFFFFu - static_cast<uint32_t>(cand_idx[e]));
-    }
-    s[i] = w;
-  }
-  __syncthreads();
-  // bitonic sort, descending
-  for (int size = 2; size <= np; size <<= 1)
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const bool desc = (i & size) == 0;
-          const unsigned long long a = s[i], b = s[j];
-          if (desc ? (a < b) : (a > b)) {
-            s[i] = b;
-            s[j] = a;
-          }
-        }
-      }
-      __syncthreads();
-    }
+__global__ void __launch_bounds__(kMergeThreads)
+topk_merge_kernel(const uint32_t* cand_key, const int* cand_idx, int lists, int k, Idx* out_idx, float* out_val) {
+  dep_sync();
+  __shared__ unsigned long long list[kMergeMax];
+  __shared__ TopkMergeShared M;
+  const int scene = blockIdx.x;
+  const size_t off = static_cast<size_t>(scene) * lists * k;
+  block_topk_merge<kMergeMax / kMergeThreads>(cand_key + off, cand_idx + off, lists, k, list, M);
   if (threadIdx.x < k) {
-    const unsigned long long w = s[threadIdx.x];
-    out_idx[scene * k + threadIdx.x] = static_cast<Idx>(0xFFFFFFFFu - static_cast<uint32_t>(w));
-    out_val[scene * k + threadIdx.x] = key_to_float(static_cast<uint32_t>(w >> 32));
+    const unsigned long long w = M.best[threadIdx.x];
+    out_idx[scene * k + threadIdx.x] = static_cast<Idx>(merge_index(w));
+    out_val[scene * k + threadIdx.x] = key_to_float(merge_key(w));
   }
-}
-
-template <typename Idx>
-__global__ void __launch_bounds__(1024)
-topk_merge_kernel(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, Idx* out_idx,
-                  float* out_val) {
-  dep_sync();
-  topk_merge_body<Idx>(cand_key, cand_idx, ncand, k, out_idx, out_val, blockIdx.x);
-}
-
-__global__ void __launch_bounds__(1024) topk_merge_multi_kernel(const TopkMergeJobs J) {
-  dep_sync();
-  const TopkMergeJob& j = J.j[blockIdx.z];
-  if (static_cast<int>(blockIdx.x) >= j.B) return;
-  topk_merge_body<int>(j.cand_key, j.cand_idx, j.ncand, j.k, j.out_idx, j.out_val, blockIdx.x);
 }
 
 int topk_slices(long long n) { return static_cast<int>((n + kTopkSlice - 1) / kTopkSlice); }
@@ -124,24 +89,10 @@ int topk_slices(long long n) { return static_cast<int>((n + kTopkSlice - 1) / kT
 void launch_topk_blocks_multi(const TopkJobs& J, int max_slices, int max_b, cudaStream_t st) {
   launch_dep(topk_blocks_multi_kernel, dim3(max_slices, max_b, J.n), kTopkBlockThreads, 0, st, J);
 }
-void launch_topk_merge_multi(const TopkMergeJobs& J, int max_b, cudaStream_t st) {
-  launch_dep(topk_merge_multi_kernel, dim3(max_b, 1, J.n), 1024, 0, st, J);
-}
 
 void launch_topk_blocks(const uint32_t* keys, long long n, int k, int B, uint32_t* cand_key, int* cand_idx,
                         cudaStream_t st) {
   launch_dep(topk_blocks_kernel<false>, dim3(topk_slices(n), B), kTopkBlockThreads, 0, st, keys, n, k, cand_key, cand_idx);
-}
-
-void launch_topk(const uint32_t* keys, long long n, int k, int B, uint32_t* cand_key, int* cand_idx,
-                 int* out_idx, float* out_val, cudaStream_t st) {
-  launch_topk_blocks(keys, n, k, B, cand_key, cand_idx, st);
-  launch_dep(topk_merge_kernel<int>, B, 1024, 0, st, cand_key, cand_idx, topk_slices(n) * k, k, out_idx, out_val);
-}
-
-void launch_topk_merge(const uint32_t* cand_key, const int* cand_idx, int ncand, int k, int B,
-                       int* out_idx, float* out_val, cudaStream_t st) {
-  launch_dep(topk_merge_kernel<int>, B, 1024, 0, st, cand_key, cand_idx, ncand, k, out_idx, out_val);
 }
 
 // Candidate scratch of the score top-k: per row, one k-list per 8192-score slice.
@@ -167,7 +118,7 @@ void topk_scores(const float* scores, long long n, int k, int batch, void* scrat
   uint32_t* ck = static_cast<uint32_t*>(scratch);
   int* ci = reinterpret_cast<int*>(ck + static_cast<size_t>(batch) * nblk * k);
   launch_dep(topk_blocks_kernel<true>, dim3(nblk, batch), kTopkBlockThreads, 0, st, scores, n, k, ck, ci);
-  launch_dep(topk_merge_kernel<int64_t>, batch, 1024, 0, st, ck, ci, nblk * k, k, indices, values);
+  launch_dep(topk_merge_kernel<int64_t>, batch, kMergeThreads, 0, st, ck, ci, nblk, k, indices, values);
 }
 
 }  // namespace fbme

@@ -1,10 +1,11 @@
 // Block-wide top-k (k <= 32) over order-preserving 32-bit keys held in
 // registers, with the index-order tie break of a stable descending sort.
 //
-// Used twice per selection: many CTAs per scene each reduce a slice of the
-// grid to k candidates, then one CTA per scene merges the candidates; the
-// result is exactly the k largest keys of the scene (largest first, ties by
-// lower index), which is what torch.topk returns at solver.py:1931/4410.
+// Many CTAs per scene each reduce a slice of the grid to a sorted list of k
+// candidates (block_topk, block_topk_pruned), then one CTA per scene merges
+// the lists (block_topk_merge): the result is exactly the k largest keys of
+// the scene (largest first, ties by lower index), which is what torch.topk
+// returns at solver.py:1931/4410.
 #pragma once
 
 #include "common.cuh"
@@ -61,36 +62,6 @@ FBME_DEV void radix_pick_bin(TopkShared& S, int shift, uint32_t prefix, uint32_t
     S.prefix = prefix | (static_cast<uint32_t>(sel) << shift);
     S.mask = mask | (255u << shift);
   }
-}
-
-// k-th largest of the valid keys held one per thread (1 <= k <= their
-// number): radix select with 8-bit digits, histogram counts aggregated per
-// warp (the keys crowd into few top-byte bins).  Ends on a barrier.
-FBME_DEV uint32_t block_kth_key(uint32_t key, bool valid, int k, TopkShared& S) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) {
-    S.prefix = 0;
-    S.mask = 0;
-    S.remaining = k;
-  }
-#pragma unroll 1
-  for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 24 - 8 * pass;
-    for (int b = tid; b < 256; b += blockDim.x) S.hist[b] = 0;
-    __syncthreads();
-    const uint32_t prefix = S.prefix, mask = S.mask;
-    const bool part = valid && (key & mask) == prefix;
-    const unsigned act = __ballot_sync(0xffffffffu, part);
-    if (part) {
-      const uint32_t bin = (key >> shift) & 255u;
-      const unsigned peers = __match_any_sync(act, bin);
-      if (__ffs(peers) - 1 == lane) atomicAdd(&S.hist[bin], static_cast<uint32_t>(__popc(peers)));
-    }
-    __syncthreads();
-    if (warp == 0) radix_pick_bin(S, shift, prefix, mask);
-    __syncthreads();
-  }
-  return S.prefix;
 }
 
 // Block-wide top-k (k <= 32) of the valid (key, gidx) pairs held KPT per
@@ -251,18 +222,19 @@ struct TopkPrunedShared {
 
 // How block_topk_pruned finds its bound T0: kWarpSort sorts each warp's
 // lane maxima and ranks the warps' k largest by counting (few warps x small
-// k); kRadix runs a radix select over the lane maxima (large k).
-enum class TopkBound { kWarpSort, kRadix };
+// k); kQuads takes the k-th largest maximum of four lanes' keys, ranked by
+// counting too (any k up to 32 on blocks of 128 threads or more).
+enum class TopkBound { kWarpSort, kQuads };
 
 // Block-wide top-k (k <= 32) with the result of block_topk, for key sets
 // whose k best are few among many.  Every thread's largest key is a lane
-// maximum; the k-th largest lane maximum T0 is a lower bound on the
-// block's k-th key (k different threads hold a key >= T0), so the block's
-// top k are among the keys >= T0, typically little more than k of them.
-// The keys >= T0 go on a shared list, where each finds its output place by
-// counting the entries ahead of it (key desc, index asc).  A zero bound,
-// fewer than k threads with a key, or a list longer than kPrunedCap falls
-// back to the radix select over all keys.  valid: bit i set when entry i
+// maximum; the k-th largest maximum T0 of the lanes (or of the quads of
+// lanes) is a lower bound on the block's k-th key (k different ones hold a
+// key >= T0), so the block's top k are among the keys >= T0, typically
+// little more than k of them.  The keys >= T0 go on a shared list, where each
+// finds its output place by counting the entries ahead of it (key desc,
+// index asc).  A zero bound (as with fewer than k maxima) or a list longer
+// than kPrunedCap falls back to the radix select over all keys.  valid: bit i set when entry i
 // counts; gidx(i): its index.  The block is whole warps.
 template <int KPT, bool AGG, TopkBound BOUND = TopkBound::kWarpSort, typename GIdx>
 FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx gidx, int k,
@@ -314,12 +286,32 @@ FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx
     __syncthreads();
     t0 = P.t0;
   } else {
-    if (tid == 0) P.ncand = 0;
-    if (__syncthreads_count(valid != 0u) < k) {
+    const int quads = blockDim.x >> 2;
+    if (quads < k || quads > kPrunedLaneMax) {
       radix();
       return;
     }
-    t0 = block_kth_key(m, valid != 0u, k, P.radix);
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    if ((tid & 3) == 0) P.lane_max[tid >> 2] = m;
+    if (tid == 0) {
+      P.t0 = 0u;
+      P.ncand = 0;
+    }
+    __syncthreads();
+    if (tid < quads) {
+      // place among the maxima, ties by position: unique
+      const uint32_t me = P.lane_max[tid];
+      int rank = 0;
+#pragma unroll 8
+      for (int j = 0; j < quads; ++j) {
+        const uint32_t o = P.lane_max[j];
+        rank += (o > me || (o == me && j < tid)) ? 1 : 0;
+      }
+      if (rank == k - 1) P.t0 = me;
+    }
+    __syncthreads();
+    t0 = P.t0;
   }
   if (t0 == 0u) {
     radix();
@@ -348,6 +340,86 @@ FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx
       out_key[rank] = me.x;
       out_idx[rank] = static_cast<int>(me.y);
     }
+  }
+  __syncthreads();
+}
+
+// Candidates of a merge: at most kMergeMax, in lists of k sorted (key desc,
+// index asc).  One candidate is one 64-bit word (key, ~index).
+constexpr int kMergeMax = 2048;
+struct TopkMergeShared {
+  unsigned long long hi[32], lo[32];  // per warp
+  unsigned long long best[32];        // the result, largest first
+  int n;
+};
+FBME_DEV uint32_t merge_key(unsigned long long w) { return static_cast<uint32_t>(w >> 32); }
+FBME_DEV int merge_index(unsigned long long w) { return static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(w)); }
+
+// The k best (k <= 32) of `lists` lists, into M.best, by one block of at
+// least kMergeMax / NR threads; `list` is shared scratch of kMergeMax words.
+// Each list's k-th entry bounds the k-th of all from below, and so does the
+// smallest of the lists' ceil(k / lists)-th entries (at least k entries are
+// as large); the candidates at or above the larger bound, typically two or
+// three times k, find their places by counting those ahead of them.  Two
+// rounds of loads and three barriers where a bitonic sort of all candidates
+// takes 36 (8 lists of 32) to 66 barriers.  In the polish kernel that reads
+// the result it adds 4 us to a replay's path where the merge's own launch
+// took 7 (one scene of 256^2 151 -> 147 us, 512 scenes 3125 -> 3086 us with
+// the shorter bound of the slices).
+template <int NR>
+FBME_DEV void block_topk_merge(const uint32_t* ck, const int* ci, int lists, int k, unsigned long long* list,
+                               TopkMergeShared& M) {
+  const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x, nw = nt >> 5;
+  const int n = lists * k, mid = (k + lists - 1) / lists - 1;
+  auto word = [&](int i) {
+    return (static_cast<unsigned long long>(ck[i]) << 32) |
+           static_cast<unsigned long long>(0xFFFFFFFFu - static_cast<uint32_t>(ci[i]));
+  };
+  unsigned long long c[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r) c[r] = tid + r * nt < n ? word(tid + r * nt) : 0ull;
+  unsigned long long hi = 0ull, lo = ~0ull;
+  for (int l = tid; l < lists; l += nt) {
+    hi = max(hi, word(l * k + k - 1));
+    lo = min(lo, word(l * k + mid));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+  }
+  if (lane == 0) {
+    M.hi[tid >> 5] = hi;
+    M.lo[tid >> 5] = lo;
+  }
+  if (tid == 0) M.n = 0;
+  __syncthreads();
+  for (int w = 0; w < nw; ++w) {
+    hi = max(hi, M.hi[w]);
+    lo = min(lo, M.lo[w]);
+  }
+  const unsigned long long bound = max(hi, lo);
+#pragma unroll
+  for (int r = 0; r < NR; ++r) {
+    const bool in = tid + r * nt < n && c[r] >= bound;
+    const unsigned ball = __ballot_sync(0xffffffffu, in);
+    if (ball == 0u) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&M.n, __popc(ball));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (in) list[base + __popc(ball & ((1u << lane) - 1u))] = c[r];
+  }
+  __syncthreads();
+  const int m = M.n;
+  for (int i = tid; i < m; i += nt) {
+    const unsigned long long me = list[i];
+    int rank = 0;
+#pragma unroll 8
+    for (int j = 0; j < m; ++j) {
+      const unsigned long long o = list[j];
+      rank += (o > me || (o == me && j < i)) ? 1 : 0;
+    }
+    if (rank < k) M.best[rank] = me;
   }
   __syncthreads();
 }
