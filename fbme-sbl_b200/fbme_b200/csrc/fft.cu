@@ -393,62 +393,50 @@ __host__ __device__ constexpr int fast_row_area(int L) {
   while (a % 16 != P % 16) ++a;
   return a;
 }
-// two buffers of ROWS rows (the input rows, then in place the exchange
-// and the output staging)
-constexpr size_t fast_smem_bytes(int L) {
-  return 2 * static_cast<size_t>(kFftThreads / fast_threads_per_row(L)) * fast_row_area(L) * sizeof(float2);
+// one buffer of ROWS rows (the exchange, then in place the output staging)
+__host__ __device__ constexpr size_t fast_smem_bytes(int L) {
+  return static_cast<size_t>(kFftThreads / fast_threads_per_row(L)) * fast_row_area(L) * sizeof(float2);
+}
+// Blocks per SM: three where a row's Q values leave room for 80 registers a
+// thread, else two of up to 128 registers; two for the denoiser, whose
+// operands want the registers (512 scenes of 256^2: 263 us a sweep, 277 with
+// three blocks).
+__host__ __device__ constexpr int fast_blocks(int L, int epi) {
+  return epi != 2 && L / fast_threads_per_row(L) <= 16 ? 3 : 2;
 }
 
-FBME_DEV void cp_async8(float2* dst, const float2* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-FBME_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 FBME_DEV void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-template <int N>
-FBME_DEV void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// Asynchronous copy of the values thread (lr, p) transforms in tile t:
-// x[p + P q] of row lr with p + P q < K (the rest of the row is zero and is
-// never copied); one commit group.
+// The values thread (lr, p) transforms: x[p + P q] of row r for p + P q < K,
+// straight into its registers.
 template <int L>
-FBME_DEV void fast_issue(const FftStage& st, const FftIo& io, int t, float2* buf, int lr, int p) {  // t: the item's tile
-  constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P, A = fast_row_area(L);
-  const int unit = t / st.tiles, tile = t - unit * st.tiles;
-  const int r = tile * ROWS + lr;
-  if (r < st.rows) {
-    const float2* src = io.in + unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
-    float2* dst = buf + lr * A + p;
+FBME_DEV void row_values(const FftStage& st, const float2* in, int unit, int r, int p,
+                         float2 (&v)[L / fast_threads_per_row(L)]) {
+  constexpr int P = fast_threads_per_row(L), Q = L / P;
+  const bool live = r < st.rows;
+  const float2* src = in + unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
-      if (p + P * q < st.kin) cp_async8(dst + P * q, src + P * q);
+  for (int q = 0; q < Q; ++q)
+    v[q] = live && p + P * q < st.kin ? __ldg(src + P * q) : make_float2(0.f, 0.f);
+}
+// Rows r0 .. r0 + rows of a stage's input into L2.
+FBME_DEV void rows_prefetch(const FftStage& st, const float2* in, int unit, int r0, int rows) {
+  const int lines = (st.kin * 8 + 127) / 128 + 1;  // 128-byte lines a row touches, at most
+  const long long last = static_cast<long long>(st.rows) * st.in_ld - 1;
+  for (int i = threadIdx.x; i < rows * lines; i += kFftThreads) {
+    const long long e = static_cast<long long>(r0 + i / lines) * st.in_ld + (i % lines) * 16;
+    prefetch_l2(in + unit * st.in_stride + (e < last ? e : last));
   }
-  cp_async_commit();
 }
 
 // The values thread (lr, p) transforms in tile t under mode 4, straight into
 // its registers: the message update of x[p + P q] for p + P q < K, written to
 // the new message as well.  A batch's loads are issued before its stores.
-// The next tile's rows are prefetched into L2, not into shared memory: the two
-// blocks of an SM overlap each other's loads.  512 scenes of 256^2 / 128^2:
-// message kernel and stage 48 + 51 us, fused 87 us; 61 us is the copy rate's
-// time for the bytes that remain.
-FBME_DEV void message_prefetch(const FftStage& st, const MessageArgs& ms, int unit, int r0, int rows) {
-  const int lines = (st.kin * 8 + 127) / 128 + 1;  // 128-byte lines a row touches, at most
-  const long long last = static_cast<long long>(st.rows) * st.in_ld - 1;
-  for (int i = threadIdx.x; i < rows * lines; i += kFftThreads) {
-    const long long in_row = static_cast<long long>(r0 + i / lines) * st.in_ld + (i % lines) * 16;
-    const long long e = unit * st.in_stride + (in_row < last ? in_row : last);
-    prefetch_l2(ms.y + e);
-    prefetch_l2(ms.pred + e);
-    prefetch_l2(ms.in + e);
-  }
-}
+// 512 scenes of 256^2 / 128^2: message kernel and stage 48 + 51 us, fused 85;
+// 61 us is the copy rate's time for the bytes that remain.
 template <int L>
 FBME_DEV void message_rows(const FftStage& st, const MessageArgs& ms, int unit, int r, int p,
                            float2 (&v)[L / fast_threads_per_row(L)]) {
-  constexpr int P = fast_threads_per_row(L), Q = L / P, NB = Q % 8 == 0 && Q <= 16 ? 8 : Q % 4 == 0 ? 4 : 3;
+  constexpr int P = fast_threads_per_row(L), Q = L / P, NB = Q % 4 == 0 ? 4 : 3;
   static_assert(Q % NB == 0, "whole batches");
   const bool live = r < st.rows;
   const long long e0 = unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
@@ -481,28 +469,28 @@ FBME_DEV void message_rows(const FftStage& st, const MessageArgs& ms, int unit, 
 }
 
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (tile t = unit x
-// tiles + row tile); the copy of its next tile is in flight while the
-// current one is transformed.
+// tiles + row tile); the rows (and epilogue operands) of its next tile are
+// prefetched into L2 while the current one is transformed.  HBM and the
+// latency of the loads bound it.  The rows go straight to registers: copied
+// through a second shared-memory buffer (cp.async) they took a third of the
+// shared-memory traffic and half of the SM's shared memory, which left one
+// block an SM at L = 192 and 512 and two at 256, and little L1.  Forward
+// stage 1 of 512 scenes of 256^2 / 128^2 94 -> 81 us (61 at the copy rate),
+// residual stage 70 -> 65; a replay of 64 uneven scenes 1118 -> 1011 us, of
+// 32 scenes of 512^2 1255 -> 1173.
 // EPI: 0 store (modes 0 and 1), 1 residual (mode 2), 2 denoiser (mode 3),
 // 3 store of the message update (mode 4)
 template <int L, int S, int EPI>
-__global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage st, const FftIo io) {
+__global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_kernel(const FftStage st, const FftIo io) {
   dep_sync();
   constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P;
   constexpr int J = (Q + P - 1) / P;     // output columns k1 per thread in pass 2
   constexpr int A = fast_row_area(L);    // row stride of a buffer
-  constexpr int BUF = ROWS * A;
   extern __shared__ float2 fsm[];
   const int lr = threadIdx.x / P, p = threadIdx.x % P;
   const int total = st.tiles * st.units;
   int t = blockIdx.x;
-  if (EPI != 3 && t < total) fast_issue<L>(st, io, t, fsm, lr, p);
-  for (int it = 0; t < total; ++it, t += gridDim.x) {
-    float2* buf = fsm + (it & 1) * BUF;
-    if (EPI != 3 && t + static_cast<int>(gridDim.x) < total)
-      fast_issue<L>(st, io, t + gridDim.x, fsm + ((it + 1) & 1) * BUF, lr, p);
-    else
-      cp_async_commit();  // empty group: the wait below counts the same
+  for (; t < total; t += gridDim.x) {
     if constexpr (EPI == 1 || EPI == 2) {
       // the next tile's epilogue operands (observations; prior, mean and
       // variance) into L2, one line per output column and array, so their
@@ -523,24 +511,26 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
         }
       }
     }
-    if constexpr (EPI == 3) {
-      const int tn = t + gridDim.x;
-      if (tn < total) message_prefetch(st, io.ms, tn / st.tiles, (tn % st.tiles) * ROWS, ROWS);
+    if (t + static_cast<int>(gridDim.x) < total) {
+      const int tn = t + gridDim.x, un = tn / st.tiles, rn = (tn - un * st.tiles) * ROWS;
+      if constexpr (EPI == 3) {
+        rows_prefetch(st, io.ms.y, un, rn, ROWS);
+        rows_prefetch(st, io.ms.pred, un, rn, ROWS);
+        rows_prefetch(st, io.ms.in, un, rn, ROWS);
+      } else {
+        rows_prefetch(st, io.in, un, rn, ROWS);
+      }
     }
-    cp_async_wait<1>();   // this thread's copies of tile t (it reads only its own)
     const int unit = t / st.tiles, tile = t - unit * st.tiles;
     const int r0 = tile * ROWS;
-    const bool live = r0 + lr < st.rows;
-    float2* ya = buf + lr * A;
+    float2* ya = fsm + lr * A;
 
     // pass 1: DFT-Q of x[p + P q] in registers
     float2 v[Q];
     if constexpr (EPI == 3) {
       message_rows<L>(st, io.ms, unit, r0 + lr, p, v);
     } else {
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+      row_values<L>(st, io.in, unit, r0 + lr, p, v);
     }
     if (io.ysum) {
       float acc = 0.f;
@@ -549,7 +539,6 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
       const double w = warp_sum(static_cast<double>(acc));
       if ((threadIdx.x & 31) == 0) *part_slot(io.part, unit, tile, 3 * kPartWarps + (threadIdx.x >> 5)) = w;
     }
-    __syncwarp();  // the row's inputs are read before the exchange overwrites them
     RegDft<Q, S>::run(v);
 #pragma unroll
     for (int k1 = 0; k1 < Q; ++k1) {
@@ -599,14 +588,14 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
     // CH columns ahead, the first chunk before the barrier, so that their
     // latency overlaps it.
     constexpr int NC = L / P;
-    constexpr int CH = NC <= 16 ? NC : (NC % 16 == 0 ? 16 : 8);
+    constexpr int CH = fast_blocks(L, EPI) == 3 && NC % 8 == 0 ? 8 : NC <= 16 ? NC : (NC % 16 == 0 ? 16 : 8);
     const int row = threadIdx.x % ROWS, c0 = threadIdx.x / ROWS;
     const int rr = r0 + row;
     const bool live_out = rr < st.rows;
     const long long base = unit * st.out_stride;
     const long long o0 = static_cast<long long>(c0) * st.out_ld + rr;
     const long long step = static_cast<long long>(P) * st.out_ld;
-    const float2* sp = buf + row * A + row;
+    const float2* sp = fsm + row * A + row;
     if constexpr (EPI == 0 || EPI == 3) {
       __syncthreads();
       float acc = 0.f;
@@ -663,7 +652,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
       if ((threadIdx.x & 31) == 0) *part_slot(io.part, unit, tile, 2 * kPartWarps + (threadIdx.x >> 5)) = w;
     } else {
       // four registers a column: chunks of at most 8 columns
-      constexpr int CD = NC % 8 == 0 ? 8 : (NC % 4 == 0 ? 4 : NC);
+      constexpr int CD = fast_blocks(L, EPI) == 2 && NC % 8 == 0 ? 8 : (NC % 4 == 0 ? 4 : NC);
       const DenoiseArgs& dn = io.dn;
       float gv[CD], vv[CD];
       float2 mv[CD];
@@ -711,9 +700,8 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
         *part_slot(io.part, unit, tile, 1 * kPartWarps + (threadIdx.x >> 5)) = w1;
       }
     }
-    __syncthreads();  // this buffer takes the copy issued at the top of the next tile
+    __syncthreads();  // the next tile's exchange overwrites the staging
   }
-  cp_async_wait<0>();
 }
 
 // The same kernel over a set of same-length stages (uneven plans' shape
@@ -721,31 +709,25 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_kernel(const FftStage
 // computed exactly as that item's own launch computes it.  A separate
 // kernel, so that the single-stage kernel keeps its code.
 template <int L, int S, int EPI, int NMAX>
-__global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftSet<NMAX> set) {
+__global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_set_kernel(const FftSet<NMAX> set) {
   dep_sync();
   constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P;
   constexpr int J = (Q + P - 1) / P;     // output columns k1 per thread in pass 2
   constexpr int A = fast_row_area(L);    // row stride of a buffer
-  constexpr int BUF = ROWS * A;
   extern __shared__ float2 fsm[];
   const int lr = threadIdx.x / P, p = threadIdx.x % P;
   const int total = set.tile0[set.n];
   int t = blockIdx.x;
-  if (EPI != 3 && t < total) {
-    const int i = fft_set_item(set, t);
-    fast_issue<L>(set.st[i], set.io[i], t - set.tile0[i], fsm, lr, p);
-  }
-  for (int it = 0; t < total; ++it, t += gridDim.x) {
+  for (; t < total; t += gridDim.x) {
     const int item = fft_set_item(set, t);
     const FftStage& st = set.st[item];
     const FftIo& io = set.io[item];
-    float2* buf = fsm + (it & 1) * BUF;
     const int tn = t + gridDim.x;
     if (EPI != 3 && tn < total) {
       const int in_ = fft_set_item(set, tn);
       const FftStage& sn = set.st[in_];
       const int tl = tn - set.tile0[in_];
-      fast_issue<L>(sn, set.io[in_], tl, fsm + ((it + 1) & 1) * BUF, lr, p);
+      rows_prefetch(sn, set.io[in_].in, tl / sn.tiles, (tl % sn.tiles) * ROWS, ROWS);
       if constexpr (EPI == 1 || EPI == 2) {
         // the next tile's epilogue operands (observations; prior, mean and
         // variance) into L2, one line per output column and array, so their
@@ -764,24 +746,18 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
           }
         }
       }
-    } else {
-      cp_async_commit();  // empty group: the wait below counts the same
     }
-    cp_async_wait<1>();   // this thread's copies of tile t (it reads only its own)
     const int tloc = t - set.tile0[item];
     const int unit = tloc / st.tiles, tile = tloc - unit * st.tiles;
     const int r0 = tile * ROWS;
-    const bool live = r0 + lr < st.rows;
-    float2* ya = buf + lr * A;
+    float2* ya = fsm + lr * A;
 
     // pass 1: DFT-Q of x[p + P q] in registers
     float2 v[Q];
     if constexpr (EPI == 3) {
       message_rows<L>(st, io.ms, unit, r0 + lr, p, v);
     } else {
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        v[q] = (live && p + P * q < st.kin) ? ya[p + P * q] : make_float2(0.f, 0.f);
+      row_values<L>(st, io.in, unit, r0 + lr, p, v);
     }
     if (io.ysum) {
       float acc = 0.f;
@@ -790,7 +766,6 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
       const double w = warp_sum(static_cast<double>(acc));
       if ((threadIdx.x & 31) == 0) *part_slot(io.part, unit, tile, 3 * kPartWarps + (threadIdx.x >> 5)) = w;
     }
-    __syncwarp();  // the row's inputs are read before the exchange overwrites them
     RegDft<Q, S>::run(v);
 #pragma unroll
     for (int k1 = 0; k1 < Q; ++k1) {
@@ -840,14 +815,14 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
     // CH columns ahead, the first chunk before the barrier, so that their
     // latency overlaps it.
     constexpr int NC = L / P;
-    constexpr int CH = NC <= 16 ? NC : (NC % 16 == 0 ? 16 : 8);
+    constexpr int CH = fast_blocks(L, EPI) == 3 && NC % 8 == 0 ? 8 : NC <= 16 ? NC : (NC % 16 == 0 ? 16 : 8);
     const int row = threadIdx.x % ROWS, c0 = threadIdx.x / ROWS;
     const int rr = r0 + row;
     const bool live_out = rr < st.rows;
     const long long base = unit * st.out_stride;
     const long long o0 = static_cast<long long>(c0) * st.out_ld + rr;
     const long long step = static_cast<long long>(P) * st.out_ld;
-    const float2* sp = buf + row * A + row;
+    const float2* sp = fsm + row * A + row;
     if constexpr (EPI == 0 || EPI == 3) {
       __syncthreads();
       float acc = 0.f;
@@ -904,7 +879,7 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
       if ((threadIdx.x & 31) == 0) *part_slot(io.part, unit, tile, 2 * kPartWarps + (threadIdx.x >> 5)) = w;
     } else {
       // four registers a column: chunks of at most 8 columns
-      constexpr int CD = NC % 8 == 0 ? 8 : (NC % 4 == 0 ? 4 : NC);
+      constexpr int CD = fast_blocks(L, EPI) == 2 && NC % 8 == 0 ? 8 : (NC % 4 == 0 ? 4 : NC);
       const DenoiseArgs& dn = io.dn;
       float gv[CD], vv[CD];
       float2 mv[CD];
@@ -952,9 +927,8 @@ __global__ void __launch_bounds__(kFftThreads, 2) fft_fast_set_kernel(const FftS
         *part_slot(io.part, unit, tile, 1 * kPartWarps + (threadIdx.x >> 5)) = w1;
       }
     }
-    __syncthreads();  // this buffer takes the copy issued at the top of the next tile
+    __syncthreads();  // the next tile's exchange overwrites the staging
   }
-  cp_async_wait<0>();
 }
 
 template <int L, int S, int EPI>
@@ -1098,10 +1072,10 @@ cudaError_t set_fft_attributes() {
 // One FFT stage of `units` transforms (the geometry of the GEMM stage `g`,
 // whose contracted length K is padded to the transform length L).
 // The fused denoiser epilogue and the message update formed in the load pay
-// where two CTAs fit on an SM; at L = 512 (one CTA of 147 KB) their loads find
-// too few warps, and the elementwise kernels at full occupancy are faster (32
-// scenes of 512^2 / 256^2: message update fused 1.27 ms a replay, by itself
-// 1.25 ms; 512 scenes of 256^2 / 128^2: fused 3.13 ms, by itself 3.17 ms).
+// where a row's values leave their operands registers; at L = 512 (32 values
+// a thread) the elementwise kernels at full occupancy are faster (32 scenes
+// of 512^2 / 256^2: both fused 1.25 ms a replay, by themselves 1.17 ms; 512
+// scenes of 256^2 / 128^2: message fused 3.13 ms, by itself 3.17 ms).
 int fft_message_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
 int fft_denoise_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
 
