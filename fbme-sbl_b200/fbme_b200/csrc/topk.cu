@@ -46,7 +46,7 @@ FBME_DEV void topk_blocks_body(const void* in, long long n, int k, uint32_t* can
     }
   }
   const size_t off = (static_cast<size_t>(scene) * nblk + blk) * k;
-  block_topk_pruned<kTopkKpt, false, TopkBound::kQuads>(
+  block_topk_pruned<kTopkKpt, false>(
       key, valid, [&](int i) { return static_cast<int>(base + static_cast<long long>(i) * kTopkBlockThreads); }, k,
       S, cand_key + off, cand_idx + off);
 }

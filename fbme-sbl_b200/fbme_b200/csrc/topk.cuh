@@ -210,7 +210,7 @@ FBME_DEV void block_topk(const uint32_t (&key)[KPT], const int (&gidx)[KPT], con
 }
 
 constexpr int kPrunedCap = 256;
-constexpr int kPrunedLaneMax = 256;  // warps x k lane maxima ranked for the bound
+constexpr int kPrunedLaneMax = 256;  // quad maxima ranked for the bound
 
 struct TopkPrunedShared {
   TopkShared radix;  // the fallback's
@@ -220,27 +220,22 @@ struct TopkPrunedShared {
   uint2 cand[kPrunedCap];  // (key, index)
 };
 
-// How block_topk_pruned finds its bound T0: kWarpSort sorts each warp's
-// lane maxima and ranks the warps' k largest by counting (few warps x small
-// k); kQuads takes the k-th largest maximum of four lanes' keys, ranked by
-// counting too (any k up to 32 on blocks of 128 threads or more).
-enum class TopkBound { kWarpSort, kQuads };
-
 // Block-wide top-k (k <= 32) with the result of block_topk, for key sets
-// whose k best are few among many.  Every thread's largest key is a lane
-// maximum; the k-th largest maximum T0 of the lanes (or of the quads of
-// lanes) is a lower bound on the block's k-th key (k different ones hold a
-// key >= T0), so the block's top k are among the keys >= T0, typically
-// little more than k of them.  The keys >= T0 go on a shared list, where each
-// finds its output place by counting the entries ahead of it (key desc,
-// index asc).  A zero bound (as with fewer than k maxima) or a list longer
-// than kPrunedCap falls back to the radix select over all keys.  valid: bit i set when entry i
+// whose k best are few among many.  The k-th largest maximum T0 of the quads
+// of lanes is a lower bound on the block's k-th key (k different quads hold a
+// key >= T0), so the block's top k are among the keys >= T0, typically little
+// more than k of them; two shuffles and a count over the quads find it (the
+// exchange of 512 scenes: 330 us with a sort of each warp's lane maxima,
+// 322).  The keys >= T0 go on a shared list, where each finds its output
+// place by counting the entries ahead of it (key desc, index asc).  A zero
+// bound (as with fewer than k maxima) or a list longer than kPrunedCap falls
+// back to the radix select over all keys.  valid: bit i set when entry i
 // counts; gidx(i): its index.  The block is whole warps.
-template <int KPT, bool AGG, TopkBound BOUND = TopkBound::kWarpSort, typename GIdx>
+template <int KPT, bool AGG, typename GIdx>
 FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx gidx, int k,
                                 TopkPrunedShared& P, uint32_t* out_key, int* out_idx) {
   static_assert(KPT <= 32, "the valid mask holds 32 entries");
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   auto radix = [&]() {
     block_topk_fn<KPT, AGG>(
         key, [&](int i) { return ((valid >> i) & 1u) != 0u; }, gidx, k, P.radix, out_key, out_idx);
@@ -249,70 +244,32 @@ FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx
 #pragma unroll
   for (int i = 0; i < KPT; ++i)
     if ((valid >> i) & 1u) m = max(m, key[i]);
-  uint32_t t0 = 0u;
-  if constexpr (BOUND == TopkBound::kWarpSort) {
-    // each warp offers its k largest lane maxima, which hold the block's k
-    // largest; T0 is found among them by counting
-    const int offered = (blockDim.x >> 5) * k;
-    if (offered > kPrunedLaneMax) {
-      radix();
-      return;
-    }
-    // bitonic sort of the warp's lane maxima, descending
-#pragma unroll
-    for (int size = 2; size <= 32; size <<= 1)
-#pragma unroll
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        const uint32_t o = __shfl_xor_sync(0xffffffffu, m, stride);
-        const bool keep_max = ((lane & stride) == 0) == ((lane & size) == 0);
-        m = keep_max ? max(m, o) : min(m, o);
-      }
-    if (lane < k) P.lane_max[warp * k + lane] = m;
-    if (tid == 0) {
-      P.t0 = 0u;
-      P.ncand = 0;
-    }
-    __syncthreads();
-    if (tid < offered) {
-      // place among the offered maxima, ties by position: unique
-      const uint32_t me = P.lane_max[tid];
-      int rank = 0;
-      for (int j = 0; j < offered; ++j) {
-        const uint32_t o = P.lane_max[j];
-        rank += (o > me || (o == me && j < tid)) ? 1 : 0;
-      }
-      if (rank == k - 1) P.t0 = me;
-    }
-    __syncthreads();
-    t0 = P.t0;
-  } else {
-    const int quads = blockDim.x >> 2;
-    if (quads < k || quads > kPrunedLaneMax) {
-      radix();
-      return;
-    }
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    if ((tid & 3) == 0) P.lane_max[tid >> 2] = m;
-    if (tid == 0) {
-      P.t0 = 0u;
-      P.ncand = 0;
-    }
-    __syncthreads();
-    if (tid < quads) {
-      // place among the maxima, ties by position: unique
-      const uint32_t me = P.lane_max[tid];
-      int rank = 0;
-#pragma unroll 8
-      for (int j = 0; j < quads; ++j) {
-        const uint32_t o = P.lane_max[j];
-        rank += (o > me || (o == me && j < tid)) ? 1 : 0;
-      }
-      if (rank == k - 1) P.t0 = me;
-    }
-    __syncthreads();
-    t0 = P.t0;
+  const int quads = blockDim.x >> 2;
+  if (quads < k || quads > kPrunedLaneMax) {
+    radix();
+    return;
   }
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if ((tid & 3) == 0) P.lane_max[tid >> 2] = m;
+  if (tid == 0) {
+    P.t0 = 0u;
+    P.ncand = 0;
+  }
+  __syncthreads();
+  if (tid < quads) {
+    // place among the maxima, ties by position: unique
+    const uint32_t me = P.lane_max[tid];
+    int rank = 0;
+#pragma unroll 8
+    for (int j = 0; j < quads; ++j) {
+      const uint32_t o = P.lane_max[j];
+      rank += (o > me || (o == me && j < tid)) ? 1 : 0;
+    }
+    if (rank == k - 1) P.t0 = me;
+  }
+  __syncthreads();
+  const uint32_t t0 = P.t0;
   if (t0 == 0u) {
     radix();
     return;
@@ -324,7 +281,7 @@ FBME_DEV void block_topk_pruned(const uint32_t (&key)[KPT], uint32_t valid, GIdx
       if (pos < kPrunedCap) P.cand[pos] = make_uint2(key[i], static_cast<uint32_t>(gidx(i)));
     }
   __syncthreads();
-  const int n = P.ncand;  // >= k: k threads hold a valid key >= t0
+  const int n = P.ncand;  // >= k: k quads hold a valid key >= t0
   if (n > kPrunedCap) {
     radix();
     return;
