@@ -34,7 +34,7 @@ for _p in (str(REPO), str(REPO / "fbme-sbl_b200")):
 METRIC = "scenes/s at equal NMSE: plain vs learned+batched FBME on 1 B200; % roofline"
 UNIT = "scenes/s"
 GRID, PREFIX = (256, 256), (128, 128)
-DFT_FORMS = {0: "FP32 FFT stages (two-pass register FFT, cp.async double-buffered)",
+DFT_FORMS = {0: "FP32 FFT stages (two-pass register FFT)",
              3: "tcgen05 split-BF16 3-term, FP32 accumulation",
              6: "tcgen05 split-BF16 6-term, FP32 accumulation"}
 WORKLOAD = ("FBME-Stable replay, 256x256 grid / 128x128 prefix, 200 Rayleigh points, 15 dB, "
@@ -636,7 +636,8 @@ def physical_bytes(group: str, grid, prefix, fused_denoise: bool = False) -> int
     """Bytes one scene moves to and from HBM in one launch of a kernel group,
     intermediates included (each array read or written once).  With
     `fused_denoise` (the FP32 FFT stages) adjoint stage 2 runs the denoiser
-    in its epilogue: the group reads U instead of the lift A^H m."""
+    in its epilogue: the group reads U instead of the lift A^H m; and adjoint
+    stage 1 forms the message it transforms."""
     n1, n2 = grid
     m1, m2 = prefix
     n, m = n1 * n2, m1 * m2
@@ -645,7 +646,8 @@ def physical_bytes(group: str, grid, prefix, fused_denoise: bool = False) -> int
         # read lift 8 (fused: U), mu 8, gamma 4, v 4; write mu 8, v 4, gamma 4
         "adjoint_denoise": (t_adj + 32 * n) if fused_denoise else 40 * n,
         "message": 32 * m,                    # read y, prediction, message; write message
-        "adjoint_1": 8 * m + t_adj,           # read message; write U
+        # read message (fused: y, prediction, message; write message); write U
+        "adjoint_1": (32 if fused_denoise else 8) * m + t_adj,
         "adjoint_2": t_adj + 8 * n,           # read U; write lift
         "forward_1": 8 * n + t_fwd,           # read mu; write T
         "forward_residual": t_fwd + 16 * m,   # read T, y; write prediction
