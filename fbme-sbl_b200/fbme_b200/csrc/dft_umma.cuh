@@ -514,12 +514,12 @@ dft_stage_kernel(const __grid_constant__ StageSet<Pro, Epi, NI> set) {
 // Two complex values at base[e] (avail of them valid), zero outside.
 FBME_DEV float4 load_pair(const float2* base, long long e, int avail, bool vec) {
   if (avail >= 2) {
-    if (vec) return __ldg(reinterpret_cast<const float4*>(base + e));
-    const float2 a = __ldg(base + e), b = __ldg(base + e + 1);
+    if (vec) return *reinterpret_cast<const float4*>(base + e);
+    const float2 a = base[e], b = base[e + 1];
     return make_float4(a.x, a.y, b.x, b.y);
   }
   if (avail == 1) {
-    const float2 a = __ldg(base + e);
+    const float2 a = base[e];
     return make_float4(a.x, a.y, 0.f, 0.f);
   }
   return make_float4(0.f, 0.f, 0.f, 0.f);

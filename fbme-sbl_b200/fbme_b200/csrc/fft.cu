@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kFftThreads) fft_stage_kernel(const FftStage S
     const int row = idx / L, k = idx - row * L;
     const int r = r0 + row;
     float2 v = make_float2(0.f, 0.f);
-    if (r < S.rows && k < S.kin) v = __ldg(in + static_cast<long long>(r) * S.in_ld + k);
+    if (r < S.rows && k < S.kin) v = in[static_cast<long long>(r) * S.in_ld + k];
     if (io.ysum) acc += abs_sq(v);
     a[row * pitch + k] = v;
   }
@@ -416,7 +416,7 @@ FBME_DEV void row_values(const FftStage& st, const float2* in, int unit, int r, 
   const float2* src = in + unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
 #pragma unroll
   for (int q = 0; q < Q; ++q)
-    v[q] = live && p + P * q < st.kin ? __ldg(src + P * q) : make_float2(0.f, 0.f);
+    v[q] = live && p + P * q < st.kin ? src[P * q] : make_float2(0.f, 0.f);
 }
 // Rows r0 .. r0 + rows of a stage's input into L2.
 FBME_DEV void rows_prefetch(const FftStage& st, const float2* in, int unit, int r0, int rows) {

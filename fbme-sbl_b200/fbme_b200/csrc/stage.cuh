@@ -49,12 +49,12 @@ FBME_DEV bool vec_ok(const DftGeom& g) { return g.vec4 != 0; }
 // Two consecutive complex values at base[e] through the read-only path.
 FBME_DEV void load2c(const float2* base, long long e, int avail, bool vec, float2& a, float2& b) {
   if (avail >= 2 && vec) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(base + e));
+    const float4 v = *reinterpret_cast<const float4*>(base + e);
     a = make_float2(v.x, v.y);
     b = make_float2(v.z, v.w);
   } else {
-    a = __ldg(base + e);
-    b = avail >= 2 ? __ldg(base + e + 1) : make_float2(0.f, 0.f);
+    a = base[e];
+    b = avail >= 2 ? base[e + 1] : make_float2(0.f, 0.f);
   }
 }
 

@@ -214,7 +214,7 @@ FBME_DEV void denoise_body(Blk k, BatchShape s, DenoiseArgs a, const float2* lif
     for (long long j = first; j < n / 2; j += stride) {
       const long long e = base + 2 * j;
       const float4 m = *reinterpret_cast<const float4*>(a.mu + e);
-      const float4 l = __ldg(reinterpret_cast<const float4*>(lift + e));
+      const float4 l = *reinterpret_cast<const float4*>(lift + e);
       const float2 v = *reinterpret_cast<const float2*>(a.var + e);
       const float2 g = *reinterpret_cast<const float2*>(a.gamma + e);
       const DenoiseOut o0 = one(e, g.x, make_float2(m.x, m.y), v.x, make_float2(l.x, l.y));
