@@ -336,7 +336,8 @@ FBME_DEV EvalOut evaluate(const PolishArgs& A, PolishShared& S, const float2* d1
 
 // ||y - A_S mu||^2 by the Gram identity, FP64, on the whole block (every
 // warp returns the sum): warp w adds the columns j = w, w + 8, ... of G mu.
-FBME_DEV double residual_energy(const PolishArgs& A, PolishShared& S, const float2* d1, const float2* d2, int K,
+using GramSums = double2[kPolishWarps][kMaxPolish];
+FBME_DEV double residual_energy(const PolishArgs& A, GramSums& gm, const float2* d1, const float2* d2, int K,
                                 int my_idx, float2 my_mu, float2 my_c, float data_energy) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const BatchShape& s = A.s;
@@ -355,7 +356,7 @@ FBME_DEV double residual_energy(const PolishArgs& A, PolishShared& S, const floa
     }
   }
   __syncthreads();  // an earlier call's sums have been read
-  S.gm[w][lane] = make_double2(gr, gi);
+  gm[w][lane] = make_double2(gr, gi);
   __syncthreads();
   double cross = 0.0, quad = 0.0;
   if (lane < K) {
@@ -363,7 +364,7 @@ FBME_DEV double residual_energy(const PolishArgs& A, PolishShared& S, const floa
     gr = gi = 0.0;
 #pragma unroll
     for (int v = 0; v < kPolishWarps; ++v) {
-      const double2 t = S.gm[v][lane];
+      const double2 t = gm[v][lane];
       gr += t.x;
       gi += t.y;
     }
@@ -534,7 +535,7 @@ FBME_DEV void polish_body(const PolishArgs& A, PolishShared& S, TopkMergeShared&
     const float keep = c.polish_damping;
     const float upd_g = keep * bg + (1.0f - keep) * ng;
     const float2 bc = on ? bp[bidx] : make_float2(0.f, 0.f);
-    const double er = residual_energy(A, S, d1, d2, K, bidx, bmu, bc, data_energy);
+    const double er = residual_energy(A, S.gm, d1, d2, K, bidx, bmu, bc, data_energy);
     float dof = on ? fminf(fmaxf(1.0f - bpv / fmaxf(bg, kTinyP), 0.f), 1.f) : 0.f;
     dof = warp_sum(dof);
     float un;
@@ -777,7 +778,7 @@ using ExWidest = ExTile<4, 8, 64, 256, 512>;
 
 // Final K-space outputs, fixed-budget diagnostics, effective DOF
 // (solver.py:1989-2021, 2081-2092, 3408-3496, 2108-2126).
-FBME_DEV void polish_finish_body(const PolishArgs& A, PolishShared& S, const FbmeOutputs& out, int scene) {
+FBME_DEV void polish_finish_body(const PolishArgs& A, GramSums& gm, const FbmeOutputs& out, int scene) {
   extern __shared__ float2 dtab[];
   const int lane = threadIdx.x & 31;
   if (scene >= A.s.B) return;
@@ -826,7 +827,7 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, PolishShared& S, const Fbm
     float dofd = on ? fminf(fmaxf(1.0f - pv / ag, 0.f), 1.f) : 0.f;
     dofd = warp_sum(dofd);
     const float2 cv = on ? A.p.bp[scene * N + idx] : make_float2(0.f, 0.f);
-    const double er = residual_energy(A, S, d1, d2, K, idx, mu, cv, A.p.sc.data_energy[scene]);
+    const double er = residual_energy(A, gm, d1, d2, K, idx, mu, cv, A.p.sc.data_energy[scene]);
     float nt;
     if (c.fixed_noise > 0.f) {
       nt = nu;
@@ -852,8 +853,8 @@ FBME_DEV void polish_finish_body(const PolishArgs& A, PolishShared& S, const Fbm
 }
 __global__ void __launch_bounds__(kPolishThreads) polish_finish_kernel(PolishArgs A, FbmeOutputs out) {
   dep_sync();
-  __shared__ PolishShared S;
-  polish_finish_body(A, S, out, blockIdx.x);
+  __shared__ GramSums gm;
+  polish_finish_body(A, gm, out, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -1421,8 +1422,8 @@ __global__ void __launch_bounds__(T::threads, 2) exchange_set_kernel(const Polis
 
 __global__ void __launch_bounds__(kPolishThreads) polish_finish_set_kernel(const PolishSet set) {
   dep_sync();
-  __shared__ PolishShared S;
-  polish_finish_body(set.a[blockIdx.z], S, set.out[blockIdx.z], blockIdx.x);
+  __shared__ GramSums gm;
+  polish_finish_body(set.a[blockIdx.z], gm, set.out[blockIdx.z], blockIdx.x);
 }
 
 __global__ void __launch_bounds__(256) output_set_kernel(const PolishSet S) {
@@ -1451,8 +1452,25 @@ static cudaError_t set_exchange_smem() {
   return e;
 }
 
+// Dynamic shared memory of the kernels that hold the Dirichlet tables: plans
+// run for N1 + N2 <= kDirichletMax, whose tables (32 KB) and the block's own
+// 23 KB are more than the 48 KB a kernel may take without asking.  The
+// certificate scan holds D1 and four forms of D2 (N2 <= 512).
+constexpr int kDirichletMax = 4032;
+
+template <typename K>
+static cudaError_t set_smem(K kern, size_t bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
 cudaError_t set_polish_attributes() {
-  cudaError_t e = set_exchange_smem<ExSmall>();
+  constexpr size_t tables = kDirichletMax * sizeof(float2);
+  constexpr size_t scan = tables + 512 * (4 * 2 * sizeof(float) - sizeof(float2));
+  cudaError_t e = set_smem(polish_kernel, tables);
+  if (e == cudaSuccess) e = set_smem(polish_set_kernel, tables);
+  if (e == cudaSuccess) e = set_smem(cert_step_kernel, tables);
+  if (e == cudaSuccess) e = set_smem(cert_scan_kernel<false>, scan);
+  if (e == cudaSuccess) e = set_exchange_smem<ExSmall>();
   if (e == cudaSuccess) e = set_exchange_smem<ExMid>();
   if (e == cudaSuccess) e = set_exchange_smem<ExWide>();
   if (e == cudaSuccess) e = set_exchange_smem<ExWidest>();
