@@ -187,7 +187,7 @@ FBME_DEV void gamma_prefetch(const TileCtx& t, int row, int c0, const float* gam
   const int jb = t.col0() + (c0 >> 1);
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    p.g[i] = (r < g.rows && jb + i < g.cols) ? __ldg(gm + (jb + i) * g.out_ld) : 0.f;
+    p.g[i] = (r < g.rows && jb + i < g.cols) ? gm[(jb + i) * g.out_ld] : 0.f;
 }
 
 struct EpiGamma {
@@ -325,7 +325,7 @@ struct EpiEnergy {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       if (jb + i < g.cols) {
-        const float2 yy = __ldg(y + base + static_cast<long long>(jb + i) * g.out_ld);
+        const float2 yy = y[base + static_cast<long long>(jb + i) * g.out_ld];
         const float dr = yy.x - v[2 * i], di = yy.y - v[2 * i + 1];
         const float h = hypotf(dr, di);
         acc += static_cast<double>(h * h);

@@ -44,8 +44,9 @@ static inline int sm_count() {
 // No kernel allows the next one's launch before its own end
 // (griddepcontrol.launch_dependents): the waiting blocks then settle beside
 // the running ones, and the same replays took 204, 349, 234 and 3199 us.
-// What the predecessor has written is read by plain loads: __ldg marks it as
-// constant for the kernel, which may start before the predecessor ends.
+// What the chain writes is read by plain loads: __ldg marks it as constant for
+// the kernel, which may start before its predecessor ends.  Only tables and
+// masks laid out before a replay are read that way.
 FBME_DEV void dep_sync() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(kFftThreads) fft_stage_kernel(const FftStage S
     if (io.mode == 1) {
       acc += abs_sq(v);
     } else if (io.mode == 2 && (!io.mask || io.mask[o])) {
-      const float2 yy = __ldg(ys + o);
+      const float2 yy = ys[o];
       const float dr = yy.x - v.x, di = yy.y - v.y;
       acc += dr * dr + di * di;
     }
@@ -453,9 +453,9 @@ FBME_DEV void message_rows(const FftStage& st, const MessageArgs& ms, int unit, 
       y[i] = pd[i] = m[i] = make_float2(0.f, 0.f);
       obs[i] = true;
       if (in[i]) {
-        y[i] = __ldg(ms.y + e0 + k);
-        pd[i] = __ldg(ms.pred + e0 + k);
-        m[i] = __ldg(ms.in + e0 + k);
+        y[i] = ms.y[e0 + k];
+        pd[i] = ms.pred[e0 + k];
+        m[i] = ms.in[e0 + k];
         if (mask) obs[i] = __ldg(mask + k) != 0;
       }
     }
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
             const int ii = g * CH + i;
             const long long o = o0 + ii * step;
             if (c0 + P * ii < st.cols && (!io.mask || io.mask[o])) {
-              yv[i] = __ldg(io.y + base + o);
+              yv[i] = io.y[base + o];
               obs |= 1u << i;
             }
           }
@@ -849,7 +849,7 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_set
             const int ii = g * CH + i;
             const long long o = o0 + ii * step;
             if (c0 + P * ii < st.cols && (!io.mask || io.mask[o])) {
-              yv[i] = __ldg(io.y + base + o);
+              yv[i] = io.y[base + o];
               obs |= 1u << i;
             }
           }

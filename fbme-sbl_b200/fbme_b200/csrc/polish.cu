@@ -949,7 +949,7 @@ FBME_DEV CertBest cert_scan(const PolishArgs& A, CertShared& S, int K, float nu,
     const int j1 = static_cast<int>(p / ppr), j2 = 2 * static_cast<int>(p - static_cast<long long>(j1) * ppr);
     const int j = j1 * n2 + j2;
     const bool two = j2 + 1 < n2;
-    const float2 b0 = __ldg(bp + j), b1 = two ? __ldg(bp + j + 1) : make_float2(0.f, 0.f);
+    const float2 b0 = bp[j], b1 = two ? bp[j + 1] : make_float2(0.f, 0.f);
     float2 qx = make_float2(-b0.x, -b1.x), qy = make_float2(-b0.y, -b1.y);  // minus q of the pair
     unsigned act = 0u;
     float2 vx[kMaxPolish], vy[kMaxPolish];
@@ -1504,7 +1504,7 @@ __global__ void __launch_bounds__(256) exchange_masked_kernel(PolishArgs A) {
   for (long long n = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; n < N;
        n += static_cast<long long>(gridDim.x) * blockDim.x) {
     const int n1 = static_cast<int>(n / s.n2), n2 = static_cast<int>(n % s.n2);
-    float2 r = __ldg(bp + n);
+    float2 r = bp[n];
     bool act = false;
     for (int k = 0; k < K; ++k) {
       act |= atom[k] == n;

@@ -77,7 +77,7 @@ struct EpiPredict {
     const int jb = t.col0() + (c0 >> 1);
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      p.y[i] = (r < g.rows && jb + i < g.cols) ? __ldg(ys + (jb + i) * g.out_ld + r)
+      p.y[i] = (r < g.rows && jb + i < g.cols) ? ys[(jb + i) * g.out_ld + r]
                                                : make_float2(0.f, 0.f);
   }
   FBME_DEV void consume(const TileCtx& t, int row, int c0, const float* v, const Pre& pre) {
@@ -171,7 +171,7 @@ FBME_DEV void gamma0_body(Blk k, BatchShape s, DevConfig c, Scalars sc, const fl
   if ((n & 1) == 0) {  // two coefficients per step, 16- and 8-byte accesses
     for (long long j = first; j < n / 2; j += stride) {
       const long long e = scene * n + 2 * j;
-      const float4 b = __ldg(reinterpret_cast<const float4*>(bp + e));
+      const float4 b = *reinterpret_cast<const float4*>(bp + e);
       const float g0 = prior(make_float2(b.x, b.y));
       const float g1 = prior(make_float2(b.z, b.w));
       *reinterpret_cast<float2*>(gamma + e) = make_float2(g0, g1);
@@ -263,9 +263,9 @@ FBME_DEV void message_body(Blk k, BatchShape s, const float2* y, const float2* p
   if ((m & 1) == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0) {
     for (long long j = first; j < m / 2; j += stride) {
       const long long e = scene * m + 2 * j;
-      const float4 a = __ldg(reinterpret_cast<const float4*>(y + e));
-      const float4 p = __ldg(reinterpret_cast<const float4*>(pred + e));
-      const float4 q = __ldg(reinterpret_cast<const float4*>(msg_in + e));
+      const float4 a = *reinterpret_cast<const float4*>(y + e);
+      const float4 p = *reinterpret_cast<const float4*>(pred + e);
+      const float4 q = *reinterpret_cast<const float4*>(msg_in + e);
       float2 o0 = step(make_float2(a.x, a.y), make_float2(p.x, p.y), make_float2(q.x, q.y));
       float2 o1 = step(make_float2(a.z, a.w), make_float2(p.z, p.w), make_float2(q.z, q.w));
       if (mask) {
@@ -325,7 +325,7 @@ FBME_DEV void sweep1_body(Blk k, BatchShape s, DevConfig c, Scalars sc, DenoiseA
     for (long long j = first; j < n / 2; j += stride) {
       const long long e = scene * n + 2 * j;
       const float2 g = *reinterpret_cast<const float2*>(a.gamma + e);
-      const float4 b = __ldg(reinterpret_cast<const float4*>(bp + e));
+      const float4 b = *reinterpret_cast<const float4*>(bp + e);
       const DenoiseOut o0 = one(g.x, make_float2(b.x, b.y));
       const DenoiseOut o1 = one(g.y, make_float2(b.z, b.w));
       *reinterpret_cast<float4*>(a.mu + e) = make_float4(o0.mean.x, o0.mean.y, o1.mean.x, o1.mean.y);
