@@ -198,6 +198,7 @@ __device__ __forceinline__ void diag_factor(DiagShared& S, double2 (&r)[kDiagCol
     const double rq = rsqrt(d > 0.0 ? d : 2.2250738585072014e-308);
     S.L[q][lane] = lane > q ? make_double2(v.x * rq, v.y * rq) : make_double2(0.0, 0.0);
     S.rl[q] = rq;  // the same value from every lane
+    __syncwarp();  // this warp reads the column without waiting at its barrier
     diag_arrive(q);
     v = make_double2(0.0, 0.0);
     failed |= d > 0.0 ? 0 : isfinite(d) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;

@@ -228,6 +228,7 @@ FBME_DEV EvalOut evaluate(const PolishArgs& A, PolishShared& S, const float2* d1
     const float2 a = make_float2(lane == q ? piv : lane > q ? v.x * rq : 0.f, lane > q ? v.y * rq : 0.f);
     S.L[q][lane] = a;
     S.rl[q] = rq;  // the same value from every lane
+    __syncwarp();  // this warp reads the column without waiting at its barrier
     column_arrive(q);
     v = make_float2(0.f, 0.f);
     failed |= sdiag > 0.f ? 0 : isfinite(sdiag) ? FBME_STATUS_CHOLESKY : FBME_STATUS_NONFINITE;

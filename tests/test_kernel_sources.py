@@ -38,3 +38,12 @@ def test_dependent_kernels_wait_for_their_predecessor():
     for name in names:
         body = re.search(r"\b%s\([^;{]*\) \{(.*?)^\}" % name, code, re.S | re.M)
         assert body and "dep_sync();" in body.group(1), name
+
+
+@pytest.mark.parametrize("name", ["polish.cu", "dense.cu"])
+def test_posted_column_is_ordered_within_its_warp(name):
+    """The warp that posts a column of a factorisation only arrives at the
+    column's barrier, which orders nothing for its own later reads."""
+    body = re.search(r"auto post = \[&\]\(int q, .*?\n  \};", (CSRC / name).read_text(), re.S).group(0)
+    stores, arrive = body.rindex("S.rl[q] ="), re.search(r"\w+_arrive\(q\)", body).start()
+    assert "__syncwarp();" in body[stores:arrive]
