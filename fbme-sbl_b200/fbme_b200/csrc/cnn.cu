@@ -278,6 +278,17 @@ FBME_DEV void ldmatrix_x2_t(uint32_t addr, uint32_t& a0, uint32_t& a1) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(a0), "=r"(a1) : "r"(addr));
 }
 
+// Whether one of eight values, rounded to BF16 pairs w, is infinite.
+FBME_DEV bool any_infinite(const uint32_t (&w)[4]) {
+  auto mag = [](uint32_t v) {
+    v &= 0x7fff7fffu;
+    return *reinterpret_cast<const __nv_bfloat162*>(&v);
+  };
+  const __nv_bfloat162 m = __hmax2(__hmax2(mag(w[0]), mag(w[1])), __hmax2(mag(w[2]), mag(w[3])));
+  const uint32_t u = *reinterpret_cast<const uint32_t*>(&m);
+  return (u & 0xffffu) == 0x7f80u || (u >> 16) == 0x7f80u;
+}
+
 __global__ void __launch_bounds__(256, 3)
 wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask, int B, int H, int W,
              float* partial) {
@@ -353,10 +364,24 @@ wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const __nv_bfloat162 h = __float22bfloat162_rn(make_float2(v[2 * c], v[2 * c + 1]));
-          const float2 f = __bfloat1622float2(h);
-          v[2 * c] -= f.x;
-          v[2 * c + 1] -= f.y;
           w[c] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        if (p == 0 && any_infinite(w)) {
+          // values past BF16's range: the first part is cut instead of
+          // rounded, and an infinity leaves nothing for the other parts, so
+          // that sums over it are infinite and not NaN
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint32_t cut = __float_as_uint(v[c]) & 0xffff0000u;
+            w[c / 2] = c & 1 ? (w[c / 2] & 0xffffu) | cut : cut >> 16;
+            v[c] = isinf(v[c]) ? 0.f : v[c] - __uint_as_float(cut);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            v[2 * c] -= __uint_as_float(w[c] << 16);
+            v[2 * c + 1] -= __uint_as_float(w[c] & 0xffff0000u);
+          }
         }
         gs[p][tid + 256 * j] = make_uint4(w[0], w[1], w[2], w[3]);
       }

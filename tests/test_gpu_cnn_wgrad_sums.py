@@ -113,3 +113,20 @@ def test_sums_are_unbiased():
         acc = np.where(up > s, np.nextafter(up, np.float32(0)), up)
     exact = runs[:28].astype(np.float64).sum(0)
     assert float(np.mean(exact - acc) / np.mean(exact)) > 1e-7
+
+
+@pytest.mark.gpu
+def test_infinite_gradient_gives_infinite_sums():
+    need_gpu()
+
+    def target(out, rng):
+        t = torch.zeros_like(out)
+        t[0, 37] = float("inf")
+        return t
+
+    for x, g, mask, dw, db in _train(1, (16, 32), target):
+        with np.errstate(invalid="ignore"):
+            ref = _sums(x, g, mask)
+        for a, b in zip((dw, db), ref):
+            assert np.array_equal(np.isnan(a), np.isnan(b))
+            assert np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))
