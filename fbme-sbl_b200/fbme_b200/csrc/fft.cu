@@ -394,13 +394,27 @@ __host__ __device__ constexpr int fast_row_area(int L) {
   return a;
 }
 // one buffer of ROWS rows (the exchange, then in place the output staging)
-__host__ __device__ constexpr size_t fast_smem_bytes(int L) {
+__host__ __device__ constexpr size_t fast_buf_bytes(int L) {
   return static_cast<size_t>(kFftThreads / fast_threads_per_row(L)) * fast_row_area(L) * sizeof(float2);
+}
+// Two buffers, the next tile's rows copied into one while the other is
+// transformed, for the denoiser (epi 2) where two blocks' four buffers take
+// at most 164 KB of the SM: its two blocks are too few to hide the latency of
+// rows loaded straight into registers.  That is L = 64, 96 and 256 (B200, 16.8 M
+// coefficients a sweep, one buffer -> two: 146 -> 146, 154 -> 154, 139 -> 134 us;
+// 512 scenes of 256^2 264 -> 256).  At the other lengths the second buffer
+// costs a block or the L1: 128, 192, 384, 48 and 32 take 134, 157, 172, 152
+// and 146 us with one buffer, 134, 206, 193, 233 and 160 with two.
+__host__ __device__ constexpr bool fast_two_buffers(int L, int epi) {
+  return epi == 2 && 4 * fast_buf_bytes(L) <= 164 * 1024;
+}
+__host__ __device__ constexpr size_t fast_smem_bytes(int L, int epi) {
+  return (fast_two_buffers(L, epi) ? 2 : 1) * fast_buf_bytes(L);
 }
 // Blocks per SM: three where a row's Q values leave room for 80 registers a
 // thread, else two of up to 128 registers; two for the denoiser, whose
-// operands want the registers (512 scenes of 256^2: 263 us a sweep, 277 with
-// three blocks).
+// operands want the registers (512 scenes of 256^2, one buffer: 263 us a
+// sweep, 277 with three blocks).
 __host__ __device__ constexpr int fast_blocks(int L, int epi) {
   return epi != 2 && L / fast_threads_per_row(L) <= 16 ? 3 : 2;
 }
@@ -417,6 +431,26 @@ FBME_DEV void row_values(const FftStage& st, const float2* in, int unit, int r, 
 #pragma unroll
   for (int q = 0; q < Q; ++q)
     v[q] = live && p + P * q < st.kin ? src[P * q] : make_float2(0.f, 0.f);
+}
+FBME_DEV void row_copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// All of this thread's copies but the last group's have landed.
+FBME_DEV void row_copy_wait() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+// The same values of tile t's row, asynchronously, into the places of the row
+// that the thread reads them from (the rest is zero and is not copied); one
+// commit group.
+template <int L>
+FBME_DEV void row_copy(const FftStage& st, const float2* in, int t, float2* buf, int lr, int p) {
+  constexpr int P = fast_threads_per_row(L), Q = L / P, ROWS = kFftThreads / P;
+  const int unit = t / st.tiles, r = (t - unit * st.tiles) * ROWS + lr;
+  if (r < st.rows) {
+    const float2* src = in + unit * st.in_stride + static_cast<long long>(r) * st.in_ld + p;
+    float2* dst = buf + lr * fast_row_area(L) + p;
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+      if (p + P * q < st.kin)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst + P * q)), "l"(src + P * q) : "memory");
+  }
+  row_copy_commit();
 }
 // Rows r0 .. r0 + rows of a stage's input into L2.
 FBME_DEV void rows_prefetch(const FftStage& st, const float2* in, int unit, int r0, int rows) {
@@ -471,7 +505,8 @@ FBME_DEV void message_rows(const FftStage& st, const MessageArgs& ms, int unit, 
 // Persistent: CTA b takes tiles b, b + gridDim.x, ... (tile t = unit x
 // tiles + row tile); the rows (and epilogue operands) of its next tile are
 // prefetched into L2 while the current one is transformed.  HBM and the
-// latency of the loads bound it.  The rows go straight to registers: copied
+// latency of the loads bound it.  The rows go straight to registers but for
+// the denoiser's (fast_two_buffers): copied
 // through a second shared-memory buffer (cp.async) they took a third of the
 // shared-memory traffic and half of the SM's shared memory, which left one
 // block an SM at L = 192 and 512 and two at 256, and little L1.  Forward
@@ -489,8 +524,18 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
   extern __shared__ float2 fsm[];
   const int lr = threadIdx.x / P, p = threadIdx.x % P;
   const int total = st.tiles * st.units;
+  constexpr bool TWO = fast_two_buffers(L, EPI);
   int t = blockIdx.x;
-  for (; t < total; t += gridDim.x) {
+  if constexpr (TWO)
+    if (t < total) row_copy<L>(st, io.in, t, fsm, lr, p);
+  for (int it = 0; t < total; ++it, t += gridDim.x) {
+    float2* buf = TWO ? fsm + (it & 1) * ROWS * A : fsm;
+    if constexpr (TWO) {  // ahead of the prefetches below; after them the stage takes 265 us, not 256
+      if (t + static_cast<int>(gridDim.x) < total)
+        row_copy<L>(st, io.in, t + gridDim.x, fsm + ((it + 1) & 1) * ROWS * A, lr, p);
+      else
+        row_copy_commit();  // an empty group, so that the wait counts the same
+    }
     if constexpr (EPI == 1 || EPI == 2) {
       // the next tile's epilogue operands (observations; prior, mean and
       // variance) into L2, one line per output column and array, so their
@@ -511,7 +556,7 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
         }
       }
     }
-    if (t + static_cast<int>(gridDim.x) < total) {
+    if (!TWO && t + static_cast<int>(gridDim.x) < total) {
       const int tn = t + gridDim.x, un = tn / st.tiles, rn = (tn - un * st.tiles) * ROWS;
       if constexpr (EPI == 3) {
         rows_prefetch(st, io.ms.y, un, rn, ROWS);
@@ -523,12 +568,18 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
     }
     const int unit = t / st.tiles, tile = t - unit * st.tiles;
     const int r0 = tile * ROWS;
-    float2* ya = fsm + lr * A;
+    float2* ya = buf + lr * A;
 
     // pass 1: DFT-Q of x[p + P q] in registers
     float2 v[Q];
     if constexpr (EPI == 3) {
       message_rows<L>(st, io.ms, unit, r0 + lr, p, v);
+    } else if constexpr (TWO) {
+      row_copy_wait();  // a thread reads only what it copied
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        v[q] = r0 + lr < st.rows && p + P * q < st.kin ? ya[p + P * q] : make_float2(0.f, 0.f);
+      __syncwarp();  // the row's values are read before the exchange overwrites them
     } else {
       row_values<L>(st, io.in, unit, r0 + lr, p, v);
     }
@@ -595,7 +646,7 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
     const long long base = unit * st.out_stride;
     const long long o0 = static_cast<long long>(c0) * st.out_ld + rr;
     const long long step = static_cast<long long>(P) * st.out_ld;
-    const float2* sp = fsm + row * A + row;
+    const float2* sp = buf + row * A + row;
     if constexpr (EPI == 0 || EPI == 3) {
       __syncthreads();
       float acc = 0.f;
@@ -700,7 +751,7 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_ker
         *part_slot(io.part, unit, tile, 1 * kPartWarps + (threadIdx.x >> 5)) = w1;
       }
     }
-    __syncthreads();  // the next tile's exchange overwrites the staging
+    __syncthreads();  // the next tile's exchange, or the copies after it, overwrite the staging
   }
 }
 
@@ -935,28 +986,28 @@ template <int L, int S, int EPI>
 void launch_fast_as(const FftStage& S_, const FftIo& io, cudaStream_t st) {
   auto kern = fft_fast_kernel<L, S, EPI>;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFftThreads, fast_smem_bytes(L)) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFftThreads, fast_smem_bytes(L, EPI)) !=
           cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   const long long total = static_cast<long long>(S_.tiles) * S_.units;
   const long long cap = static_cast<long long>(sm_count()) * per_sm;
   const int grid = static_cast<int>(total < cap ? total : cap);
-  if (grid > 0) launch_dep(kern, grid, kFftThreads, fast_smem_bytes(L), st, S_, io);
+  if (grid > 0) launch_dep(kern, grid, kFftThreads, fast_smem_bytes(L, EPI), st, S_, io);
 }
 
 template <int L, int S, int EPI>
 void launch_fast_set_as(const FftSet<kFftSetMax>& set, cudaStream_t st) {
   auto kern = fft_fast_set_kernel<L, S, EPI, kFftSetMax>;
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFftThreads, fast_smem_bytes(L)) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFftThreads, fast_buf_bytes(L)) !=
           cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   const long long total = set.tile0[set.n];
   const long long cap = static_cast<long long>(sm_count()) * per_sm;
   const int grid = static_cast<int>(total < cap ? total : cap);
-  if (grid > 0) kern<<<grid, kFftThreads, fast_smem_bytes(L), st>>>(set);
+  if (grid > 0) kern<<<grid, kFftThreads, fast_buf_bytes(L), st>>>(set);
 }
 
 // Forward stages store or take the residual; adjoint stages store or run
@@ -990,11 +1041,11 @@ cudaError_t smem_attr(K kern, int bytes) {
 }
 template <int L>
 cudaError_t set_fast_attr() {
-  const int bytes = static_cast<int>(fast_smem_bytes(L));
+  const int bytes = static_cast<int>(fast_smem_bytes(L, 0)), bytes2 = static_cast<int>(fast_smem_bytes(L, 2));
   cudaError_t e = smem_attr(fft_fast_kernel<L, -1, 0>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, -1, 1>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 0>, bytes);
-  if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 2>, bytes);
+  if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 2>, bytes2);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 3>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 0, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 1, kFftSetMax>, bytes);
