@@ -278,17 +278,6 @@ FBME_DEV void ldmatrix_x2_t(uint32_t addr, uint32_t& a0, uint32_t& a1) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(a0), "=r"(a1) : "r"(addr));
 }
 
-// Whether one of eight values, rounded to BF16 pairs w, is infinite.
-FBME_DEV bool any_infinite(const uint32_t (&w)[4]) {
-  auto mag = [](uint32_t v) {
-    v &= 0x7fff7fffu;
-    return *reinterpret_cast<const __nv_bfloat162*>(&v);
-  };
-  const __nv_bfloat162 m = __hmax2(__hmax2(mag(w[0]), mag(w[1])), __hmax2(mag(w[2]), mag(w[3])));
-  const uint32_t u = *reinterpret_cast<const uint32_t*>(&m);
-  return (u & 0xffffu) == 0x7f80u || (u >> 16) == 0x7f80u;
-}
-
 __global__ void __launch_bounds__(256, 3)
 wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask, int B, int H, int W,
              float* partial) {
@@ -364,24 +353,10 @@ wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const __nv_bfloat162 h = __float22bfloat162_rn(make_float2(v[2 * c], v[2 * c + 1]));
+          const float2 f = __bfloat1622float2(h);
+          v[2 * c] -= f.x;
+          v[2 * c + 1] -= f.y;
           w[c] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        if (p == 0 && any_infinite(w)) {
-          // values past BF16's range: the first part is cut instead of
-          // rounded, and an infinity leaves nothing for the other parts, so
-          // that sums over it are infinite and not NaN
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint32_t cut = __float_as_uint(v[c]) & 0xffff0000u;
-            w[c / 2] = c & 1 ? (w[c / 2] & 0xffffu) | cut : cut >> 16;
-            v[c] = isinf(v[c]) ? 0.f : v[c] - __uint_as_float(cut);
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            v[2 * c] -= __uint_as_float(w[c] << 16);
-            v[2 * c + 1] -= __uint_as_float(w[c] & 0xffff0000u);
-          }
         }
         gs[p][tid + 256 * j] = make_uint4(w[0], w[1], w[2], w[3]);
       }
@@ -407,6 +382,48 @@ wgrad_kernel(const __nv_bfloat16* x, const float* gin, const __nv_bfloat16* mask
         mma_bf16_16816(hi, a[0], a[1], a[2], a[3], bh[0], bh[1]);
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[m][j] += hi[j] + lo[j];
+      }
+    }
+  }
+  // An infinite gradient's lower parts are inf - inf, and an infinite
+  // activation's products with a zero part, or with the zero gradient of a
+  // pixel outside the image, are inf x 0: NaN where the sum of products is
+  // infinite.  A warp whose sums are not finite forms them again, product by
+  // product.
+  bool odd = false;
+#pragma unroll
+  for (int m = 0; m < 5; ++m)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) odd |= !isfinite(acc[m][j]);
+  if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[m][j] = 0.f;
+#pragma unroll 1
+    for (tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+      const int rem = static_cast<int>(tile % (tx_n * ty_n)), x0 = (rem % tx_n) * kGtW;
+      const int y1 = (rem / tx_n) * kGtH + 2 * warp;
+      const long long img = tile / (tx_n * ty_n) * H * W;
+#pragma unroll 1
+      for (int i = 0; i < 2 * kGtW; ++i) {
+        const int gy = y1 + i / kGtW, gx = x0 + i % kGtW;
+        if (gy >= H || gx >= W) continue;
+        float gv[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const long long e = (img + static_cast<long long>(gy) * W + gx) * kHid + 2 * (lane & 3) + c;
+          gv[c] = mask && !(__bfloat162float(mask[e]) > 0.f) ? 0.f : gin[e];
+        }
+#pragma unroll
+        for (int tap = 0; tap < 10; ++tap) {
+          const int sy = gy - 1 + tap / 3, sx = gx - 1 + tap % 3;
+          float xv = tap < 9 ? 0.f : 1.f;
+          if (tap < 9 && sy >= 0 && sy < H && sx >= 0 && sx < W)
+            xv = __bfloat162float(x[(img + static_cast<long long>(sy) * W + sx) * kHid + (lane >> 2)]);
+#pragma unroll
+          for (int c = 0; c < 2; ++c) acc[tap / 2][2 * (tap & 1) + c] = fmaf(xv, gv[c], acc[tap / 2][2 * (tap & 1) + c]);
+        }
       }
     }
   }
