@@ -49,6 +49,8 @@ static inline int sm_count() {
 // masks laid out before a replay are read that way.
 FBME_DEV void dep_sync() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A refused launch stays the runtime's last error, which the callers query
+// once after their chain, as after plain launches.
 template <typename... P, typename... A>
 static inline void launch_dep(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute at{};

@@ -569,8 +569,7 @@ struct EpiStoreT {
 //   [unit][c / 128][r / 32][part][c % 128 rows x 128 B].
 // A warp's 32 lanes hold 32 consecutive r, one 128-byte operand row per
 // column and part: fully coalesced stores.  Rows r past this stage's rows
-// carry exact zeros (their inputs read as zero), which is the next stage's
-// K padding; columns past `cols` are never written, and the next stage's
+// are written as zeros, the next stage's K padding; columns past `cols` are never written, and the next stage's
 // rows that read them are discarded by its epilogue.
 struct EpiSplitT {
   using Pre = NoPre;

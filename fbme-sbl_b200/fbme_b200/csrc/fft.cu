@@ -380,6 +380,14 @@ __host__ __device__ constexpr int fast_threads_per_row(int L) {
   return L == 512 || L == 384 || L == 256 ? 16 : L == 192 || L == 128 || L == 96 || L == 64 ? 8
                                                  : L == 48 || L == 32 ? 4 : 0;
 }
+// Whether the denoiser epilogue and the message update formed in the load are
+// built for L.  They pay where a row's values leave their operands registers;
+// at L = 512 (32 values a thread) the elementwise kernels at full occupancy are
+// faster (32 scenes of 512^2 / 256^2: both fused 1.25 ms a replay, by
+// themselves 1.17 ms).  Message fused against by itself: 512 scenes of 256^2 /
+// 128^2 3.13 and 3.17 ms; 256 x 384 / 128 x 192 1721 and 1721 us for 170
+// scenes, 221 and 224 for 4, 212 and 216 for one.
+__host__ __device__ constexpr bool fast_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
 // Complex values of one row's area: at least Q (P + 2) for the exchange
 // (column k1 at k1 (P + 2): 16-byte aligned for the pass-2 vector reads,
 // whose 8-lane phases then fall on distinct banks) and L + ROWS for the
@@ -774,6 +782,8 @@ __global__ void __launch_bounds__(kFftThreads, fast_blocks(L, EPI)) fft_fast_set
     const FftStage& st = set.st[item];
     const FftIo& io = set.io[item];
     const int tn = t + gridDim.x;
+    // not the message update's rows: three arrays to walk for a few tiles a
+    // block (16 and 64 uneven scenes 443 and 911 us without, 445 and 912 with)
     if (EPI != 3 && tn < total) {
       const int in_ = fft_set_item(set, tn);
       const FftStage& sn = set.st[in_];
@@ -1018,9 +1028,11 @@ void launch_fast(const FftStage& S, const FftIo& io, int sign, cudaStream_t st) 
     if (io.mode == 2) launch_fast_as<L, -1, 1>(S, io, st);
     else launch_fast_as<L, -1, 0>(S, io, st);
   } else {
-    if (io.mode == 3) launch_fast_as<L, 1, 2>(S, io, st);
-    else if (io.mode == 4) launch_fast_as<L, 1, 3>(S, io, st);
-    else launch_fast_as<L, 1, 0>(S, io, st);
+    if constexpr (fast_fused(L)) {
+      if (io.mode == 3) return launch_fast_as<L, 1, 2>(S, io, st);
+      if (io.mode == 4) return launch_fast_as<L, 1, 3>(S, io, st);
+    }
+    launch_fast_as<L, 1, 0>(S, io, st);
   }
 }
 template <int L>
@@ -1029,9 +1041,11 @@ void launch_fast_set(const FftSet<kFftSetMax>& set, int sign, int mode, cudaStre
     if (mode == 2) launch_fast_set_as<L, -1, 1>(set, st);
     else launch_fast_set_as<L, -1, 0>(set, st);
   } else {
-    if (mode == 3) launch_fast_set_as<L, 1, 2>(set, st);
-    else if (mode == 4) launch_fast_set_as<L, 1, 3>(set, st);
-    else launch_fast_set_as<L, 1, 0>(set, st);
+    if constexpr (fast_fused(L)) {
+      if (mode == 3) return launch_fast_set_as<L, 1, 2>(set, st);
+      if (mode == 4) return launch_fast_set_as<L, 1, 3>(set, st);
+    }
+    launch_fast_set_as<L, 1, 0>(set, st);
   }
 }
 
@@ -1045,13 +1059,15 @@ cudaError_t set_fast_attr() {
   cudaError_t e = smem_attr(fft_fast_kernel<L, -1, 0>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, -1, 1>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 0>, bytes);
-  if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 2>, bytes2);
-  if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 3>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 0, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, -1, 1, kFftSetMax>, bytes);
   if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 0, kFftSetMax>, bytes);
-  if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 2, kFftSetMax>, bytes);
-  if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 3, kFftSetMax>, bytes);
+  if constexpr (fast_fused(L)) {
+    if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 2>, bytes2);
+    if (e == cudaSuccess) e = smem_attr(fft_fast_kernel<L, 1, 3>, bytes);
+    if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 2, kFftSetMax>, bytes);
+    if (e == cudaSuccess) e = smem_attr(fft_fast_set_kernel<L, 1, 3, kFftSetMax>, bytes);
+  }
   return e;
 }
 
@@ -1122,13 +1138,8 @@ cudaError_t set_fft_attributes() {
 
 // One FFT stage of `units` transforms (the geometry of the GEMM stage `g`,
 // whose contracted length K is padded to the transform length L).
-// The fused denoiser epilogue and the message update formed in the load pay
-// where a row's values leave their operands registers; at L = 512 (32 values
-// a thread) the elementwise kernels at full occupancy are faster (32 scenes
-// of 512^2 / 256^2: both fused 1.25 ms a replay, by themselves 1.17 ms; 512
-// scenes of 256^2 / 128^2: message fused 3.13 ms, by itself 3.17 ms).
-int fft_message_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
-int fft_denoise_fused(int L) { return fast_threads_per_row(L) != 0 && L < 512; }
+int fft_message_fused(int L) { return fast_fused(L); }
+int fft_denoise_fused(int L) { return fast_fused(L); }
 
 static FftStage fft_stage_of(const DftGeom& g, int L, int sign, const float2* tw) {
   FftStage S;

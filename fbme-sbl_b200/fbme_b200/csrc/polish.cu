@@ -100,8 +100,9 @@ FBME_DEV void load_dirichlet(const PolishArgs& A, float2* d1, float2* d2) {
 // there to shorten a step, not to add throughput: four entries of a row and
 // of the inverse a thread instead of up to 32 each.  Measured (B200, K = 32):
 // the three polish launches of one Stable scene 138 us in a single warp, 60 us
-// so; of a 512-scene replay 157 -> 128 us.  Every entry keeps its operations
-// and their order.
+// so; of a 512-scene replay 157 -> 128 us.  Every entry of the factorisation
+// keeps its operations and their order; the FP64 sums of the residual energy
+// are added per warp first (residual_energy).
 constexpr int kPolishWarps = 8;
 constexpr int kPolishThreads = 32 * kPolishWarps;
 constexpr int kPolishCols = kMaxPolish / kPolishWarps;  // columns of a row per thread
@@ -115,7 +116,6 @@ struct PolishShared {
   double ev[3][kMaxPolish];              // logarithms of the evidence
   double log_nu;
   double2 gm[kPolishWarps][kMaxPolish];  // G mu, one partial sum per warp
-  float trace[kMaxEval];
   int status;
 };
 
@@ -861,9 +861,10 @@ __global__ void __launch_bounds__(kPolishThreads) polish_finish_kernel(PolishArg
 // ---------------------------------------------------------------------------
 // Global certificate and support repairs (solver.py:3522-3588 inactive
 // certificate, 3219-3317 active certificate, 4511-4628 repairs, 4851-4870
-// and 5388-5460 final diagnostics).  One CTA per scene: warp 0 runs the
-// K-dimensional algebra (evaluate(), as in the polish), every thread scores
-// grid atoms.  For atom j, with g_i = a_j^H a_i from the Dirichlet tables,
+// and 5388-5460 final diagnostics).  A block per scene runs the K-dimensional
+// algebra (evaluate(), as in the polish) between grid scans on many blocks,
+// whose threads score a pair of atoms at a time.  For atom j, with
+// g_i = a_j^H a_i from the Dirichlet tables,
 //   q_j   = (A^H y)[j] - sum_i g_i mu_i             (nu a_j^H C^-1 y)
 //   v     = L^-1 D^-1 conj(g)                       (forward substitution)
 //   s_j   = M / nu - ||v||^2 / nu^2                 (a_j^H C^-1 a_j)

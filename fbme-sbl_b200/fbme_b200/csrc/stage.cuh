@@ -46,7 +46,8 @@ FBME_DEV double unit_sum(const double* part, int unit, int sum, int tiles, int w
 
 FBME_DEV bool vec_ok(const DftGeom& g) { return g.vec4 != 0; }
 
-// Two consecutive complex values at base[e] through the read-only path.
+// Two consecutive complex values at base[e], by plain loads: the chain's own
+// kernels write what the dependent stages read here.
 FBME_DEV void load2c(const float2* base, long long e, int avail, bool vec, float2& a, float2& b) {
   if (avail >= 2 && vec) {
     const float4 v = *reinterpret_cast<const float4*>(base + e);

@@ -2,10 +2,10 @@
 // registers, with the index-order tie break of a stable descending sort.
 //
 // Many CTAs per scene each reduce a slice of the grid to a sorted list of k
-// candidates (block_topk, block_topk_pruned), then one CTA per scene merges
-// the lists (block_topk_merge): the result is exactly the k largest keys of
-// the scene (largest first, ties by lower index), which is what torch.topk
-// returns at solver.py:1931/4410.
+// candidates (block_topk_pruned), then one CTA per scene merges the lists
+// (block_topk_merge): the result is exactly the k largest keys of the scene
+// (largest first, ties by lower index), which is what torch.topk returns at
+// solver.py:1931/4410.
 #pragma once
 
 #include "common.cuh"
@@ -202,13 +202,6 @@ FBME_DEV void block_topk_fn(const uint32_t (&key)[KPT], Valid valid, GIdx gidx, 
   __syncthreads();
 }
 
-template <int KPT, bool AGG = false>
-FBME_DEV void block_topk(const uint32_t (&key)[KPT], const int (&gidx)[KPT], const bool (&valid)[KPT],
-                         int k, TopkShared& S, uint32_t* out_key, int* out_idx) {
-  block_topk_fn<KPT, AGG>(
-      key, [&](int i) { return valid[i]; }, [&](int i) { return gidx[i]; }, k, S, out_key, out_idx);
-}
-
 constexpr int kPrunedCap = 256;
 constexpr int kPrunedLaneMax = 256;  // quad maxima ranked for the bound
 
@@ -220,7 +213,7 @@ struct TopkPrunedShared {
   uint2 cand[kPrunedCap];  // (key, index)
 };
 
-// Block-wide top-k (k <= 32) with the result of block_topk, for key sets
+// Block-wide top-k (k <= 32) with the result of block_topk_fn, for key sets
 // whose k best are few among many.  The k-th largest maximum T0 of the quads
 // of lanes is a lower bound on the block's k-th key (k different quads hold a
 // key >= T0), so the block's top k are among the keys >= T0, typically little
