@@ -233,6 +233,7 @@ SIGNATURES = {
                                  c_void_p]),
     "fbme_topk_static_error": (c_char_p, []),
     "fbme_cg_workspace_bytes": (c_size_t, [POINTER(FbmeShape), c_int32, POINTER(FbmeCgConfig)]),
+    "fbme_cg_workspace_bytes_min": (c_size_t, [POINTER(FbmeShape), c_int32, POINTER(FbmeCgConfig)]),
     "fbme_cg_create": (c_int, [POINTER(FbmeShape), c_int32, POINTER(FbmeCgConfig), c_void_p,
                                c_size_t, c_void_p, POINTER(c_void_p)]),
     "fbme_cg_solve": (c_int, [c_void_p, c_void_p, c_void_p, POINTER(FbmeCgOutputs),

@@ -182,7 +182,12 @@ class CGEngine:
             msg = nat.last_error()
             nat.check(nat.FBME_ERR_UNSUPPORTED if ("not built" in msg or "more than" in msg)
                       else nat.FBME_ERR_INVALID, "fbme_cg_workspace_bytes")
-        self.workspace = torch.empty(int(nbytes) + 256, dtype=torch.uint8, device=device)
+        try:
+            self.workspace = torch.empty(int(nbytes) + 256, dtype=torch.uint8, device=device)
+        except torch.OutOfMemoryError:  # the plan without the split intermediates' padding
+            nbytes = self.lib.fbme_cg_workspace_bytes_min(ctypes.byref(self._shape), self.batch,
+                                                          ctypes.byref(self.native_cfg))
+            self.workspace = torch.empty(int(nbytes) + 256, dtype=torch.uint8, device=device)
         self._ws_ptr = (self.workspace.data_ptr() + 255) & ~255
         self._plan = ctypes.c_void_p()
         with torch.cuda.device(device):

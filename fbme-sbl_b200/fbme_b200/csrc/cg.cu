@@ -1094,6 +1094,7 @@ cudaError_t set_cg_attributes() {
 // ---------------------------------------------------------------------------
 struct CgSettings {
   int terms;            // split-BF16 products of the DFT stages (3 or 6)
+  bool split;           // matvec intermediates in split operand form (CgBuffers::layout)
   int rank;             // preconditioner rank K
   int fixed_iterations; // > 0: static PCG schedule with best-checkpoint tracking
   int max_cg_iter;
@@ -1128,8 +1129,8 @@ struct CgBuffers {
   int* any_active;
   float* hist;
   float *gsum, *dof, *change;
-  static size_t layout(const BatchShape& s, int pmax, int rank, int max_iter, size_t* offs);
-  void bind(const BatchShape& s, int pmax, int rank, int max_iter, uint8_t* w);
+  static size_t layout(const BatchShape& s, int pmax, int rank, int max_iter, bool split, size_t* offs);
+  void bind(const BatchShape& s, int pmax, int rank, int max_iter, bool split, uint8_t* w);
 };
 
 class CgEngine {
@@ -1173,7 +1174,9 @@ __global__ void cg_rank0_kernel(int B, const float* noise, const float* gsum, fl
   if (b < B) bg[b] = noise[b] + gsum[b];
 }
 
-size_t CgBuffers::layout(const BatchShape& s, int pmax, int rank, int max_iter, size_t* offs) {
+// split: room for the matvec's intermediates as operands of the next stage,
+// whose rows and columns are padded to the tile.
+size_t CgBuffers::layout(const BatchShape& s, int pmax, int rank, int max_iter, bool split, size_t* offs) {
   size_t off = 0;
   int i = 0;
   auto take = [&](size_t bytes) {
@@ -1193,10 +1196,10 @@ size_t CgBuffers::layout(const BatchShape& s, int pmax, int rank, int max_iter, 
   take(B * pmax * M * sizeof(float2) + 16);  // 6 pz
   take(B * pmax * N * sizeof(float2) + 16);  // 7 lp
   for (int v = 0; v < 8; ++v) take(U * M * sizeof(float2));  // 8..15 rhs x r z q d0 d1 best
-  // intermediates, FP32 or as the next stage's split operand (tile-padded)
-  auto mid = [](size_t rows, size_t k) {
-    return std::max(rows * k * sizeof(float2),
-                    static_cast<size_t>(split_unit_bytes(static_cast<int>(rows), static_cast<int>(k))));
+  auto mid = [&](size_t rows, size_t k) {
+    const size_t plain = rows * k * sizeof(float2);
+    return split ? std::max(plain, static_cast<size_t>(split_unit_bytes(static_cast<int>(rows), static_cast<int>(k))))
+                 : plain;
   };
   take(U * mid(s.n2, s.m1));                 // 16 t1
   take(U * mid(s.n1, s.n2));                 // 17 wide (prior-scaled / lifted)
@@ -1223,9 +1226,9 @@ size_t CgBuffers::layout(const BatchShape& s, int pmax, int rank, int max_iter, 
   return off;
 }
 
-void CgBuffers::bind(const BatchShape& s, int pmax, int rank, int max_iter, uint8_t* w) {
+void CgBuffers::bind(const BatchShape& s, int pmax, int rank, int max_iter, bool split, uint8_t* w) {
   size_t o[kSlots];
-  layout(s, pmax, rank, max_iter, o);
+  layout(s, pmax, rank, max_iter, split, o);
   const int B = s.B;
   const size_t U = static_cast<size_t>(B) * (1 + pmax);
   bp = reinterpret_cast<float2*>(w + o[0]);
@@ -1345,7 +1348,7 @@ void CgEngine::matvec(int R, const float2* v, bool direction, float2* out, bool 
   // rows are forward stage 1's contracted index; the values split are the
   // same, so the results are too (264 units of 256^2 / 128^2: adjoint 2 148 ->
   // 83 us with the prior loaded ahead, forward 1 66 -> 52, forward 2 92 -> 44)
-  const bool split = c.terms == 3;
+  const bool split = c.split;
   auto split_of = [](float2* p, const DftGeom& g2) {
     return EpiSplitT{reinterpret_cast<uint8_t*>(p), split_unit_bytes(g2.rows, g2.kcplx), g2.kchunks};
   };
@@ -1665,7 +1668,11 @@ int active_kmax(const fbme::BatchShape& s, const FbmeCgConfig& c) {
   return static_cast<int>(std::min<long long>(c.active_set_max_size, s.n()));
 }
 
-CgLayout cg_layout(const fbme::BatchShape& s, const FbmeCgConfig& c) {
+// Whether a plan can hold its matvec intermediates in split form; without the
+// room for it (fbme_cg_workspace_bytes_min) they stay FP32, same results.
+bool cg_splits(const FbmeCgConfig& c) { return c.dft_terms == 3 && !c.dense; }
+
+CgLayout cg_layout(const fbme::BatchShape& s, const FbmeCgConfig& c, bool split) {
   CgLayout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -1686,7 +1693,7 @@ CgLayout cg_layout(const fbme::BatchShape& s, const FbmeCgConfig& c) {
   L.dir2 = take(s.n2 * sizeof(float2));
   size_t offs[fbme::CgBuffers::kSlots];
   const int rank = std::min<long long>(c.preconditioner_rank, std::min(s.m(), s.n()));
-  L.buffers = take(fbme::CgBuffers::layout(s, c.probes, rank, c.max_iter, offs));
+  L.buffers = take(fbme::CgBuffers::layout(s, c.probes, rank, c.max_iter, split, offs));
   const int kmax = active_kmax(s, c);
   L.active = kmax > 0 ? take(fbme::cg_active_bytes(s.n(), kmax)) : 0;
   L.dense = c.dense ? take(fbme::dense_bytes(s)) : 0;
@@ -2017,7 +2024,13 @@ extern "C" {
 size_t fbme_cg_workspace_bytes(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg) {
   fbme::BatchShape s;
   if (cg_validate(shape, n_scenes, cfg, &s) != FBME_OK) return 0;
-  return cg_layout(s, *cfg).total;
+  return cg_layout(s, *cfg, cg_splits(*cfg)).total;
+}
+
+size_t fbme_cg_workspace_bytes_min(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg) {
+  fbme::BatchShape s;
+  if (cg_validate(shape, n_scenes, cfg, &s) != FBME_OK) return 0;
+  return cg_layout(s, *cfg, false).total;
 }
 
 int fbme_cg_create(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg, void* workspace,
@@ -2027,11 +2040,13 @@ int fbme_cg_create(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig*
   fbme::BatchShape s;
   int rc = cg_validate(shape, n_scenes, cfg, &s);
   if (rc != FBME_OK) return rc;
-  const CgLayout L = cg_layout(s, *cfg);
+  bool split = cg_splits(*cfg);
+  CgLayout L = cg_layout(s, *cfg, split);
+  if (split && workspace_bytes < L.total) L = cg_layout(s, *cfg, split = false);
   if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return api_fail(FBME_ERR_WORKSPACE, "workspace must be a 256-byte aligned device pointer");
   if (workspace_bytes < L.total)
-    return api_fail(FBME_ERR_WORKSPACE, "workspace smaller than fbme_cg_workspace_bytes()");
+    return api_fail(FBME_ERR_WORKSPACE, "workspace smaller than fbme_cg_workspace_bytes_min()");
   cudaError_t e = fbme::set_dft_attributes();
   if (e == cudaSuccess) e = fbme::set_cg_attributes();
   if (e != cudaSuccess)
@@ -2072,12 +2087,13 @@ int fbme_cg_create(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig*
   fbme::launch_dirichlet(P->dir1, s.m1, s.n1, st);
   fbme::launch_dirichlet(P->dir2, s.m2, s.n2, st);
   const int rank = static_cast<int>(std::min<long long>(cfg->preconditioner_rank, std::min(s.m(), s.n())));
-  P->buf.bind(s, cfg->probes, rank, cfg->max_iter, w + L.buffers);
+  P->buf.bind(s, cfg->probes, rank, cfg->max_iter, split, w + L.buffers);
   if (cfg->dense) P->dense = fbme::dense_bind(w + L.dense, s, st);
   P->act_kmax = active_kmax(s, *cfg);
   if (P->act_kmax > 0) P->act = fbme::cg_active_bind(w + L.active, s.n(), P->act_kmax);
   fbme::CgSettings cs;
   cs.terms = terms;
+  cs.split = split;
   cs.rank = rank;
   cs.fixed_iterations = cfg->cg_fixed_iterations;
   cs.max_cg_iter = cfg->cg_max_iter;

@@ -375,7 +375,11 @@ typedef struct {
 
 typedef struct FbmeCgPlan FbmeCgPlan;
 
+/* fbme_cg_create takes any workspace of at least ..._min bytes; from
+ * fbme_cg_workspace_bytes on, the operator's intermediates are kept in the
+ * next stage's operand form, which is faster and gives the same results. */
 size_t fbme_cg_workspace_bytes(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg);
+size_t fbme_cg_workspace_bytes_min(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg);
 int fbme_cg_create(const FbmeShape* shape, int32_t n_scenes, const FbmeCgConfig* cfg,
                    void* workspace, size_t workspace_bytes, fbme_stream_t stream,
                    FbmeCgPlan** plan);
